@@ -8,17 +8,25 @@
 //              products whose contraction runs over the batch.  In kernel format the result of block
 //              (i,l) is the row-major (c, b) matrix dWk[(i*d + l)*c + k, j].
 //
-// dW on the tensor cores (16-bit inputs, fp32 accumulation in TMEM): accumulator rows are k (128 per
-// tile), columns are j (up to 256), the K dimension of the MMAs is the batch, 64 entries per stage.
-// Batch-last rows of X and dY hold consecutive batch entries: both are K-major operands fetched by
-// the 4-D maps over (batch, d, features, a) that the forward kernel uses for its input.  Batch-first
-// (d = 1) rows hold consecutive features: both are MN-major operands.  Blocks have few tiles, so the
-// batch is split over CTAs; every CTA writes an fp32 partial tile and a second kernel sums the
-// partials in a fixed order (bitwise repeatable) and converts.  Other cases (fp32, batch-first with
-// d > 1, unaligned shapes) take a plain FFMA kernel.
+// dW on the tensor cores (16-bit inputs, fp32 accumulation in TMEM): accumulator rows are k, columns
+// are j, the K dimension of the MMAs is the batch, 64 entries per stage.  The two operands are
+// independent: a batch-last one has rows of consecutive batch entries (K-major, fetched by the 4-D
+// map over (batch, d, features, a) that the forward kernel uses for its input), a batch-first one
+// with d = 1 has rows of consecutive features (MN-major).  A batch-first operand with d > 1, or one
+// whose rows are not 16-byte multiples, is first copied into a batch-last tensor with padded rows in
+// the workspace.  fp32 runs on tc_wgrad_f32.cu the same way.
 //
-// Roles of the tensor kernel (192 threads): warp 0 TMA producer, warp 1 TMEM owner and MMA issuer,
-// warps 2..5 epilogue.  Waits are bounded and report through the device status word.
+// What bounds it: the traffic from L2 to the SMs.  A CTA that owns 128 x 256 outputs reads 48 KB per
+// 64 batch entries, so a (1,768,192,4) factor reads its input three times and its output gradient
+// twice; with two accumulators one above the other (MB = 2, 256 x 256 outputs, all 512 columns of
+// TMEM) the gradient, four times the larger operand, is read once.  Blocks have few tiles, so the batch
+// is split over CTAs; every CTA writes an fp32 partial tile (staged through the idle ring, TMA
+// store) and a second kernel sums the partials in a fixed order (bitwise repeatable) and converts.
+// The number of splits minimises a time model (wgrad_splits), because whole waves of CTAs, the
+// chunks per CTA and the bytes of the partials all depend on it.
+//
+// Roles of the tensor kernel (320 threads): warp 0 TMA producer, warp 1 TMEM owner and MMA issuer,
+// warps 2..9 epilogue.  Waits are bounded and report through the device status word.
 //
 // The reference has no backward: Kernel.backward is a stub
 // (src/ksmm_py/layer/kronecker_sparse/kernel.py:323-329).
@@ -27,6 +35,7 @@
 #include <algorithm>
 #include <atomic>
 
+#include "backward.h"
 #include "tc_host.h"
 #include "tc_kernel.h"
 #include "tc_ptx.cuh"
@@ -120,36 +129,38 @@ namespace tc {
 
 struct ParamsW {
   int a, b, c, d;
-  int64_t batch;
   int tiles_k, tiles_j, splits;
   int nchunks;  // ceil(batch / 64)
   uint32_t idesc;
   float* part;  // (splits, a*d, c, b) fp32
+  int tma_part;  // b % 4 == 0: partial tiles leave through TMA
   int* status;
 };
 
-constexpr int kThreadsW = 6 * 32;
+constexpr int kThreadsW = 10 * 32;
 
-template <bool BS_LAST, int NT, int SX>
+template <int MB, int NT, int SX>
 struct CfgW {
-  static constexpr int A_BYTES = 128 * 128;  // 128 k x 64 batch entries (either order)
-  static constexpr int B_BYTES = NT * 128;   // NT j x 64 batch entries
+  static constexpr int A_BYTES = MB * 128 * 128;  // MB x 128 k x 64 batch entries (either order)
+  static constexpr int B_BYTES = NT * 128;        // NT j x 64 batch entries
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int NBAR = 2 * SX + 1;
   static constexpr int BAR_BYTES = 256;
   static constexpr int SMEM_BYTES = SX * STAGE_BYTES + BAR_BYTES + 1024;
-  static constexpr int TMEM_COLS = NT;
+  static constexpr int TMEM_COLS = MB * NT;
+  static_assert(MB == 1 || MB == 2, "accumulators above one another");
   static_assert(NT == 64 || NT == 128 || NT == 256, "j tile");
   static_assert(SMEM_BYTES <= 232448, "shared memory budget");
   static_assert(SMEM_BYTES > 116 * 1024, "one CTA per SM, so that the TMEM allocation never waits");
   static_assert(8 * NBAR + 16 <= BAR_BYTES, "barrier area");
 };
 
-template <bool BS_LAST, int NT, int SX>
+// X_LAST / G_LAST: layout of the input / of the output gradient
+template <bool X_LAST, bool G_LAST, int MB, int NT, int SX>
 __global__ void __launch_bounds__(kThreadsW, 1)
     ksmm_tc_wgrad_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmG,
-                         const ParamsW P) {
-  using C = CfgW<BS_LAST, NT, SX>;
+                         const __grid_constant__ CUtensorMap tmP, const ParamsW P) {
+  using C = CfgW<MB, NT, SX>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t sm0 = (raw + 1023u) & ~1023u;
@@ -173,6 +184,11 @@ __global__ void __launch_bounds__(kThreadsW, 1)
     *abort_flag = 0;
     fence_mbar_init();
   }
+  if (warp == 0 && lane == 0) {
+    prefetch_tensormap(&tmX);
+    prefetch_tensormap(&tmG);
+    prefetch_tensormap(&tmP);
+  }
   if (warp == 1) {
     tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), C::TMEM_COLS);
     tmem_relinquish();
@@ -181,15 +197,19 @@ __global__ void __launch_bounds__(kThreadsW, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // everything above overlaps the tail of the previous kernel in the stream; memory comes after this
+  grid_dep_wait();
+  grid_dep_launch();
 
-  // CTA -> (split, block, k tile, j tile); the split owns a contiguous range of 64-entry chunks
+  // CTA -> (split, block, k tile, j tile); the split owns a contiguous range of 64-entry chunks.  The
+  // tiles of one (split, block) are neighbours: they share their operands in L2 at the same time.
   uint32_t t = blockIdx.x;
   const int tj = static_cast<int>(t % P.tiles_j); t /= P.tiles_j;
   const int tk = static_cast<int>(t % P.tiles_k); t /= P.tiles_k;
   const int sp = static_cast<int>(t % P.splits);
   const int blk = static_cast<int>(t / P.splits);
   const int i = blk / P.d, l = blk % P.d;
-  const int k0 = tk * 128, j0 = tj * NT;
+  const int k0 = tk * (MB * 128), j0 = tj * NT;
   const int ch_begin = static_cast<int>(static_cast<int64_t>(sp) * P.nchunks / P.splits);
   const int ch_end = static_cast<int>(static_cast<int64_t>(sp + 1) * P.nchunks / P.splits);
 
@@ -202,13 +222,17 @@ __global__ void __launch_bounds__(kThreadsW, 1)
         const uint32_t bar = full_bar(si);
         mbar_expect_tx(bar, C::STAGE_BYTES);
         const int n0 = ch * 64;
-        if constexpr (BS_LAST) {
-          tma_load_4d(dst, &tmX, bar, n0, l, k0, i);
+        if constexpr (X_LAST) {
+#pragma unroll
+          for (int mb = 0; mb < MB; ++mb) tma_load_4d(dst + mb * 128 * 128, &tmX, bar, n0, l, k0 + mb * 128, i);
+        } else {
+          // 64 batch rows x 64 features per box; M groups of 64 follow one another
+#pragma unroll
+          for (int kb = 0; kb < 2 * MB; ++kb) tma_load_3d(dst + kb * 64 * 128, &tmX, bar, k0 + kb * 64, blk, n0);
+        }
+        if constexpr (G_LAST) {
           tma_load_4d(dst + C::A_BYTES, &tmG, bar, n0, l, j0, i);
         } else {
-          // 64 batch rows x 64 features per box; M / N groups of 64 follow one another
-          tma_load_3d(dst, &tmX, bar, k0, blk, n0);
-          tma_load_3d(dst + 64 * 128, &tmX, bar, k0 + 64, blk, n0);
 #pragma unroll
           for (int jb = 0; jb < NT / 64; ++jb)
             tma_load_3d(dst + C::A_BYTES + jb * 64 * 128, &tmG, bar, j0 + jb * 64, blk, n0);
@@ -223,20 +247,24 @@ __global__ void __launch_bounds__(kThreadsW, 1)
       constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
       // K-major (batch-last): 32 bytes per k step inside the swizzle row, LBO unused;
       // MN-major (batch-first): LBO = one 64-wide group (64 rows x 128 bytes), 16 rows per k step
-      constexpr uint32_t kLbo = BS_LAST ? (1u << 16) : (static_cast<uint32_t>((64 * 128) >> 4) << 16);
-      constexpr uint32_t kStep = BS_LAST ? (32u >> 4) : ((16u * 128u) >> 4);
+      constexpr uint32_t kLboK = 1u << 16, kLboMN = static_cast<uint32_t>((64 * 128) >> 4) << 16;
+      constexpr uint32_t kStepK = 32u >> 4, kStepMN = (16u * 128u) >> 4;
       uint32_t si = 0, sph = 0;
       bool ok = true;
       for (int ch = ch_begin; ch < ch_end; ++ch) {
         if (!mbar_wait<0>(full_bar(si), sph, abort_flag, P.status, 52)) { ok = false; break; }
         tc_fence_after();
         const uint32_t asrc = ring0 + si * C::STAGE_BYTES, bsrc = asrc + C::A_BYTES;
-        const uint32_t alo = (asrc >> 4) | kLbo, blo = (bsrc >> 4) | kLbo;
+        const uint32_t alo = (asrc >> 4) | (X_LAST ? kLboK : kLboMN), blo = (bsrc >> 4) | (G_LAST ? kLboK : kLboMN);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          const uint64_t adesc = (static_cast<uint64_t>(kDescHi) << 32) | (alo + k * kStep);
-          const uint64_t bdesc = (static_cast<uint64_t>(kDescHi) << 32) | (blo + k * kStep);
-          umma<2>(tmem_base, adesc, bdesc, P.idesc, (ch != ch_begin || k != 0) ? 1u : 0u);
+          const uint64_t bdesc = (static_cast<uint64_t>(kDescHi) << 32) | (blo + k * (G_LAST ? kStepK : kStepMN));
+#pragma unroll
+          for (int mb = 0; mb < MB; ++mb) {
+            const uint64_t adesc = (static_cast<uint64_t>(kDescHi) << 32) |
+                                   (alo + mb * ((128 * 128) >> 4) + k * (X_LAST ? kStepK : kStepMN));
+            umma<2>(tmem_base + mb * NT, adesc, bdesc, P.idesc, (ch != ch_begin || k != 0) ? 1u : 0u);
+          }
         }
         umma_commit(empty_bar(si));
         if (++si == SX) { si = 0; sph ^= 1u; }
@@ -245,43 +273,56 @@ __global__ void __launch_bounds__(kThreadsW, 1)
     }
     __syncwarp();
   } else {
-    // epilogue: lane = accumulator row k; 32 columns (j) per TMEM load, stored as fp32 partials
-    const int q = warp & 3;
+    // epilogue: lane = accumulator row k; 32 columns (j) per TMEM load.  MB = 2: four warps per
+    // accumulator; MB = 1: the two groups of four warps take alternate column groups.
+    const int q = warp & 3, h = (warp - 2) >> 2;
+    const int mb = MB == 2 ? h : 0;
     int got = 1;
     if (lane == 0) got = mbar_wait<128>(tfull_bar, 0u, abort_flag, P.status, 53) ? 1 : 0;
     got = __shfl_sync(0xffffffffu, got, 0);
-    if (got && ch_end > ch_begin) {
+    const int krow0 = k0 + mb * 128 + q * 32;
+    if (got && krow0 < P.c) {
       tc_fence_after();
-      const int k = k0 + q * 32 + lane;
-      float* row = P.part + ((static_cast<int64_t>(sp) * P.a * P.d + blk) * P.c + k) * P.b + j0;
-      const bool vec = (P.b % 4 == 0);
+      const int k = krow0 + lane;
+      const int pz = sp * P.a * P.d + blk;
+      // every load has been consumed by the MMAs: the ring is free for staging tiles
+      const uint32_t stg0 = ring0 + (warp - 2) * 2 * 4096;
+      uint32_t sti = 0;
 #pragma unroll 1
-      for (int cg = 0; cg < NT / 32; ++cg) {
+      for (int cg = MB == 2 ? 0 : h; cg < NT / 32; cg += MB == 2 ? 1 : 2) {
         if (j0 + cg * 32 >= P.b) break;
         uint32_t r[32];
-        tmem_ld32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + cg * 32, r);
-        tmem_ld_wait();
-        if (k < P.c) {
-          if (vec && j0 + cg * 32 + 32 <= P.b) {
+        if (ch_end > ch_begin) {
+          tmem_ld32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + mb * NT + cg * 32, r);
+          tmem_ld_wait();
+        } else {  // a split without chunks: its partial tile is zero
 #pragma unroll
-            for (int e = 0; e < 32; e += 4)
-              *reinterpret_cast<float4*>(row + cg * 32 + e) =
-                  make_float4(__uint_as_float(r[e]), __uint_as_float(r[e + 1]), __uint_as_float(r[e + 2]),
-                              __uint_as_float(r[e + 3]));
-          } else {
+          for (int e = 0; e < 32; ++e) r[e] = 0u;
+        }
+        if (P.tma_part) {
+          const uint32_t stg = stg0 + sti * 4096u;
+          sti ^= 1u;
+          if (lane == 0) bulk_wait_read<1>();  // the store before the last has read this staging tile
+          __syncwarp();
 #pragma unroll
-            for (int e = 0; e < 32; ++e)
-              if (j0 + cg * 32 + e < P.b) row[cg * 32 + e] = __uint_as_float(r[e]);
+          for (int ch = 0; ch < 8; ++ch)
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stg + lane * 128 + ((ch ^ (lane & 7)) << 4)),
+                         "r"(r[ch * 4]), "r"(r[ch * 4 + 1]), "r"(r[ch * 4 + 2]), "r"(r[ch * 4 + 3])
+                         : "memory");
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_3d(&tmP, stg, j0 + cg * 32, krow0, pz);
+            bulk_commit();
           }
+        } else if (k < P.c) {
+          float* row = P.part + (static_cast<int64_t>(pz) * P.c + k) * P.b + j0 + cg * 32;
+#pragma unroll
+          for (int e = 0; e < 32; ++e)
+            if (j0 + cg * 32 + e < P.b) row[e] = __uint_as_float(r[e]);
         }
       }
-    } else if (got) {
-      // a split without chunks (more splits than chunks): its partial tile is zero
-      const int k = k0 + q * 32 + lane;
-      if (k < P.c) {
-        float* row = P.part + ((static_cast<int64_t>(sp) * P.a * P.d + blk) * P.c + k) * P.b + j0;
-        for (int e = 0; e < NT && j0 + e < P.b; ++e) row[e] = 0.f;
-      }
+      if (lane == 0) bulk_wait<0>();
     }
     __syncwarp();
   }
@@ -298,36 +339,43 @@ __global__ void __launch_bounds__(kThreadsW, 1)
   }
 }
 
-// sums the partial tiles of the splits in a fixed order and converts to the weights' type
-template <typename T>
+// Sums the partial tiles of the splits in a fixed order and converts to the weights' type.  Four
+// elements per thread (elems is a multiple of 4 in the vector form), four splits in flight.
+template <typename T, int V>
 __global__ void __launch_bounds__(256)
     wgrad_reduce_kernel(const float* __restrict__ part, T* __restrict__ dw, int64_t elems, int splits) {
-  for (int64_t e = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x; e < elems;
+  grid_dep_wait();
+  grid_dep_launch();
+  const int64_t n = elems / V;
+  for (int64_t e = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x; e < n;
        e += static_cast<int64_t>(gridDim.x) * 256) {
-    float s = 0.f;
-    for (int q = 0; q < splits; ++q) s += part[q * elems + e];
-    dw[e] = ElemTraits<T>::from_float(s);
+    float s[V] = {};
+#pragma unroll 4
+    for (int q = 0; q < splits; ++q) {
+      float v[V];
+      load_vec<float, V>(part + q * elems + e * V, v);
+#pragma unroll
+      for (int u = 0; u < V; ++u) s[u] += v[u];
+    }
+    store_vec<T, V>(dw + e * V, s);
   }
 }
 
-static int wgrad_splits(const Problem& p, int nt) {
-  const int64_t tiles = static_cast<int64_t>(p.a) * p.d * ((p.c + 127) / 128) * ((p.b + nt - 1) / nt);
-  const int64_t nchunks = (p.batch + 63) / 64;
-  int sms = num_sms();
-  if (sms <= 0) sms = 148;
-  int64_t s = (2 * sms + tiles - 1) / tiles;   // about two CTAs' worth of work per SM
-  if (s > nchunks / 8) s = nchunks / 8;        // at least eight chunks per split
-  if (s < 1) s = 1;
-  if (s > 64) s = 64;
-  return static_cast<int>(s);
+template <typename T>
+static cudaError_t launch_reduce(const float* part, void* dw, int64_t elems, int splits, cudaStream_t stream) {
+  const bool vec = elems % 4 == 0 && reinterpret_cast<uintptr_t>(dw) % 16 == 0;
+  const int64_t items = vec ? elems / 4 : elems;
+  const unsigned grid = static_cast<unsigned>(std::min<int64_t>((items + 255) / 256, 148 * 8));
+  if (vec)
+    return launch_pdl(wgrad_reduce_kernel<T, 4>, grid, 256, 0, stream, part, static_cast<T*>(dw), elems, splits);
+  return launch_pdl(wgrad_reduce_kernel<T, 1>, grid, 256, 0, stream, part, static_cast<T*>(dw), elems, splits);
 }
 
-static int wgrad_nt(const Problem& p) { return p.b <= 64 ? 64 : (p.b <= 128 ? 128 : 256); }
-
-template <bool BS_LAST, int NT, int SX>
-static int launch_w(const Problem& p, const void* grad_out, float* part, int splits, cudaStream_t stream) {
-  using C = CfgW<BS_LAST, NT, SX>;
-  auto kern = ksmm_tc_wgrad_kernel<BS_LAST, NT, SX>;
+template <bool X_LAST, bool G_LAST, int MB, int NT, int SX>
+static int launch_w(const Problem& p, const WgradOperand& x, const WgradOperand& g, float* part, int splits,
+                    cudaStream_t stream) {
+  using C = CfgW<MB, NT, SX>;
+  auto kern = ksmm_tc_wgrad_kernel<X_LAST, G_LAST, MB, NT, SX>;
   static std::atomic<bool> attr_set[64];
   int dev = 0;
   cudaGetDevice(&dev);
@@ -339,129 +387,217 @@ static int launch_w(const Problem& p, const void* grad_out, float* part, int spl
     attr_set[dev] = true;
   }
   const uint64_t a = p.a, b = p.b, c = p.c, d = p.d, B = p.batch;
-  CUtensorMap tmX, tmG;
+  CUtensorMap tmX, tmG, tmP;
   int st;
-  if (BS_LAST) {
-    const uint64_t xd[4] = {B, d, c, a};
-    const uint64_t xs[4] = {1, B, d * B, c * d * B};
-    const uint32_t xb[4] = {64, 1, 128, 1};
-    if ((st = encode_map(&tmX, p.in_dtype, 4, p.in, xd, xs, xb)) != KSMM_OK) return st;
-    const uint64_t gd[4] = {B, d, b, a};
-    const uint64_t gs[4] = {1, B, d * B, b * d * B};
-    const uint32_t gb[4] = {64, 1, static_cast<uint32_t>(NT), 1};
-    if ((st = encode_map(&tmG, p.in_dtype, 4, grad_out, gd, gs, gb)) != KSMM_OK) return st;
-  } else {
-    const uint64_t xd[3] = {c, a, B};
-    const uint64_t xs[3] = {1, c, a * c};
-    const uint32_t xb[3] = {64, 1, 64};
-    if ((st = encode_map(&tmX, p.in_dtype, 3, p.in, xd, xs, xb)) != KSMM_OK) return st;
-    const uint64_t gd[3] = {b, a, B};
-    const uint64_t gs[3] = {1, b, a * b};
-    const uint32_t gb[3] = {64, 1, 64};
-    if ((st = encode_map(&tmG, p.in_dtype, 3, grad_out, gd, gs, gb)) != KSMM_OK) return st;
-  }
+  // batch-last: (batch, d, features, a), 64 batch entries x 128 (NT) features per box;
+  // batch-first (d = 1): (features, a, batch), 64 features x 64 batch entries per box
+  auto operand_map = [&](CUtensorMap* tm, bool last, const WgradOperand& o, uint64_t f, uint32_t rows) {
+    if (last) {
+      const uint64_t L = o.ld;
+      const uint64_t dims[4] = {B, d, f, a}, str[4] = {1, L, d * L, f * d * L};
+      const uint32_t box[4] = {64, 1, rows, 1};
+      return encode_map(tm, p.in_dtype, 4, o.ptr, dims, str, box);
+    }
+    const uint64_t dims[3] = {f, a, B}, str[3] = {1, f, a * f};
+    const uint32_t box[3] = {64, 1, 64};
+    return encode_map(tm, p.in_dtype, 3, o.ptr, dims, str, box);
+  };
+  if ((st = operand_map(&tmX, X_LAST, x, c, 128)) != KSMM_OK) return st;
+  if ((st = operand_map(&tmG, G_LAST, g, b, NT)) != KSMM_OK) return st;
   ParamsW P;
   P.a = p.a; P.b = p.b; P.c = p.c; P.d = p.d;
-  P.batch = p.batch;
-  P.tiles_k = (p.c + 127) / 128;
+  P.tiles_k = (p.c + MB * 128 - 1) / (MB * 128);
   P.tiles_j = (p.b + NT - 1) / NT;
   P.splits = splits;
   P.nchunks = static_cast<int>((p.batch + 63) / 64);
   P.part = part;
+  P.tma_part = p.b % 4 == 0 ? 1 : 0;
+  tmP = tmX;  // unused otherwise
+  if (P.tma_part) {
+    const uint64_t dims[3] = {b, c, static_cast<uint64_t>(splits) * a * d}, str[3] = {1, b, b * c};
+    const uint32_t box[3] = {32, 32, 1};
+    if ((st = encode_map(&tmP, KSMM_F32, 3, part, dims, str, box)) != KSMM_OK) return st;
+  }
   P.status = status_word();
   if (!P.status) return set_error(KSMM_ERR_CUDA, "cannot resolve the device status word");
   const uint32_t fmt = p.in_dtype == KSMM_BF16 ? 1u : 0u;
-  // fp32 accumulate, M = 128, N = NT; batch-last: both operands K-major; batch-first: both MN-major
-  P.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (BS_LAST ? 0u : ((1u << 15) | (1u << 16))) |
+  // fp32 accumulate, M = 128, N = NT; batch-last operands are K-major, batch-first ones MN-major
+  P.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (X_LAST ? 0u : 1u << 15) | (G_LAST ? 0u : 1u << 16) |
             (static_cast<uint32_t>(NT >> 3) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);
   const int64_t grid = static_cast<int64_t>(p.a) * p.d * splits * P.tiles_k * P.tiles_j;
   if (grid <= 0 || grid > 0x7fffffffLL)
     return set_error(KSMM_ERR_UNSUPPORTED, "weight gradient: %lld tiles exceed the grid limit",
                      static_cast<long long>(grid));
-  kern<<<static_cast<unsigned>(grid), kThreadsW, C::SMEM_BYTES, stream>>>(tmX, tmG, P);
+  cudaError_t err = launch_pdl(kern, static_cast<unsigned>(grid), kThreadsW, C::SMEM_BYTES, stream, tmX, tmG, tmP, P);
   count_launch();
-  cudaError_t err = cudaGetLastError();
+  if (err == cudaSuccess) err = cudaGetLastError();
   if (err != cudaSuccess)
     return set_error(KSMM_ERR_CUDA, "weight-gradient kernel launch failed: %s", cudaGetErrorString(err));
   return KSMM_OK;
 }
 
+template <bool X_LAST, bool G_LAST>
+static int launch_w_tile(const Problem& p, const WgradOperand& x, const WgradOperand& g, float* part, int mb, int nt,
+                         int splits, cudaStream_t stream) {
+  if (mb == 2) {
+    if (nt == 64) return launch_w<X_LAST, G_LAST, 2, 64, 5>(p, x, g, part, splits, stream);
+    if (nt == 128) return launch_w<X_LAST, G_LAST, 2, 128, 4>(p, x, g, part, splits, stream);
+    return launch_w<X_LAST, G_LAST, 2, 256, 3>(p, x, g, part, splits, stream);
+  }
+  if (nt == 64) return launch_w<X_LAST, G_LAST, 1, 64, 8>(p, x, g, part, splits, stream);
+  if (nt == 128) return launch_w<X_LAST, G_LAST, 1, 128, 6>(p, x, g, part, splits, stream);
+  return launch_w<X_LAST, G_LAST, 1, 256, 4>(p, x, g, part, splits, stream);
+}
+
 }  // namespace tc
 
-// can the tensor-core dW kernel run this problem (p.in = X, p.out = dW; grad_out separately)?
-bool wgrad_tc_supported(const Problem& p, const void* grad_out, bool check_pointers) {
-  if (p.in_dtype != KSMM_F16 && p.in_dtype != KSMM_BF16) return false;
-  if (p.batch <= 0 || p.batch > 0x7fffffffLL) return false;
-  if (p.bs_last) {
-    if ((p.batch * 2) % 16 != 0) return false;
-  } else {
-    if (p.d != 1 || (p.c * 2) % 16 != 0 || (p.b * 2) % 16 != 0) return false;
+// ---------------------------------------------------------------------------
+// plan of one weight gradient
+// ---------------------------------------------------------------------------
+namespace {
+
+constexpr size_t align256(size_t v) { return (v + 255) / 256 * 256; }
+
+struct WgradPlan {
+  bool tc = false;                 // tensor cores; else the FFMA kernel
+  bool copy_x = false, copy_g = false;
+  int64_t ld_copy = 0;             // row stride of the copies
+  int mb = 1, nt = 256, splits = 1;
+  size_t x_bytes = 0, g_bytes = 0, part_bytes = 0;
+  size_t total() const { return x_bytes + g_bytes + part_bytes; }
+};
+
+// Splits of the batch.  A CTA's time is its chunks plus its partial tile, both as bytes that cross
+// L2 (about 45 GB/s per SM in these kernels), plus a fixed 2 us; CTAs run in waves of one per SM; the
+// reduction then reads all partials.
+int wgrad_splits(int64_t tiles, int64_t nchunks, double chunk_bytes, double tile_bytes, double elems) {
+  int sms = tc::num_sms();
+  if (sms <= 0) sms = 148;
+  const int64_t most = std::min<int64_t>(64, std::max<int64_t>(1, nchunks / 2));
+  double best = 1e30;
+  int pick = 1;
+  for (int64_t s = 1; s <= most; ++s) {
+    const double waves = static_cast<double>((tiles * s + sms - 1) / sms);
+    const double chunks = static_cast<double>((nchunks + s - 1) / s);
+    const double us = waves * ((chunks * chunk_bytes + tile_bytes) / 45e3 + 2.0) + s * elems * 4.0 / 5e6;
+    if (us < best * 0.995) { best = us; pick = static_cast<int>(s); }
   }
-  if (check_pointers &&
-      (reinterpret_cast<uintptr_t>(p.in) % 16 || reinterpret_cast<uintptr_t>(grad_out) % 16))
-    return false;
-  return true;
+  return pick;
 }
 
-size_t wgrad_workspace_bytes(const Problem& p) {
-  if (!wgrad_tc_supported(p, nullptr, false)) return 0;
-  const size_t elems = static_cast<size_t>(p.a) * p.b * p.c * p.d;
-  return static_cast<size_t>(tc::wgrad_splits(p, tc::wgrad_nt(p))) * elems * sizeof(float);
+bool wgrad_operand_direct(const Problem& p, const WgradOperand& o, int feat, bool check_pointers) {
+  const int es = dtype_size(p.in_dtype);
+  if (check_pointers && reinterpret_cast<uintptr_t>(o.ptr) % 16) return false;
+  if (o.last) return (o.ld * es) % 16 == 0;
+  // fp32 batch-first operands are addressed in atoms of 32 features
+  return p.d == 1 && (p.in_dtype == KSMM_F32 ? feat % 32 == 0 : (feat * es) % 16 == 0);
 }
 
-// p.in = X, p.out = dW (kernel format, input dtype); grad_out = dY
-int wgrad_launch(const Problem& p, const void* grad_out, void* workspace, size_t workspace_bytes,
+WgradPlan plan_wgrad(const Problem& p, const WgradOperand& x, const WgradOperand& g, bool check_pointers) {
+  WgradPlan w;
+  if (p.batch <= 0 || p.batch > 0x7fffffffLL) return w;
+  const bool f32 = p.in_dtype == KSMM_F32;
+  if (!f32 && p.in_dtype != KSMM_F16 && p.in_dtype != KSMM_BF16) return w;
+  w.copy_x = !wgrad_operand_direct(p, x, p.c, check_pointers);
+  w.copy_g = !wgrad_operand_direct(p, g, p.b, check_pointers);
+  // The padding of a tile is all the work there is for blocks of a few rows; the FFMA kernel, one CTA
+  // per 16 x 16 outputs, takes those unless the 16-bit operands can be used as they stand.
+  if ((p.b < 16 || p.c < 16) && (f32 || w.copy_x || w.copy_g)) return w;
+  w.tc = true;
+  w.ld_copy = (p.batch + 63) / 64 * 64;
+  const size_t es = dtype_size(p.in_dtype), ad = static_cast<size_t>(p.a) * p.d;
+  if (w.copy_x) w.x_bytes = align256(ad * p.c * w.ld_copy * es);
+  if (w.copy_g) w.g_bytes = align256(ad * p.b * w.ld_copy * es);
+  const double elems = static_cast<double>(ad) * p.b * p.c;
+  const int64_t blocks = static_cast<int64_t>(ad);
+  if (f32) {
+    w.mb = 1;
+    w.nt = p.b <= 64 ? 64 : 128;
+    // the three products per term are the time of a chunk of 32 entries (about 0.65 us), not its bytes
+    w.splits = wgrad_splits(blocks * ((p.c + 127) / 128) * ((p.b + w.nt - 1) / w.nt), (p.batch + 31) / 32,
+                            w.nt == 64 ? 22e3 : 30e3, 128.0 * w.nt * 4, elems);
+  } else {
+    w.mb = p.c > 128 ? 2 : 1;
+    w.nt = p.b <= 64 ? 64 : (p.b <= 128 ? 128 : 256);
+    const int cr = std::min(p.c, w.mb * 128), br = std::min(p.b, w.nt);  // rows that exist
+    w.splits = wgrad_splits(blocks * ((p.c + w.mb * 128 - 1) / (w.mb * 128)) * ((p.b + w.nt - 1) / w.nt),
+                            (p.batch + 63) / 64, 128.0 * (cr + br), 4.0 * cr * br, elems);
+  }
+  w.part_bytes = static_cast<size_t>(w.splits) * static_cast<size_t>(elems) * sizeof(float);
+  return w;
+}
+
+// batch-last copy with padded rows of an operand that the tensor kernels cannot address
+int wgrad_copy(const Problem& p, WgradOperand* o, int feat, void* dst, int64_t ld, cudaStream_t stream) {
+  const int64_t rows = static_cast<int64_t>(p.a) * feat * p.d;
+  const int es = dtype_size(p.in_dtype);
+  const int st = o->last ? launch_copy_rows(o->ptr, o->ld, dst, ld, rows, p.batch, es, stream)
+                         : launch_transpose(o->ptr, dst, p.batch, rows, es, stream, ld);
+  *o = WgradOperand{dst, 1, ld};
+  return st;
+}
+
+}  // namespace
+
+size_t wgrad_workspace_bytes(const Problem& p, const WgradOperand& x, const WgradOperand& g) {
+  return plan_wgrad(p, x, g, false).total();
+}
+
+// p.out = dW (kernel format, input dtype); x = X, g = dY
+int wgrad_launch(const Problem& p, WgradOperand x, WgradOperand g, void* workspace, size_t workspace_bytes,
                  cudaStream_t stream) {
   const int64_t elems = static_cast<int64_t>(p.a) * p.b * p.c * p.d;
   if (p.batch == 0) {
     cudaError_t e = cudaMemsetAsync(p.out, 0, elems * dtype_size(p.in_dtype), stream);
     return e == cudaSuccess ? KSMM_OK : set_error(KSMM_ERR_CUDA, "memset failed: %s", cudaGetErrorString(e));
   }
-  if (wgrad_tc_supported(p, grad_out, true) && workspace &&
-      reinterpret_cast<uintptr_t>(workspace) % 16 == 0 && workspace_bytes >= wgrad_workspace_bytes(p)) {
-    const int nt = tc::wgrad_nt(p);
-    const int splits = tc::wgrad_splits(p, nt);
-    float* part = static_cast<float*>(workspace);
-    int st;
-    if (p.bs_last)
-      st = nt == 64 ? tc::launch_w<true, 64, 8>(p, grad_out, part, splits, stream)
-                    : (nt == 128 ? tc::launch_w<true, 128, 6>(p, grad_out, part, splits, stream)
-                                 : tc::launch_w<true, 256, 4>(p, grad_out, part, splits, stream));
-    else
-      st = nt == 64 ? tc::launch_w<false, 64, 8>(p, grad_out, part, splits, stream)
-                    : (nt == 128 ? tc::launch_w<false, 128, 6>(p, grad_out, part, splits, stream)
-                                 : tc::launch_w<false, 256, 4>(p, grad_out, part, splits, stream));
+  const WgradPlan w = plan_wgrad(p, x, g, true);
+  if (w.tc && workspace && reinterpret_cast<uintptr_t>(workspace) % 16 == 0 && workspace_bytes >= w.total()) {
+    char* ws = static_cast<char*>(workspace);
+    float* part = reinterpret_cast<float*>(ws + w.x_bytes + w.g_bytes);
+    int st = KSMM_OK;
+    if (w.copy_x && (st = wgrad_copy(p, &x, p.c, ws, w.ld_copy, stream)) != KSMM_OK) return st;
+    if (w.copy_g && (st = wgrad_copy(p, &g, p.b, ws + w.x_bytes, w.ld_copy, stream)) != KSMM_OK) return st;
+    if (p.in_dtype == KSMM_F32) {
+      st = wgrad_f32_launch(p, x, g, part, w.nt, w.splits, stream);
+    } else if (x.last) {
+      st = g.last ? tc::launch_w_tile<true, true>(p, x, g, part, w.mb, w.nt, w.splits, stream)
+                  : tc::launch_w_tile<true, false>(p, x, g, part, w.mb, w.nt, w.splits, stream);
+    } else {
+      st = g.last ? tc::launch_w_tile<false, true>(p, x, g, part, w.mb, w.nt, w.splits, stream)
+                  : tc::launch_w_tile<false, false>(p, x, g, part, w.mb, w.nt, w.splits, stream);
+    }
     if (st != KSMM_OK) return st;
-    const unsigned grid = static_cast<unsigned>(std::min<int64_t>((elems + 255) / 256, 148 * 8));
-    if (p.in_dtype == KSMM_F16)
-      tc::wgrad_reduce_kernel<__half><<<grid, 256, 0, stream>>>(part, static_cast<__half*>(p.out), elems, splits);
-    else
-      tc::wgrad_reduce_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(part, static_cast<__nv_bfloat16*>(p.out),
-                                                                     elems, splits);
+    cudaError_t err = p.in_dtype == KSMM_F32  ? tc::launch_reduce<float>(part, p.out, elems, w.splits, stream)
+                      : p.in_dtype == KSMM_F16 ? tc::launch_reduce<__half>(part, p.out, elems, w.splits, stream)
+                                               : tc::launch_reduce<__nv_bfloat16>(part, p.out, elems, w.splits, stream);
     count_launch();
-    cudaError_t err = cudaGetLastError();
+    if (err == cudaSuccess) err = cudaGetLastError();
     if (err != cudaSuccess)
       return set_error(KSMM_ERR_CUDA, "weight-gradient reduction launch failed: %s", cudaGetErrorString(err));
     return KSMM_OK;
   }
+  if (x.last != g.last || (x.last && (x.ld != p.batch || g.ld != p.batch)))
+    return set_error(KSMM_ERR_WORKSPACE, "weight gradient: operands in two layouts need a workspace of %zu bytes",
+                     w.total());
   const int64_t nblk = static_cast<int64_t>(p.a) * p.d;
   if (nblk > 65535 || (p.c + 15) / 16 > 65535)
     return set_error(KSMM_ERR_UNSUPPORTED, "weight gradient: too many blocks for the fallback kernel");
   dim3 grid((p.b + 15) / 16, (p.c + 15) / 16, static_cast<unsigned>(nblk));
   if (p.in_dtype == KSMM_F32)
-    wgrad_simt_kernel<float><<<grid, 256, 0, stream>>>(static_cast<const float*>(p.in),
-                                                       static_cast<const float*>(grad_out),
+    wgrad_simt_kernel<float><<<grid, 256, 0, stream>>>(static_cast<const float*>(x.ptr),
+                                                       static_cast<const float*>(g.ptr),
                                                        static_cast<float*>(p.out), p.batch, p.a, p.b, p.c, p.d,
-                                                       p.bs_last);
+                                                       x.last);
   else if (p.in_dtype == KSMM_F16)
-    wgrad_simt_kernel<__half><<<grid, 256, 0, stream>>>(static_cast<const __half*>(p.in),
-                                                        static_cast<const __half*>(grad_out),
+    wgrad_simt_kernel<__half><<<grid, 256, 0, stream>>>(static_cast<const __half*>(x.ptr),
+                                                        static_cast<const __half*>(g.ptr),
                                                         static_cast<__half*>(p.out), p.batch, p.a, p.b, p.c, p.d,
-                                                        p.bs_last);
+                                                        x.last);
   else if (p.in_dtype == KSMM_BF16)
     wgrad_simt_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(p.in), static_cast<const __nv_bfloat16*>(grad_out),
-        static_cast<__nv_bfloat16*>(p.out), p.batch, p.a, p.b, p.c, p.d, p.bs_last);
+        static_cast<const __nv_bfloat16*>(x.ptr), static_cast<const __nv_bfloat16*>(g.ptr),
+        static_cast<__nv_bfloat16*>(p.out), p.batch, p.a, p.b, p.c, p.d, x.last);
   else
     return set_error(KSMM_ERR_UNSUPPORTED, "weight gradients exist for fp32, fp16 and bf16");
   count_launch();

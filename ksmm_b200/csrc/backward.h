@@ -1,0 +1,35 @@
+// Host interface of the backward kernels (backward.cu, tc_wgrad_f32.cu).
+#pragma once
+
+#include "common.cuh"
+
+namespace ksmm {
+
+// One operand of a weight gradient: the factor's input or the gradient of its output.  `ld` is the
+// row stride in elements of a batch-last operand (the batch, or more where rows are padded).
+struct WgradOperand {
+  const void* ptr;
+  int last;    // 1: (features, batch), 0: (batch, features)
+  int64_t ld;
+};
+
+// block transposes of kernel-format weights: (nblk, c, b) -> (nblk, b, c)
+int launch_transpose_blocks(const void* in, void* out, int64_t nblk, int c, int b, int es, cudaStream_t stream);
+
+// dW of the factor of `p` (pattern, batch, type; p.out = dW in kernel format).  The workspace holds
+// copies of operands that cannot be addressed as they stand, and the partial sums.
+size_t wgrad_workspace_bytes(const Problem& p, const WgradOperand& x, const WgradOperand& g);
+int wgrad_launch(const Problem& p, WgradOperand x, WgradOperand g, void* workspace, size_t workspace_bytes,
+                 cudaStream_t stream);
+// the fp32 tensor-core kernel: partial tiles (splits, a*d, c, b) into `part`; nt = 64 or 128 columns
+int wgrad_f32_launch(const Problem& p, const WgradOperand& x, const WgradOperand& g, float* part, int nt, int splits,
+                     cudaStream_t stream);
+
+// in: rows x cols row-major, out: cols x rows with row stride out_ld (0 = rows)
+int launch_transpose(const void* in, void* out, int64_t rows, int64_t cols, int es, cudaStream_t stream,
+                     int64_t out_ld = 0);
+// rows x cols from row stride in_ld to row stride out_ld (elements of es bytes)
+int launch_copy_rows(const void* in, int64_t in_ld, void* out, int64_t out_ld, int64_t rows, int64_t cols, int es,
+                     cudaStream_t stream);
+
+}  // namespace ksmm

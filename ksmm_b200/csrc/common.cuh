@@ -135,6 +135,9 @@ struct Problem {
   int in_dtype, out_dtype;
   int bs_last;             // layout of the input (and of the output unless out_bs_last says otherwise)
   int out_bs_last = -1;    // -1: same as the input; 0 / 1: batch-first / batch-last output (d = 1 factors)
+  // Row strides in elements of a batch-last input / output; 0 = the batch.  Intermediates whose batch
+  // is not a whole number of 16-byte pieces have padded rows, so that tensor maps can address them.
+  int64_t in_ld = 0, out_ld = 0;
   float alpha;
   // Chains only.  out_regroup_d > 0: store the output regrouped by the blocks of the next factor
   // (c = out_regroup_c, d = out_regroup_d): feature (i2*c + k)*d + l goes to (i2*d + l)*c + k.
@@ -157,6 +160,15 @@ struct Problem {
   int groups = 1;
   int group_shared_input = 1;
 };
+
+inline bool in_is_last(const Problem& p) { return p.bs_last != 0; }
+inline bool out_is_last(const Problem& p) { return p.out_bs_last < 0 ? p.bs_last != 0 : p.out_bs_last != 0; }
+__host__ __device__ inline int64_t in_stride(const Problem& p) { return p.in_ld ? p.in_ld : p.batch; }
+__host__ __device__ inline int64_t out_stride(const Problem& p) { return p.out_ld ? p.out_ld : p.batch; }
+// true if a batch-last input or output has padded rows
+inline bool has_padded_rows(const Problem& p) {
+  return (in_is_last(p) && in_stride(p) != p.batch) || (out_is_last(p) && out_stride(p) != p.batch);
+}
 
 // element-wise epilogue function (ksmm_activation_t)
 // erf by the rational approximation 7.1.26 of Abramowitz and Stegun (absolute error below

@@ -232,6 +232,7 @@ static int launch(const Problem& p, cudaStream_t stream) {
 
 bool ffma_tma_supported(const Problem& p, bool check_pointers) {
   if (p.in_dtype != KSMM_F32 || p.out_dtype != KSMM_F32 || !p.bs_last) return false;
+  if (has_padded_rows(p)) return false;
   if (p.batch <= 0 || p.batch > 0x7fffffffLL || p.batch % 4 != 0 || p.b % 4 != 0) return false;
   if (check_pointers) {
     if (reinterpret_cast<uintptr_t>(p.in) % 16 || reinterpret_cast<uintptr_t>(p.w) % 16 ||

@@ -12,6 +12,7 @@
 #include <tuple>
 #include <vector>
 
+#include "backward.h"
 #include "common.cuh"
 #include "tc_kernel.h"
 
@@ -54,13 +55,6 @@ int ffma_tma_launch(const Problem& p, int wide, cudaStream_t stream);
 // fp32 batch-first kernel with TMA-staged operands (ffma_tma_first.cu): configuration kFfmaTmaFirst
 bool ffma_tma_first_supported(const Problem& p, bool check_pointers);
 int ffma_tma_first_launch(const Problem& p, cudaStream_t stream);
-int launch_transpose(const void* in, void* out, int64_t rows, int64_t cols, int es,
-                     cudaStream_t stream);
-// backward.cu
-int launch_transpose_blocks(const void* in, void* out, int64_t nblk, int c, int b, int es, cudaStream_t stream);
-size_t wgrad_workspace_bytes(const Problem& p);
-int wgrad_launch(const Problem& p, const void* grad_out, void* workspace, size_t workspace_bytes,
-                 cudaStream_t stream);
 static constexpr int kFfmaTmaWide = 6, kFfmaTmaNarrow = 7, kFfmaTmaFirst = 8, kNumFfmaConfigs = 9;
 
 static int simt_launch_raw(const Problem& p, int config, cudaStream_t stream) {
@@ -155,7 +149,8 @@ static int residual_pass(const Problem& p, cudaStream_t stream) {
 static int simt_launch(const Problem& p, int config, cudaStream_t stream) {
   int st = simt_launch_raw(p, config, stream);
   if (st != KSMM_OK || p.activation == 0) return st;
-  const int64_t n = static_cast<int64_t>(p.a) * p.b * p.d * p.batch;
+  // (the padding of a batch-last output's rows goes through the function as well)
+  const int64_t n = static_cast<int64_t>(p.a) * p.b * p.d * (out_is_last(p) ? out_stride(p) : p.batch);
   const unsigned grid = static_cast<unsigned>(std::min<int64_t>((n + 255) / 256, 148 * 16));
   if (p.out_dtype == KSMM_F32)
     activation_kernel<float><<<grid, 256, 0, stream>>>(static_cast<float*>(p.out), n, p.activation);
@@ -1090,7 +1085,7 @@ size_t ksmm_cu_backward_weights_workspace_bytes(int64_t batch, int a, int b, int
                                                 int bs_last) {
   if (batch <= 0 || a <= 0 || b <= 0 || c <= 0 || d <= 0) return 0;
   Problem p = backward_problem(nullptr, nullptr, nullptr, batch, a, b, c, d, dtype, bs_last);
-  return wgrad_workspace_bytes(p);
+  return wgrad_workspace_bytes(p, WgradOperand{nullptr, bs_last ? 1 : 0, batch}, WgradOperand{nullptr, bs_last ? 1 : 0, batch});
 }
 
 int ksmm_cu_backward_weights(const void* input, const void* grad_output, void* grad_values, void* workspace,
@@ -1099,7 +1094,8 @@ int ksmm_cu_backward_weights(const void* input, const void* grad_output, void* g
   Problem p = backward_problem(input, grad_output, grad_values, batch, a, b, c, d, dtype, bs_last);
   int st = check_backward(p);
   if (st != KSMM_OK) return st;
-  return wgrad_launch(p, grad_output, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
+  return wgrad_launch(p, WgradOperand{input, bs_last, batch}, WgradOperand{grad_output, bs_last, batch}, workspace,
+                      workspace_bytes, static_cast<cudaStream_t>(stream));
 }
 
 int ksmm_cu_chain_forward_static(const void* input, const void* const* values, void* output,

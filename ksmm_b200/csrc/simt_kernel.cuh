@@ -61,7 +61,8 @@ __global__ void __launch_bounds__(WJ* WN * 32, 512 / (WJ * WN * 32))
   const Problem& p = sp.p;
   const int a = p.a, b = p.b, c = p.c, d = p.d;
   (void)a;
-  const int64_t B = p.batch;
+  const int64_t B = p.batch, ldx = in_stride(p), ldy = out_stride(p);
+  (void)ldx; (void)ldy;
   const bool xvec = sp.flags & 1u, wvec = sp.flags & 2u, yvec = sp.flags & 4u;
 
   // block -> (batch tile, j tile, block (i,l)); batch tile fastest so that
@@ -107,7 +108,7 @@ __global__ void __launch_bounds__(WJ* WN * 32, 512 / (WJ * WN * 32))
           const int64_t gn = n0 + n4 * 4;
           if (gk < c && gn < B) {
             const int64_t row = (static_cast<int64_t>(i) * c + gk) * d + l;
-            load_vec<TIn, 4>(X + row * B + gn, tmp);
+            load_vec<TIn, 4>(X + row * ldx + gn, tmp);
           }
         } else {
           const int n = v / (KC / 4), k4 = v % (KC / 4);
@@ -131,7 +132,7 @@ __global__ void __launch_bounds__(WJ* WN * 32, 512 / (WJ * WN * 32))
           const int64_t gn = n0 + n;
           if (gk < c && gn < B) {
             const int64_t row = (static_cast<int64_t>(i) * c + gk) * d + l;
-            val = ElemTraits<TIn>::to_float(X[row * B + gn]);
+            val = ElemTraits<TIn>::to_float(X[row * ldx + gn]);
           }
         } else {
           const int n = v / KC, k = v % KC;
@@ -276,11 +277,11 @@ __global__ void __launch_bounds__(WJ* WN * 32, 512 / (WJ * WN * 32))
 #pragma unroll
         for (int t = 0; t < 4; ++t) v[t] = fmaf(alpha, acc[m][half * 4 + t], bv);
         if (yvec) {
-          if (gn < B) store_vec<TOut, 4>(Y + row * B + gn, v);
+          if (gn < B) store_vec<TOut, 4>(Y + row * ldy + gn, v);
         } else {
 #pragma unroll
           for (int t = 0; t < 4; ++t)
-            if (gn + t < B) Y[row * B + gn + t] = ElemTraits<TOut>::from_float(v[t]);
+            if (gn + t < B) Y[row * ldy + gn + t] = ElemTraits<TOut>::from_float(v[t]);
         }
       }
     }
@@ -354,8 +355,9 @@ int simt_launch_one(const Problem& p, cudaStream_t stream) {
   const uintptr_t bptr = reinterpret_cast<uintptr_t>(p.bias);
   unsigned flags = 0;
   if (BS_LAST) {
-    if (p.batch % 4 == 0 && xin % (4 * sizeof(TIn)) == 0) flags |= 1u;
-    if (p.batch % 4 == 0 && yout % (4 * sizeof(TOut)) == 0) flags |= 4u;
+    // (a vector never straddles the end of the batch: it starts at a multiple of 4 below it)
+    if (p.batch % 4 == 0 && in_stride(p) % 4 == 0 && xin % (4 * sizeof(TIn)) == 0) flags |= 1u;
+    if (p.batch % 4 == 0 && out_stride(p) % 4 == 0 && yout % (4 * sizeof(TOut)) == 0) flags |= 4u;
   } else {
     if (p.d == 1 && p.c % 4 == 0 && xin % (4 * sizeof(TIn)) == 0) flags |= 1u;
     if (p.d == 1 && p.b % C::VJ == 0 && yout % (C::VJ * sizeof(TOut)) == 0 &&

@@ -83,6 +83,7 @@ namespace tc {
 struct ParamsF {
   int a, b, c, d;
   int64_t batch;
+  int64_t out_ld;       // row stride of a batch-last output
   int tiles_n, tiles_j;
   uint32_t rows;        // blocks * tiles_n: (block, batch tile) pairs
   uint32_t row_groups;  // CTAs per j tile
@@ -501,8 +502,8 @@ __global__ void __launch_bounds__(kThreadsF, 1)
       const bool warp_active = n0 + q * 32 < P.batch;
       // direct stores: row (i*b + j0)*d + l of the output, this lane's batch entry
       const int64_t n_row = static_cast<int64_t>(n0) + q * 32 + lane;
-      const int64_t jstride = static_cast<int64_t>(P.d) * P.batch;
-      float* row_out = P.out + ((static_cast<int64_t>(blk / P.d) * P.b + j0) * P.d + blk % P.d) * P.batch + n_row;
+      const int64_t jstride = static_cast<int64_t>(P.d) * P.out_ld;
+      float* row_out = P.out + ((static_cast<int64_t>(blk / P.d) * P.b + j0) * P.d + blk % P.d) * P.out_ld + n_row;
       (void)n_row; (void)jstride; (void)row_out;
       int jlim = P.b - j0;
       if (jlim > C::NJ) jlim = C::NJ;
@@ -639,8 +640,11 @@ static int launch_f(const Problem& p, cudaStream_t stream) {
   if (IN_LAST) {
     // input (a*c*d, batch), row (i*c + k)*d + l, seen as (n % 32, k, n / 32, l, i): one box is the
     // four atoms (32 batch entries x 32 k rows) of an MN-major operand tile
-    const uint64_t dims[5] = {32, c, B / 32, d, a};
-    const uint64_t str[5] = {1, d * B, 32, B, c * d * B};
+    // (rows are whole atoms: where the batch ends inside one, its tail feeds accumulator rows that are
+    // never stored)
+    const uint64_t L = in_stride(p);
+    const uint64_t dims[5] = {32, c, (B + 31) / 32, d, a};
+    const uint64_t str[5] = {1, d * L, 32, L, c * d * L};
     const uint32_t box[5] = {32, kKC, 4, 1, 1};
     if ((st = encode_map(&tmX, KSMM_F32, 5, p.in, dims, str, box, true, true)) != KSMM_OK) return st;
   } else {
@@ -662,7 +666,8 @@ static int launch_f(const Problem& p, cudaStream_t stream) {
   } else if (BS_LAST) {
     // output (a*b*d, batch): row (i*b + j)*d + l; store = 32 j x 32 batch entries
     const uint64_t dims[4] = {B, d, b, a};
-    const uint64_t str[4] = {1, B, d * B, b * d * B};
+    const uint64_t L = out_stride(p);
+    const uint64_t str[4] = {1, L, d * L, b * d * L};
     const uint32_t box[4] = {32, 1, 32, 1};
     if ((st = encode_map(&tmY, KSMM_F32, 4, p.out, dims, str, box, false)) != KSMM_OK) return st;
   } else {
@@ -675,6 +680,7 @@ static int launch_f(const Problem& p, cudaStream_t stream) {
   ParamsF P;
   P.a = p.a; P.b = p.b; P.c = p.c; P.d = p.d;
   P.batch = p.batch;
+  P.out_ld = out_stride(p);
   P.tiles_n = static_cast<int>((B + 127) / 128);
   P.tiles_j = static_cast<int>((b + C::NJ - 1) / C::NJ);
   P.nchunks = (p.c + kKC - 1) / kKC;
@@ -715,11 +721,10 @@ bool tc_f32x3_supported(const Problem& p, bool check_pointers) {
   if (p.batch <= 0 || p.batch > 0x7fffffffLL) return false;
   // the operand tiles are addressed in atoms of 32 columns; global strides are multiples of 16 bytes
   if (p.b % 32 != 0) return false;
-  const bool out_last = p.out_bs_last < 0 ? p.bs_last != 0 : p.out_bs_last != 0;
+  const bool out_last = out_is_last(p);
   if (out_last != (p.bs_last != 0) && (p.d != 1 || p.groups > 1)) return false;  // layout-changing factors
-  if (p.bs_last || out_last) {
-    if (p.batch % 32 != 0) return false;
-  }
+  if (p.bs_last && in_stride(p) % 32 != 0) return false;
+  if (out_last && out_stride(p) % 32 != 0) return false;
   if (!p.bs_last) {
     if (p.d != 1 || p.c % 4 != 0) return false;
   }

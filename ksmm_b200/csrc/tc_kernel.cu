@@ -669,7 +669,8 @@ static int launch_one(const Problem& p, cudaStream_t stream) {
                    (static_cast<uint32_t>(NT >> 3) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);
   if (IN_LAST) {
     const uint64_t xd[4] = {B, d, c, GX * a};
-    const uint64_t xs[4] = {1, B, d * B, c * d * B};
+    const uint64_t L = in_stride(p);
+    const uint64_t xs[4] = {1, L, d * L, c * d * L};
     const uint32_t xb[4] = {static_cast<uint32_t>(C::NBOX), 1, static_cast<uint32_t>(KC), 1};
     if ((st = encode_map(&tmX, p.in_dtype, 4, p.in, xd, xs, xb)) != KSMM_OK) return st;
   } else {
@@ -680,7 +681,8 @@ static int launch_one(const Problem& p, cudaStream_t stream) {
   }
   if (OUT_LAST) {
     const uint64_t yd[4] = {B, d, b, G * a};
-    const uint64_t ys[4] = {1, B, d * B, b * d * B};
+    const uint64_t L = out_stride(p);
+    const uint64_t ys[4] = {1, L, d * L, b * d * L};
     const uint32_t yb[4] = {static_cast<uint32_t>(C::CB), 1, 32, 1};  // one epilogue warp's rows
     if ((st = encode_map(&tmY, p.out_dtype, 4, p.out, yd, ys, yb)) != KSMM_OK) return st;
   } else if (p.out_regroup_d > 0 && OS == 2) {
@@ -811,7 +813,8 @@ bool tc_config_supported(const Problem& p, int config, bool check_pointers) {
     if (p.in_dtype == KSMM_F32) return config >= 0 && config <= 3 && tc_f32x3_supported(p, check_pointers);
     if ((p.in_dtype != KSMM_F16 && p.in_dtype != KSMM_BF16) || p.out_dtype != p.in_dtype) return false;
     if (p.batch <= 0 || p.batch > 0x7fffffffLL) return false;
-    if (p.b % 8 != 0 || p.c % 8 != 0 || p.batch % 8 != 0) return false;   // 16-byte strides on both sides
+    if (p.b % 8 != 0 || p.c % 8 != 0) return false;   // 16-byte strides on both sides
+    if ((p.bs_last ? in_stride(p) : out_stride(p)) % 8 != 0) return false;
     if (check_pointers && (reinterpret_cast<uintptr_t>(p.in) % 16 || reinterpret_cast<uintptr_t>(p.w) % 16 ||
                            reinterpret_cast<uintptr_t>(p.out) % 16))
       return false;
@@ -834,7 +837,7 @@ bool tc_config_supported(const Problem& p, int config, bool check_pointers) {
   // tensor-map rules: every global stride is a multiple of 16 bytes
   if ((static_cast<int64_t>(p.b) * es) % 16 != 0) return false;
   if (p.bs_last) {
-    if ((p.batch * es) % 16 != 0 || (p.batch * os) % 16 != 0) return false;
+    if ((in_stride(p) * es) % 16 != 0 || (out_stride(p) * os) % 16 != 0) return false;
   } else {
     if (p.d != 1) return false;
     if ((static_cast<int64_t>(p.c) * es) % 16 != 0) return false;
@@ -864,7 +867,7 @@ bool tc_fuses_residual(const Problem& p) {
   if (p.in_dtype == KSMM_F32) return false;
   const bool out_last = p.out_bs_last < 0 ? p.bs_last != 0 : p.out_bs_last != 0;
   if (out_last == (p.bs_last != 0) && !p.bs_last && p.d != 1) return false;
-  if (p.groups > 1 || p.out_regroup_d) return false;
+  if (p.groups > 1 || p.out_regroup_d || has_padded_rows(p)) return false;
   return reinterpret_cast<uintptr_t>(p.residual) % 16 == 0;
 }
 

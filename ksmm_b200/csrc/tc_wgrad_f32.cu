@@ -1,0 +1,388 @@
+// fp32 weight gradients on the tensor cores:
+//   dW[i,j,k,l] = sum_n dY4[i,j,l,n] X4[i,k,l,n],
+// a*d independent (c x B) @ (B x b) products, each term as three tf32 products (see tc_f32x3.cu for the
+// split and its error): hi(x) hi(g) + lo(x) hi(g) + hi(x) lo(g) with fp32 accumulation.
+//
+// Accumulator rows are k (128 per tile), columns j (NT = 64 or 128), the K dimension of the MMAs is
+// the batch, 32 entries per stage.  A stage holds [X hi | X lo | G hi | G lo]; the raw tiles that TMA
+// delivers are the hi operands as they stand, six splitter warps add the lo tiles at the same
+// offsets.  G lo follows G hi directly, so the two are one operand of 2 NT rows.  A batch-last operand
+// has rows of consecutive batch entries: K-major, plain 128-byte swizzle.  A batch-first one (d = 1)
+// has rows of consecutive features: MN-major, atoms of 32 features x 32 batch rows with the 128-byte
+// swizzle of 32-byte pieces.  The split is element-wise, so any combination of the two works.
+//
+// The contraction is long (a training batch), and the tensor core truncates when it adds into its
+// accumulator, once per step of 8 entries.  So the accumulator only ever sums kFlush chunks (512
+// entries, 64 additions, the error of a forward factor with c = 512); the epilogue warps then add it,
+// rounded to nearest, to sums in registers, while the MMAs fill the other accumulator buffer.
+//
+// What bounds it: the shared-memory pipe.  A chunk of 32 entries (NT = 128) is written once by TMA
+// (32 KB), read and written by the splitters (64 KB) and read by the MMAs (80 KB), about 1400
+// cycles at 128 bytes a cycle against 1080 for its eight MMAs.  The batch is split over CTAs as in
+// backward.cu; (1,768,192,2) at 6272 batch entries: 485 us on the FFMA kernel before.
+//
+// Roles (512 threads): warp 0 TMA producer, warp 1 TMEM owner and MMA issuer, warps 2..7 splitters,
+// warps 8..15 epilogue.  Waits are bounded and report through the device status word.
+#include <cuda.h>
+
+#include <atomic>
+
+#include "backward.h"
+#include "tc_host.h"
+#include "tc_kernel.h"
+#include "tc_ptx.cuh"
+
+namespace ksmm {
+namespace tc {
+
+struct ParamsWF {
+  int a, b, c, d;
+  int tiles_k, tiles_j, splits;
+  int nchunks;      // ceil(batch / 32)
+  uint32_t idesc;   // N = NT
+  uint32_t idesc2;  // N = 2 NT
+  float* part;      // (splits, a*d, c, b)
+  int tma_part;     // b % 4 == 0: partial tiles leave through TMA
+  int* status;
+};
+
+constexpr int kSplitWarpsWF = 6;
+constexpr int kThreadsWF = (2 + kSplitWarpsWF + 8) * 32;
+constexpr int kFlush = 16;  // chunks per accumulator buffer
+
+__device__ __forceinline__ void umma_tf32_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                             uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// the part of an fp32 value that a tf32 operand does not hold
+__device__ __forceinline__ uint32_t lo_of(uint32_t v) {
+  return __float_as_uint(__uint_as_float(v) - __uint_as_float(v & 0xFFFFE000u));
+}
+
+template <int NT, int ST>
+struct CfgWF {
+  static constexpr int X_BYTES = 128 * 128;  // 128 k x 32 batch entries (either order)
+  static constexpr int G_BYTES = NT * 128;   // NT j x 32 batch entries
+  static constexpr int G_OFF = 2 * X_BYTES;
+  static constexpr int STAGE_BYTES = 2 * X_BYTES + 2 * G_BYTES;
+  static constexpr int NBAR = 3 * ST + 4;
+  static constexpr int BAR_BYTES = 256;
+  static constexpr int SMEM_BYTES = ST * STAGE_BYTES + BAR_BYTES + 1024;
+  static constexpr int BUF_COLS = 2 * NT;  // leading accumulator | small-terms accumulator
+  static constexpr int TMEM_COLS = 2 * BUF_COLS;
+  static_assert(NT == 64 || NT == 128, "j tile");
+  static_assert(SMEM_BYTES <= 232448, "shared memory budget");
+  static_assert(SMEM_BYTES > 116 * 1024, "one CTA per SM, so that the TMEM allocation never waits");
+  static_assert(8 * NBAR + 16 <= BAR_BYTES, "barrier area");
+};
+
+template <bool X_LAST, bool G_LAST, int NT, int ST>
+__global__ void __launch_bounds__(kThreadsWF, 1)
+    ksmm_tc_wgrad_f32_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmG,
+                             const __grid_constant__ CUtensorMap tmP, const ParamsWF P) {
+  using C = CfgWF<NT, ST>;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = smem_u32(smem_raw);
+  const uint32_t sm0 = (raw + 1023u) & ~1023u;
+  uint8_t* sm_gen = smem_raw + (sm0 - raw);
+  const uint32_t stage0 = sm0;
+  const uint32_t bar0 = stage0 + ST * C::STAGE_BYTES;
+  uint8_t* bar_gen = sm_gen + ST * C::STAGE_BYTES;
+  auto full_bar = [&](int s) { return bar0 + 8u * s; };             // TMA: raw tiles landed
+  auto split_bar = [&](int s) { return bar0 + 8u * (ST + s); };     // splitters: lo tiles written
+  auto free_bar = [&](int s) { return bar0 + 8u * (2 * ST + s); };  // MMA commit: stage consumed
+  auto tfull_bar = [&](int q) { return bar0 + 8u * (3 * ST + q); };
+  auto tempty_bar = [&](int q) { return bar0 + 8u * (3 * ST + 2 + q); };
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_gen + 8 * C::NBAR);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(bar_gen + 8 * C::NBAR + 4);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < ST; ++s) {
+      mbar_init(full_bar(s), 1);
+      mbar_init(split_bar(s), kSplitWarpsWF);
+      mbar_init(free_bar(s), 1);
+    }
+    for (int q = 0; q < 2; ++q) {
+      mbar_init(tfull_bar(q), 1);
+      mbar_init(tempty_bar(q), 8);
+    }
+    *abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == 0 && lane == 0) {
+    prefetch_tensormap(&tmX);
+    prefetch_tensormap(&tmG);
+    prefetch_tensormap(&tmP);
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), C::TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  // everything above overlaps the tail of the previous kernel in the stream; memory comes after this
+  grid_dep_wait();
+  grid_dep_launch();
+
+  uint32_t t = blockIdx.x;
+  const int tj = static_cast<int>(t % P.tiles_j); t /= P.tiles_j;
+  const int tk = static_cast<int>(t % P.tiles_k); t /= P.tiles_k;
+  const int sp = static_cast<int>(t % P.splits);
+  const int blk = static_cast<int>(t / P.splits);
+  const int i = blk / P.d, l = blk % P.d;
+  const int k0 = tk * 128, j0 = tj * NT;
+  const int ch_begin = static_cast<int>(static_cast<int64_t>(sp) * P.nchunks / P.splits);
+  const int ch_end = static_cast<int>(static_cast<int64_t>(sp + 1) * P.nchunks / P.splits);
+
+  if (warp == 0) {
+    // ===================== TMA producer =====================
+    if (lane == 0) {
+      uint32_t si = 0, sph = 0;
+      for (int ch = ch_begin; ch < ch_end; ++ch) {
+        if (!mbar_wait<64>(free_bar(si), sph ^ 1u, abort_flag, P.status, 61)) break;
+        const uint32_t dst = stage0 + si * C::STAGE_BYTES;
+        const uint32_t bar = full_bar(si);
+        mbar_expect_tx(bar, C::X_BYTES + C::G_BYTES);
+        const int n0 = ch * 32;
+        if constexpr (X_LAST) tma_load_4d(dst, &tmX, bar, n0, l, k0, i);
+        else tma_load_4d(dst, &tmX, bar, 0, n0, k0 / 32, blk);
+        if constexpr (G_LAST) tma_load_4d(dst + C::G_OFF, &tmG, bar, n0, l, j0, i);
+        else tma_load_4d(dst + C::G_OFF, &tmG, bar, 0, n0, j0 / 32, blk);
+        if (++si == ST) { si = 0; sph ^= 1u; }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ===================== MMA issuer =====================
+    if (lane == 0) {
+      uint32_t si = 0, sph = 0, ut = 0;
+      bool ok = true;
+      for (int ch = ch_begin; ch < ch_end && ok; ++ut) {
+        const uint32_t buf = ut & 1u, bph = (ut >> 1) & 1u;
+        if (!mbar_wait<0>(tempty_bar(buf), bph ^ 1u, abort_flag, P.status, 62)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t dcol = tmem_base + buf * C::BUF_COLS, dsmall = dcol + NT;
+        const int stop = min(ch + kFlush, ch_end);
+        for (bool first = true; ch < stop; ++ch, first = false) {
+          if (!mbar_wait<0>(split_bar(si), sph, abort_flag, P.status, 63)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t xb = stage0 + si * C::STAGE_BYTES, gb = xb + C::G_OFF;
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks) {
+            // K-major rows of 32 entries: a k step is 32 bytes inside the row; MN-major atoms of 32
+            // features: 4 KB between atoms, 512 bytes between groups of 4 batch rows
+            const uint64_t xhi = X_LAST ? make_desc(xb + ks * 32, 16, 1024, 2) : make_desc(xb + ks * 1024, 4096, 512, 1);
+            const uint64_t xlo = X_LAST ? make_desc(xb + C::X_BYTES + ks * 32, 16, 1024, 2)
+                                        : make_desc(xb + C::X_BYTES + ks * 1024, 4096, 512, 1);
+            const uint64_t gst = G_LAST ? make_desc(gb + ks * 32, 16, 1024, 2) : make_desc(gb + ks * 1024, 4096, 512, 1);
+            // hi(x) * [hi(g) | lo(g)]: the leading accumulator and, next to it, the small one
+            umma_tf32_ss(dcol, xhi, gst, P.idesc2, (first && ks == 0) ? 0u : 1u);
+            // lo(x) * hi(g): only the first NT rows of the same operand
+            umma_tf32_ss(dsmall, xlo, gst, P.idesc, 1u);
+          }
+          umma_commit(free_bar(si));
+          if (++si == ST) { si = 0; sph ^= 1u; }
+        }
+        if (ok) umma_commit(tfull_bar(buf));
+      }
+    }
+    __syncwarp();
+  } else if (warp < 2 + kSplitWarpsWF) {
+    // ===================== splitters =====================
+    const int tt = (warp - 2) * 32 + lane;
+    constexpr int kXP = C::X_BYTES / 16, kP = (C::X_BYTES + C::G_BYTES) / 16;
+    uint32_t si = 0, sph = 0;
+    for (int ch = ch_begin; ch < ch_end; ++ch) {
+      int got = 1;
+      if (lane == 0) got = mbar_wait<32>(full_bar(si), sph, abort_flag, P.status, 64) ? 1 : 0;
+      got = __shfl_sync(0xffffffffu, got, 0);
+      if (!got) break;
+      const uint32_t sb = stage0 + si * C::STAGE_BYTES;
+#pragma unroll 4
+      for (int pc = tt; pc < kP; pc += kSplitWarpsWF * 32) {
+        const bool on_g = pc >= kXP;
+        const uint32_t hb = sb + (on_g ? C::G_OFF + (pc - kXP) * 16 : pc * 16);
+        const uint32_t lb = hb + (on_g ? C::G_BYTES : C::X_BYTES);
+        uint32_t v[4];
+        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                     : "r"(hb)
+                     : "memory");
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(lb), "r"(lo_of(v[0])), "r"(lo_of(v[1])),
+                     "r"(lo_of(v[2])), "r"(lo_of(v[3]))
+                     : "memory");
+      }
+      fence_proxy_async();  // the tiles are read by the tensor core through the async proxy
+      __syncwarp();
+      if (lane == 0) mbar_arrive(split_bar(si));
+      if (++si == ST) { si = 0; sph ^= 1u; }
+    }
+    __syncwarp();
+  } else {
+    // ===================== epilogue =====================
+    // lane = accumulator row k, NT / 2 columns per warp, summed in registers over the buffers
+    const int q = warp & 3, h = (warp - 2 - kSplitWarpsWF) >> 2;
+    const uint32_t tm = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + h * (NT / 2);
+    float acc[NT / 2];
+#pragma unroll
+    for (int e = 0; e < NT / 2; ++e) acc[e] = 0.f;
+    bool ok = true;
+    uint32_t ut = 0;
+    for (int ch = ch_begin; ch < ch_end; ch += kFlush, ++ut) {
+      const uint32_t buf = ut & 1u, bph = (ut >> 1) & 1u;
+      int got = 1;
+      if (lane == 0) got = mbar_wait<128>(tfull_bar(buf), bph, abort_flag, P.status, 65) ? 1 : 0;
+      got = __shfl_sync(0xffffffffu, got, 0);
+      if (!got) { ok = false; break; }
+      tc_fence_after();
+#pragma unroll
+      for (int cg = 0; cg < NT / 2; cg += 16) {
+        uint32_t r[16], rs[16];
+        tmem_ld16(tm + buf * C::BUF_COLS + cg, r);
+        tmem_ld16(tm + buf * C::BUF_COLS + NT + cg, rs);
+        tmem_ld_wait();
+#pragma unroll
+        for (int e = 0; e < 16; ++e) acc[cg + e] += __uint_as_float(r[e]) + __uint_as_float(rs[e]);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(tempty_bar(buf));
+    }
+    const int krow0 = k0 + q * 32;
+    if (ok && krow0 < P.c) {
+      // the last buffer is complete, so every stage has been consumed: the ring is free for staging
+      const int pz = sp * P.a * P.d + blk;
+#pragma unroll
+      for (int cg = 0; cg < NT / 64; ++cg) {
+        const int jc = j0 + h * (NT / 2) + cg * 32;
+        if (jc >= P.b) break;
+        if (P.tma_part) {
+          const uint32_t stg = stage0 + ((warp - 2 - kSplitWarpsWF) * 2 + cg) * 4096;
+#pragma unroll
+          for (int c4 = 0; c4 < 8; ++c4)
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stg + lane * 128 + ((c4 ^ (lane & 7)) << 4)),
+                         "r"(__float_as_uint(acc[cg * 32 + c4 * 4])), "r"(__float_as_uint(acc[cg * 32 + c4 * 4 + 1])),
+                         "r"(__float_as_uint(acc[cg * 32 + c4 * 4 + 2])), "r"(__float_as_uint(acc[cg * 32 + c4 * 4 + 3]))
+                         : "memory");
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_3d(&tmP, stg, jc, krow0, pz);
+            bulk_commit();
+          }
+        } else if (krow0 + lane < P.c) {
+          float* row = P.part + (static_cast<int64_t>(pz) * P.c + krow0 + lane) * P.b + jc;
+#pragma unroll
+          for (int e = 0; e < 32; ++e)
+            if (jc + e < P.b) row[e] = acc[cg * 32 + e];
+        }
+      }
+      if (lane == 0) bulk_wait<0>();
+    }
+    __syncwarp();
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (*abort_flag) {
+    __nanosleep(20000);
+    __syncthreads();
+  }
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, C::TMEM_COLS);
+  }
+}
+
+template <bool X_LAST, bool G_LAST, int NT, int ST>
+static int launch_wf(const Problem& p, const WgradOperand& x, const WgradOperand& g, float* part, int splits,
+                     cudaStream_t stream) {
+  using C = CfgWF<NT, ST>;
+  auto kern = ksmm_tc_wgrad_f32_kernel<X_LAST, G_LAST, NT, ST>;
+  static std::atomic<bool> attr_set[64];  // zero-initialised; set once per device (a repeated set is harmless)
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
+    if (e != cudaSuccess)
+      return set_error(KSMM_ERR_CUDA, "cannot reserve %d bytes of shared memory: %s", C::SMEM_BYTES,
+                       cudaGetErrorString(e));
+    attr_set[dev] = true;
+  }
+  const uint64_t a = p.a, b = p.b, c = p.c, d = p.d, B = p.batch;
+  CUtensorMap tmX, tmG, tmP;
+  int st;
+  auto operand_map = [&](CUtensorMap* tm, bool last, const WgradOperand& o, uint64_t f, uint32_t rows) {
+    if (last) {
+      // (batch, d, features, a): 32 batch entries x `rows` features per box
+      const uint64_t L = o.ld;
+      const uint64_t dims[4] = {B, d, f, a}, str[4] = {1, L, d * L, f * d * L};
+      const uint32_t box[4] = {32, 1, rows, 1};
+      return encode_map(tm, KSMM_F32, 4, o.ptr, dims, str, box, true, false);
+    }
+    // d = 1: (feature % 32, batch, feature / 32, a): rows / 32 atoms of 32 features x 32 batch rows
+    const uint64_t dims[4] = {32, B, f / 32, a}, str[4] = {1, a * f, 32, f};
+    const uint32_t box[4] = {32, 32, rows / 32, 1};
+    return encode_map(tm, KSMM_F32, 4, o.ptr, dims, str, box, true, true);
+  };
+  if ((st = operand_map(&tmX, X_LAST, x, c, 128)) != KSMM_OK) return st;
+  if ((st = operand_map(&tmG, G_LAST, g, b, NT)) != KSMM_OK) return st;
+  ParamsWF P;
+  P.a = p.a; P.b = p.b; P.c = p.c; P.d = p.d;
+  P.tiles_k = (p.c + 127) / 128;
+  P.tiles_j = (p.b + NT - 1) / NT;
+  P.splits = splits;
+  P.nchunks = static_cast<int>((p.batch + 31) / 32);
+  P.part = part;
+  P.tma_part = p.b % 4 == 0 ? 1 : 0;
+  tmP = tmX;  // unused otherwise
+  if (P.tma_part) {
+    const uint64_t dims[3] = {b, c, static_cast<uint64_t>(splits) * a * d}, str[3] = {1, b, b * c};
+    const uint32_t box[3] = {32, 32, 1};
+    if ((st = encode_map(&tmP, KSMM_F32, 3, part, dims, str, box)) != KSMM_OK) return st;
+  }
+  P.status = status_word();
+  if (!P.status) return set_error(KSMM_ERR_CUDA, "cannot resolve the device status word");
+  // fp32 accumulate, tf32 operands, M = 128; batch-last operands are K-major, batch-first ones MN-major
+  const uint32_t common = (1u << 4) | (2u << 7) | (2u << 10) | (X_LAST ? 0u : 1u << 15) | (G_LAST ? 0u : 1u << 16) |
+                          (static_cast<uint32_t>(128 >> 4) << 24);
+  P.idesc = common | (static_cast<uint32_t>(NT >> 3) << 17);
+  P.idesc2 = common | (static_cast<uint32_t>(2 * NT >> 3) << 17);
+  const int64_t grid = static_cast<int64_t>(p.a) * p.d * splits * P.tiles_k * P.tiles_j;
+  if (grid <= 0 || grid > 0x7fffffffLL)
+    return set_error(KSMM_ERR_UNSUPPORTED, "weight gradient: %lld tiles exceed the grid limit",
+                     static_cast<long long>(grid));
+  cudaError_t err = launch_pdl(kern, static_cast<unsigned>(grid), kThreadsWF, C::SMEM_BYTES, stream, tmX, tmG, tmP, P);
+  count_launch();
+  if (err == cudaSuccess) err = cudaGetLastError();
+  if (err != cudaSuccess)
+    return set_error(KSMM_ERR_CUDA, "weight-gradient kernel launch failed: %s", cudaGetErrorString(err));
+  return KSMM_OK;
+}
+
+template <bool X_LAST, bool G_LAST>
+static int launch_wf_tile(const Problem& p, const WgradOperand& x, const WgradOperand& g, float* part, int nt,
+                          int splits, cudaStream_t stream) {
+  return nt == 64 ? launch_wf<X_LAST, G_LAST, 64, 4>(p, x, g, part, splits, stream)
+                  : launch_wf<X_LAST, G_LAST, 128, 3>(p, x, g, part, splits, stream);
+}
+
+}  // namespace tc
+
+int wgrad_f32_launch(const Problem& p, const WgradOperand& x, const WgradOperand& g, float* part, int nt, int splits,
+                     cudaStream_t stream) {
+  if (x.last)
+    return g.last ? tc::launch_wf_tile<true, true>(p, x, g, part, nt, splits, stream)
+                  : tc::launch_wf_tile<true, false>(p, x, g, part, nt, splits, stream);
+  return g.last ? tc::launch_wf_tile<false, true>(p, x, g, part, nt, splits, stream)
+                : tc::launch_wf_tile<false, false>(p, x, g, part, nt, splits, stream);
+}
+
+}  // namespace ksmm

@@ -1247,3 +1247,27 @@ def test_tc_family_batch_first_groups_of_eight_blocks(dtype):
         ref = _act_ref(0.5 * _oracle(x, w, False) + bias.float().numpy()[None, :], "gelu")
         assert ko.rel_fro_error(y, ref) < TOL[dtype], pattern
     kb.check_device()
+
+
+# ---------------------------------------------------------------------------
+# weight gradients: tile edges, ragged batches, operands that need a padded or transposed copy
+# ---------------------------------------------------------------------------
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("bs_last", [True, False])
+@pytest.mark.parametrize("pattern", [(1, 50, 70, 2), (2, 64, 129, 1), (1, 260, 96, 3), (3, 16, 16, 1), (1, 96, 300, 1)])
+def test_weight_gradient_edges(pattern, bs_last, dtype):
+    """Batches of one chunk, of an odd length and of many accumulator flushes.  Tolerances: fp32 the
+    1e-5 of the forward, 16-bit results one rounding step of the output (2^-11, 2^-8)."""
+    a, b, c, d = pattern
+    tol = {torch.float32: 1e-5, torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}[dtype]
+    for batch in (1, 33, 1001, 20011):
+        gen = torch.Generator(device=DEV).manual_seed(batch)
+        n_in, n_out = a * c * d, a * b * d
+        x = torch.randn((n_in, batch) if bs_last else (batch, n_in), device=DEV, generator=gen).to(dtype)
+        g = torch.randn((n_out, batch) if bs_last else (batch, n_out), device=DEV, generator=gen).to(dtype)
+        dw = kb.backward_weights(x, g, bs_last, a, b, c, d)
+        xt, gt = (x, g) if bs_last else (x.t(), g.t())
+        ref = torch.einsum("ikln,ijln->ilkj", xt.double().reshape(a, c, d, batch), gt.double().reshape(a, b, d, batch))
+        ref = ref.reshape(a * d * c, b)
+        assert (torch.linalg.norm(dw.double() - ref) / torch.linalg.norm(ref)).item() < tol, batch
+    kb.check_device()
