@@ -498,6 +498,7 @@ WgradPlan plan_wgrad(const Problem& p, const WgradOperand& x, const WgradOperand
   if (p.batch <= 0 || p.batch > 0x7fffffffLL) return w;
   const bool f32 = p.in_dtype == KSMM_F32;
   if (!f32 && p.in_dtype != KSMM_F16 && p.in_dtype != KSMM_BF16) return w;
+  if (f32 && p.batch < 128) return w;  // the FFMA kernel is the more exact one there (tc_wgrad_f32.cu)
   w.copy_x = !wgrad_operand_direct(p, x, p.c, check_pointers);
   w.copy_g = !wgrad_operand_direct(p, g, p.b, check_pointers);
   // The padding of a tile is all the work there is for blocks of a few rows; the FFMA kernel, one CTA

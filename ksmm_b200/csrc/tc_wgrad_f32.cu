@@ -1,25 +1,29 @@
 // fp32 weight gradients on the tensor cores:
 //   dW[i,j,k,l] = sum_n dY4[i,j,l,n] X4[i,k,l,n],
-// a*d independent (c x B) @ (B x b) products, each term as three tf32 products (see tc_f32x3.cu for the
-// split and its error): hi(x) hi(g) + lo(x) hi(g) + hi(x) lo(g) with fp32 accumulation.
+// a*d independent (c x B) @ (B x b) products, each term as three tf32 products:
+// hi(x) hi(g) + lo(x) hi(g) + hi(x) lo(g) with fp32 accumulation; hi is the value rounded to a tf32
+// operand, lo the rest.  (An infinite gradient gives NaN, its rest being inf - inf.)
 //
 // Accumulator rows are k (128 per tile), columns j (NT = 64 or 128), the K dimension of the MMAs is
-// the batch, 32 entries per stage.  A stage holds [X hi | X lo | G hi | G lo]; the raw tiles that TMA
-// delivers are the hi operands as they stand, six splitter warps add the lo tiles at the same
-// offsets.  G lo follows G hi directly, so the two are one operand of 2 NT rows.  A batch-last operand
+// the batch, 32 entries per stage.  A stage holds [X hi | X lo | G hi | G lo]; six splitter warps round
+// the raw tiles that TMA delivers in place and add the lo tiles at the same offsets.  G lo follows G hi directly, so the two are one operand of 2 NT rows.  A batch-last operand
 // has rows of consecutive batch entries: K-major, plain 128-byte swizzle.  A batch-first one (d = 1)
 // has rows of consecutive features: MN-major, atoms of 32 features x 32 batch rows with the 128-byte
 // swizzle of 32-byte pieces.  The split is element-wise, so any combination of the two works.
 //
 // The contraction is long (a training batch), and the tensor core truncates when it adds into its
-// accumulator, once per step of 8 entries.  So the accumulator only ever sums kFlush chunks (512
-// entries, 64 additions, the error of a forward factor with c = 512); the epilogue warps then add it,
-// rounded to nearest, to sums in registers, while the MMAs fill the other accumulator buffer.
+// accumulator, once per step of 8 entries.  So the accumulator only ever sums kFlush chunks (128
+// entries, 16 additions); the epilogue warps then add it, rounded to nearest, to sums in registers,
+// while the MMAs fill the other accumulator buffer.  Relative error against 64 bits for N(0,1) operands
+// (the FFMA kernel's in brackets): 1.8e-7 (1.8e-7) at 100 entries, 2.0e-7 (3.2e-7) at 320, 3.5e-7
+// (1.4e-6) at 6272.  With hi cut off instead of rounded and a flush every 512 entries it was 4.8e-7,
+// 4.9e-7 and 1.5e-6.  Below 128 entries the FFMA kernel runs: its few roundings are the smaller error.
 //
 // What bounds it: the shared-memory pipe.  A chunk of 32 entries (NT = 128) is written once by TMA
-// (32 KB), read and written by the splitters (64 KB) and read by the MMAs (80 KB), about 1400
+// (32 KB), read and written twice by the splitters (96 KB) and read by the MMAs (80 KB), about 1660
 // cycles at 128 bytes a cycle against 1080 for its eight MMAs.  The batch is split over CTAs as in
-// backward.cu; (1,768,192,2) at 6272 batch entries: 485 us on the FFMA kernel before.
+// backward.cu; (1,768,192,2) at 6272 batch entries: 49 us (485 us on the FFMA kernel, 47 us without
+// the second write of the splitters).
 //
 // Roles (512 threads): warp 0 TMA producer, warp 1 TMEM owner and MMA issuer, warps 2..7 splitters,
 // warps 8..15 epilogue.  Waits are bounded and report through the device status word.
@@ -48,7 +52,7 @@ struct ParamsWF {
 
 constexpr int kSplitWarpsWF = 6;
 constexpr int kThreadsWF = (2 + kSplitWarpsWF + 8) * 32;
-constexpr int kFlush = 16;  // chunks per accumulator buffer
+constexpr int kFlush = 4;  // chunks per accumulator buffer
 
 __device__ __forceinline__ void umma_tf32_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                              uint32_t accumulate) {
@@ -58,9 +62,14 @@ __device__ __forceinline__ void umma_tf32_ss(uint32_t d_tmem, uint64_t adesc, ui
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// the part of an fp32 value that a tf32 operand does not hold
-__device__ __forceinline__ uint32_t lo_of(uint32_t v) {
-  return __float_as_uint(__uint_as_float(v) - __uint_as_float(v & 0xFFFFE000u));
+// v = hi + lo: hi the nearest value with the 11 significant bits of a tf32 operand (towards zero where
+// rounding would leave the range), lo the exact rest, at most 12 bits of which the tensor core drops one
+__device__ __forceinline__ uint32_t hi_of(uint32_t v) {
+  const uint32_t r = (v & 0x7fffffffu) < 0x7f7ff000u ? v + 0x1000u : v;
+  return r & 0xFFFFE000u;
+}
+__device__ __forceinline__ uint32_t rest_of(uint32_t v, uint32_t hi) {
+  return __float_as_uint(__uint_as_float(v) - __uint_as_float(hi));
 }
 
 template <int NT, int ST>
@@ -215,8 +224,11 @@ __global__ void __launch_bounds__(kThreadsWF, 1)
                      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
                      : "r"(hb)
                      : "memory");
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(lb), "r"(lo_of(v[0])), "r"(lo_of(v[1])),
-                     "r"(lo_of(v[2])), "r"(lo_of(v[3]))
+        const uint32_t h0 = hi_of(v[0]), h1 = hi_of(v[1]), h2 = hi_of(v[2]), h3 = hi_of(v[3]);
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(hb), "r"(h0), "r"(h1), "r"(h2), "r"(h3)
+                     : "memory");
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(lb), "r"(rest_of(v[0], h0)),
+                     "r"(rest_of(v[1], h1)), "r"(rest_of(v[2], h2)), "r"(rest_of(v[3], h3))
                      : "memory");
       }
       fence_proxy_async();  // the tiles are read by the tensor core through the async proxy

@@ -1271,3 +1271,22 @@ def test_weight_gradient_edges(pattern, bs_last, dtype):
         ref = ref.reshape(a * d * c, b)
         assert (torch.linalg.norm(dw.double() - ref) / torch.linalg.norm(ref)).item() < tol, batch
     kb.check_device()
+
+
+@pytest.mark.parametrize("bs_last", [True, False])
+@pytest.mark.parametrize("pattern", [(1, 64, 64, 1), (1, 160, 96, 2)])
+def test_weight_gradient_fp32_error(pattern, bs_last):
+    """fp32 sums, not tf32 ones.  Bound: 16 truncated additions (half a unit of 2^-23 each on average, of
+    partial sums below the segment's) and the dropped lo * lo (2^-24) stay under 16 * 2^-25 = 4.8e-7 of the
+    result's norm at every length; the shorter batches, summed by FFMAs, are below it as well."""
+    a, b, c, d = pattern
+    for batch in (16, 127, 128, 321, 12544):
+        gen = torch.Generator(device=DEV).manual_seed(batch)
+        x = torch.randn(a * c * d, batch, device=DEV, generator=gen)
+        g = torch.randn(a * b * d, batch, device=DEV, generator=gen)
+        ref = torch.einsum("ikln,ijln->ilkj", x.double().reshape(a, c, d, batch), g.double().reshape(a, b, d, batch))
+        x, g = (x, g) if bs_last else (x.t().contiguous(), g.t().contiguous())
+        dw = kb.backward_weights(x, g, bs_last, a, b, c, d)
+        err = torch.linalg.norm(dw.double() - ref.reshape(a * d * c, b)) / torch.linalg.norm(ref)
+        assert err.item() < 4.8e-7, (batch, err.item())
+    kb.check_device()
