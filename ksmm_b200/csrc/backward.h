@@ -25,10 +25,11 @@ int wgrad_launch(const Problem& p, WgradOperand x, WgradOperand g, void* workspa
 int wgrad_f32_launch(const Problem& p, const WgradOperand& x, const WgradOperand& g, float* part, int nt, int splits,
                      cudaStream_t stream);
 
-// in: rows x cols row-major, out: cols x rows with row stride out_ld (0 = rows)
+// in: rows x cols with row stride in_ld (0 = cols), out: cols x rows with row stride out_ld (0 = rows)
 int launch_transpose(const void* in, void* out, int64_t rows, int64_t cols, int es, cudaStream_t stream,
-                     int64_t out_ld = 0);
-// rows x cols from row stride in_ld to row stride out_ld (elements of es bytes)
+                     int64_t out_ld = 0, int64_t in_ld = 0);
+// rows x cols from row stride in_ld to row stride out_ld (elements of es bytes); rows of the destination
+// are aligned to 16 bytes
 int launch_copy_rows(const void* in, int64_t in_ld, void* out, int64_t out_ld, int64_t rows, int64_t cols, int es,
                      cudaStream_t stream);
 

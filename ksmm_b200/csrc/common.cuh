@@ -138,6 +138,7 @@ struct Problem {
   // Row strides in elements of a batch-last input / output; 0 = the batch.  Intermediates whose batch
   // is not a whole number of 16-byte pieces have padded rows, so that tensor maps can address them.
   int64_t in_ld = 0, out_ld = 0;
+  int no_pad = 0;  // 1: copies and intermediates keep rows of exactly the batch (what fits without padding)
   float alpha;
   // Chains only.  out_regroup_d > 0: store the output regrouped by the blocks of the next factor
   // (c = out_regroup_c, d = out_regroup_d): feature (i2*c + k)*d + l goes to (i2*d + l)*c + k.
@@ -169,6 +170,10 @@ __host__ __device__ inline int64_t out_stride(const Problem& p) { return p.out_l
 inline bool has_padded_rows(const Problem& p) {
   return (in_is_last(p) && in_stride(p) != p.batch) || (out_is_last(p) && out_stride(p) != p.batch);
 }
+
+// Row stride of the library's own batch-last copies and intermediates: the batch where its rows are
+// whole 16-byte pieces, else the next multiple of 64 entries.
+inline int64_t padded_ld(int64_t batch, int es) { return (batch * es) % 16 == 0 ? batch : (batch + 63) / 64 * 64; }
 
 // element-wise epilogue function (ksmm_activation_t)
 // erf by the rational approximation 7.1.26 of Abramowitz and Stegun (absolute error below

@@ -37,6 +37,8 @@ struct Params {
   float alpha;
   const float* bias;
   float* out;
+  int64_t out_ld;  // row stride of the output
+  int yvec;        // output rows start on 16-byte boundaries
   int* status;
 };
 
@@ -169,7 +171,15 @@ __global__ void __launch_bounds__(WJ * 128, 512 / (WJ * 128))
         v.y = fmaf(P.alpha, acc[m][half * 4 + 1], bv);
         v.z = fmaf(P.alpha, acc[m][half * 4 + 2], bv);
         v.w = fmaf(P.alpha, acc[m][half * 4 + 3], bv);
-        *reinterpret_cast<float4*>(P.out + row * B + gn) = v;
+        float* y = P.out + row * P.out_ld + gn;
+        if (P.yvec && gn + 4 <= B) {
+          *reinterpret_cast<float4*>(y) = v;
+        } else {
+          y[0] = v.x;
+          if (gn + 1 < B) y[1] = v.y;
+          if (gn + 2 < B) y[2] = v.z;
+          if (gn + 3 < B) y[3] = v.w;
+        }
       }
     }
   }
@@ -195,7 +205,8 @@ static int launch(const Problem& p, cudaStream_t stream) {
   int st;
   {
     const uint64_t dims[4] = {B, d, c, a};
-    const uint64_t str[4] = {1, B, d * B, c * d * B};
+    const uint64_t L = in_stride(p);
+    const uint64_t str[4] = {1, L, d * L, c * d * L};
     const uint32_t box[4] = {static_cast<uint32_t>(C::TN), 1, static_cast<uint32_t>(C::KC), 1};
     if ((st = encode_map(&tmX, KSMM_F32, 4, p.in, dims, str, box, false)) != KSMM_OK) return st;
   }
@@ -214,6 +225,8 @@ static int launch(const Problem& p, cudaStream_t stream) {
   P.alpha = p.alpha;
   P.bias = static_cast<const float*>(p.bias);
   P.out = static_cast<float*>(p.out);
+  P.out_ld = out_stride(p);
+  P.yvec = rows_addressable(p.out, out_stride(p), 4) ? 1 : 0;
   P.status = status_word();
   if (!P.status) return set_error(KSMM_ERR_CUDA, "cannot resolve the device status word");
   const int64_t total = static_cast<int64_t>(P.tiles_n) * P.tiles_j * p.a * p.d;
@@ -232,11 +245,12 @@ static int launch(const Problem& p, cudaStream_t stream) {
 
 bool ffma_tma_supported(const Problem& p, bool check_pointers) {
   if (p.in_dtype != KSMM_F32 || p.out_dtype != KSMM_F32 || !p.bs_last) return false;
-  if (has_padded_rows(p)) return false;
-  if (p.batch <= 0 || p.batch > 0x7fffffffLL || p.batch % 4 != 0 || p.b % 4 != 0) return false;
+  if (p.out_bs_last == 0) return false;
+  // input rows are 16-byte multiples (of the batch, or padded to that); output rows may start anywhere
+  if (p.batch <= 0 || p.batch > 0x7fffffffLL || in_stride(p) % 4 != 0 || p.b % 4 != 0) return false;
   if (check_pointers) {
     if (reinterpret_cast<uintptr_t>(p.in) % 16 || reinterpret_cast<uintptr_t>(p.w) % 16 ||
-        reinterpret_cast<uintptr_t>(p.out) % 16)
+        reinterpret_cast<uintptr_t>(p.out) % 4)
       return false;
   }
   return true;

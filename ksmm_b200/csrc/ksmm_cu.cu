@@ -258,15 +258,26 @@ static bool conversion_possible(const Problem& p) {
   return p.batch <= 0x7fffffffLL;
 }
 
+// the batch-last problem inside a conversion: operands in the scratch (aligned to 256 bytes), rows padded
+// where the batch is not a whole number of 16-byte pieces
+static Problem batch_last_twin(const Problem& p) {
+  Problem q = p;
+  q.bs_last = 1;
+  q.in = q.out = reinterpret_cast<void*>(256);
+  q.in_ld = p.no_pad ? 0 : padded_ld(p.batch, dtype_size(p.in_dtype));
+  q.out_ld = p.no_pad ? 0 : padded_ld(p.batch, dtype_size(p.out_dtype));
+  q.scratch = nullptr;
+  q.scratch_bytes = 0;
+  return q;
+}
+
 // the heuristic: conversion pays when no direct kernel covers the factor and the batch-last
 // kernel is a tensor-core (or TMA-staged FFMA) one
 static bool conversion_applies(const Problem& p) {
   if (!conversion_possible(p)) return false;
   if (reinterpret_cast<uintptr_t>(p.w) % 16 != 0) return false;
   if (p.in_dtype == KSMM_F32) {
-    Problem q = p;
-    q.bs_last = 1;
-    q.in = q.out = reinterpret_cast<void*>(256);  // alignment is that of the scratch (256 bytes)
+    Problem q = batch_last_twin(p);
     // for compute-heavy blocks the batch-last tensor-core kernel pays for the two transposes;
     // small blocks are bandwidth problems that the direct FFMA kernel (d = 2, 4) serves better
     // (tuned at 25088 rows: (1,256,64,4) 89 us through the conversion against 109 us direct)
@@ -275,9 +286,7 @@ static bool conversion_applies(const Problem& p) {
     if (direct) return false;
     return q.b >= 48 && ffma_tma_supported(q, false);
   }
-  Problem q = p;
-  q.bs_last = 1;
-  q.in = q.out = reinterpret_cast<void*>(256);
+  Problem q = batch_last_twin(p);
   if (tc_default_config(p) >= 0) return false;  // a direct batch-first kernel covers it
   return q.b >= 32 && q.c >= 16 && tc_config_supported(q, 0, true);
 }
@@ -285,7 +294,32 @@ static bool conversion_applies(const Problem& p) {
 static size_t conversion_scratch_bytes(const Problem& p) {
   const int es = dtype_size(p.in_dtype), os = dtype_size(p.out_dtype);
   const size_t n_in = static_cast<size_t>(p.a) * p.c * p.d, n_out = static_cast<size_t>(p.a) * p.b * p.d;
-  return align_up(n_in * p.batch * es, 256) + align_up(n_out * p.batch * os, 256);
+  const Problem q = batch_last_twin(p);
+  return align_up(n_in * in_stride(q) * es, 256) + align_up(n_out * out_stride(q) * os, 256);
+}
+
+// ---------------------------------------------------------------------------
+// Batch-last factors whose rows are no 16-byte multiples: no tensor map can address the input.  With
+// scratch for it, the input is copied into padded rows and the kernel of an aligned batch runs; it
+// stores the output's rows where they are (they may start anywhere).  Against the register-staged
+// kernel, which takes any row: (6,64,64,1) and (1,768,192,2) fp16 at 6501 columns 191 us -> 27 us.
+// fp32 inputs take the TMA-staged FFMA kernel (the same sums in the same precision).
+// ---------------------------------------------------------------------------
+static constexpr int kAlgoPadRows = 100;  // beside the public families; never a cached choice
+
+static bool pad_rows_applies(const Problem& p) {
+  if (!p.bs_last || p.no_pad || p.in_ld || p.out_ld || p.out_bs_last >= 0 || p.groups > 1) return false;
+  if (p.batch <= 0 || p.batch > 0x7fffffffLL || (p.batch * dtype_size(p.in_dtype)) % 16 == 0) return false;
+  Problem q = p;
+  q.in = reinterpret_cast<void*>(256);
+  q.in_ld = padded_ld(p.batch, dtype_size(p.in_dtype));
+  if (p.in_dtype == KSMM_F32) return q.b >= 48 && ffma_tma_supported(q, true);
+  return tc_default_config(q) >= 0;
+}
+
+static size_t pad_rows_scratch_bytes(const Problem& p) {
+  const int es = dtype_size(p.in_dtype);
+  return align_up(static_cast<size_t>(p.a) * p.c * p.d * padded_ld(p.batch, es) * es, 256);
 }
 
 static int run_family(const Problem& p, int algo, int config, cudaStream_t stream);
@@ -296,23 +330,38 @@ static int forward_via_transpose(const Problem& p, cudaStream_t stream) {
     return set_error(KSMM_ERR_UNSUPPORTED, "the layout-conversion path serves batch-first factors with d > 1");
   const int es = dtype_size(p.in_dtype), os = dtype_size(p.out_dtype);
   const int64_t n_in = static_cast<int64_t>(p.a) * p.c * p.d, n_out = static_cast<int64_t>(p.a) * p.b * p.d;
-  const size_t in_bytes = align_up(static_cast<size_t>(n_in) * p.batch * es, 256);
+  Problem q = batch_last_twin(p);
+  if (!p.no_pad && p.scratch != nullptr && p.scratch_bytes < conversion_scratch_bytes(p)) {
+    // a scratch of the size without padding still serves
+    Problem u = p;
+    u.no_pad = 1;
+    if (p.scratch_bytes >= conversion_scratch_bytes(u)) return forward_via_transpose(u, stream);
+  }
+  const size_t in_bytes = align_up(static_cast<size_t>(n_in) * in_stride(q) * es, 256);
   void* base = nullptr;
   int stq = layout_scratch(p, conversion_scratch_bytes(p), stream, &base);
   if (stq != KSMM_OK) return stq;
-  void* xt = base;
-  void* yt = static_cast<char*>(base) + in_bytes;
-  int st = launch_transpose(p.in, xt, p.batch, n_in, es, stream);  // (batch, in) -> (in, batch)
+  q.in = base;
+  q.out = static_cast<char*>(base) + in_bytes;
+  int st = launch_transpose(p.in, base, p.batch, n_in, es, stream, in_stride(q));  // (batch, in) -> (in, batch)
   if (st != KSMM_OK) return st;
+  st = dispatch(q, KSMM_ALGO_AUTO, -1, stream);  // (with aligned rows a batch-last factor needs no scratch)
+  if (st != KSMM_OK) return st;
+  // (out, batch) -> (batch, out)
+  return launch_transpose(q.out, p.out, n_out, p.batch, os, stream, 0, out_stride(q));
+}
+
+static int forward_via_padded_rows(const Problem& p, cudaStream_t stream) {
+  const int es = dtype_size(p.in_dtype);
   Problem q = p;
-  q.in = xt;
-  q.out = yt;
-  q.bs_last = 1;
+  q.in_ld = padded_ld(p.batch, es);
+  q.in = p.scratch;
+  q.out_ld = p.batch;
   q.scratch = nullptr;
   q.scratch_bytes = 0;
-  st = dispatch(q, KSMM_ALGO_AUTO, -1, stream);  // (a batch-last factor never needs scratch)
+  int st = launch_copy_rows(p.in, p.batch, p.scratch, q.in_ld, static_cast<int64_t>(p.a) * p.c * p.d, p.batch, es, stream);
   if (st != KSMM_OK) return st;
-  return launch_transpose(yt, p.out, n_out, p.batch, os, stream);  // (out, batch) -> (batch, out)
+  return dispatch(q, KSMM_ALGO_AUTO, -1, stream);
 }
 
 static int run_family(const Problem& p, int algo, int config, cudaStream_t stream) {
@@ -326,6 +375,7 @@ static int run_family(const Problem& p, int algo, int config, cudaStream_t strea
   if (algo == KSMM_ALGO_SIMT) return simt_launch(p, config, stream);
   if (algo == KSMM_ALGO_TC) return tc_launch(p, config, stream);
   if (algo == KSMM_ALGO_CONVERT) return forward_via_transpose(p, stream);
+  if (algo == kAlgoPadRows) return forward_via_padded_rows(p, stream);
   return set_error(KSMM_ERR_BAD_ARGUMENT, "unknown kernel family %d", algo);
 }
 
@@ -346,6 +396,7 @@ static Choice auto_choice(const Problem& p) {
   if (lookup_choice(p, &ch) && choice_runnable(p, ch)) return ch;
   const int tc_cfg = tc_default_config(p);
   if (tc_cfg >= 0) return Choice{KSMM_ALGO_TC, tc_cfg};
+  if (pad_rows_applies(p)) return Choice{kAlgoPadRows, 0};
   if (conversion_applies(p)) return Choice{KSMM_ALGO_CONVERT, 0};
   return Choice{KSMM_ALGO_SIMT, -1};
 }
@@ -353,6 +404,7 @@ static Choice auto_choice(const Problem& p) {
 // layout scratch the given (family, configuration) needs for this problem
 static size_t scratch_need(const Problem& p, const Choice& ch) {
   if (ch.algo == KSMM_ALGO_CONVERT) return conversion_scratch_bytes(p);
+  if (ch.algo == kAlgoPadRows) return pad_rows_scratch_bytes(p);
   if (ch.algo == KSMM_ALGO_TC && !p.bs_last && p.d != 1 && ch.config == 1 && p.in_dtype != KSMM_F32)
     return tc_bsfirst_dp_scratch_bytes(p);
   return 0;
@@ -363,7 +415,11 @@ static int dispatch(const Problem& p, int algo, int config, cudaStream_t stream)
   if (st != KSMM_OK) return st;
   if (p.batch == 0) return KSMM_OK;  // empty batch: nothing to write
   if (algo == KSMM_ALGO_AUTO) {
-    const Choice ch = auto_choice(p);
+    Choice ch = auto_choice(p);
+    // the padded copy lives in scratch that the caller passed, or not at all
+    if (ch.algo == kAlgoPadRows && (p.scratch == nullptr || reinterpret_cast<uintptr_t>(p.scratch) % 16 ||
+                                    p.scratch_bytes < pad_rows_scratch_bytes(p)))
+      ch = Choice{KSMM_ALGO_SIMT, -1};
     return run_family(p, ch.algo, ch.config, stream);
   }
   return run_family(p, algo, config, stream);
@@ -557,10 +613,12 @@ int ksmm_cu_forward_ex(const ksmm_forward_desc_t* desc, void* stream) {
   return dispatch(problem_of(*desc), desc->algo, desc->config, static_cast<cudaStream_t>(stream));
 }
 
-// bytes of the intermediate activations of a chain (two alternating buffers from three factors on)
-static size_t chain_intermediate_bytes(int nfactors, const int32_t* patterns, int64_t batch, int dtype) {
+// bytes of the intermediate activations of a chain (two alternating buffers from three factors on);
+// `pad`: batch-last intermediates have padded rows
+static size_t chain_intermediate_bytes(int nfactors, const int32_t* patterns, int64_t batch, int dtype, int pad) {
   if (nfactors <= 1 || !patterns || batch <= 0) return 0;
   size_t mx = 0;
+  if (pad) batch = padded_ld(batch, dtype_size(dtype));
   for (int f = 0; f + 1 < nfactors; ++f) {
     const int32_t* q = patterns + 4 * f;
     size_t bytes = static_cast<size_t>(q[0]) * q[1] * q[3] * batch * dtype_size(dtype);
@@ -572,7 +630,7 @@ static size_t chain_intermediate_bytes(int nfactors, const int32_t* patterns, in
 
 size_t ksmm_cu_chain_workspace_bytes(int nfactors, const int32_t* patterns, int64_t batch,
                                      int dtype) {
-  return chain_intermediate_bytes(nfactors, patterns, batch, dtype);
+  return chain_intermediate_bytes(nfactors, patterns, batch, dtype, 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -590,14 +648,16 @@ struct ChainPlan {
   int in_last[kMax], out_last[kMax];
 };
 
-static bool can_switch_layout(const int32_t* q, int64_t batch, int dtype) {
+// (`pad`: batch-last tensors inside the chain have rows that tensor maps can address at any batch)
+static bool can_switch_layout(const int32_t* q, int64_t batch, int dtype, bool pad) {
   if (q[3] != 1 || q[1] < 32 || q[2] < 16) return false;
   if (dtype == KSMM_F32)  // the fp32 tensor kernel: 32-column atoms, c <= 1024
     return q[1] % 32 == 0 && q[2] % 4 == 0 && q[2] <= 1024 && batch % 32 == 0;
-  return (dtype == KSMM_F16 || dtype == KSMM_BF16) && q[1] % 8 == 0 && q[2] % 8 == 0 && batch % 8 == 0;
+  return (dtype == KSMM_F16 || dtype == KSMM_BF16) && q[1] % 8 == 0 && q[2] % 8 == 0 &&
+         (pad || batch % 8 == 0);
 }
 
-static double step_cost(const int32_t* q, int64_t batch, int dtype, int in_last, int out_last) {
+static double step_cost(const int32_t* q, int64_t batch, int dtype, int in_last, int out_last, bool pad) {
   const double bytes = static_cast<double>(dtype_size(dtype)) * q[0] * q[3] * (static_cast<double>(q[1]) + q[2]) * batch;
   if (dtype == KSMM_F32) {
     // The fp32 tensor kernel is compute-bound from blocks of about 64 x 64 on: its time is the larger
@@ -605,11 +665,11 @@ static double step_cost(const int32_t* q, int64_t batch, int dtype, int in_last,
     // d > 1 pays a transpose on either side of it.
     const double flops = 2.0 * q[0] * q[3] * static_cast<double>(q[1]) * q[2] * batch;
     const double kernel = bytes > flops / 35.0 ? bytes : flops / 35.0;
-    if (in_last != out_last) return can_switch_layout(q, batch, dtype) ? 1.05 * kernel : -1.0;
+    if (in_last != out_last) return can_switch_layout(q, batch, dtype, pad) ? 1.05 * kernel : -1.0;
     if (in_last || q[3] == 1) return kernel;
     return kernel + 1.5 * bytes;
   }
-  if (in_last != out_last) return can_switch_layout(q, batch, dtype) ? 1.05 * bytes : -1.0;
+  if (in_last != out_last) return can_switch_layout(q, batch, dtype, pad) ? 1.05 * bytes : -1.0;
   if (in_last || q[3] == 1) return bytes;
   if ((q[3] == 2 || q[3] == 4) && q[1] % 8 == 0 && (static_cast<int64_t>(q[2]) * q[3]) % 8 == 0)
     return 1.9 * bytes;   // in-kernel split of the interleaved blocks
@@ -619,7 +679,7 @@ static double step_cost(const int32_t* q, int64_t batch, int dtype, int in_last,
 }
 
 static void plan_chain(int nfactors, const int32_t* patterns, int64_t batch, int dtype, int in_last,
-                       int out_last, bool allow_switch, ChainPlan* plan) {
+                       int out_last, bool allow_switch, bool pad, ChainPlan* plan) {
   // default: every factor in the input's layout, a transpose at the end if the output differs
   for (int f = 0; f < nfactors && f < ChainPlan::kMax; ++f) plan->in_last[f] = plan->out_last[f] = in_last;
   plan->pre_transpose = false;
@@ -640,7 +700,7 @@ static void plan_chain(int nfactors, const int32_t* patterns, int64_t batch, int
       bool ok = true;
       for (int f = 0; f < nfactors && ok; ++f) {
         const int o = (mask >> f) & 1;
-        const double c = step_cost(patterns + 4 * f, batch, dtype, state, o);
+        const double c = step_cost(patterns + 4 * f, batch, dtype, state, o, pad);
         if (c < 0) ok = false;
         cost += c;
         state = o;
@@ -667,7 +727,7 @@ static int chain_walk(bool run, const void* input, const void* const* values, vo
                       size_t scratch_bytes, int no_alloc, int64_t batch, int nfactors,
                       const int32_t* patterns, int dtype, int bs_last, int out_bs_last, int activation,
                       cudaStream_t stream, size_t* scratch_max, int allow_switch,
-                      const void* residual = nullptr);
+                      int pad, const void* residual = nullptr);
 
 // One pass over a chain: either plans it (run == false: returns through *scratch_max the layout
 // scratch it needs under the current dispatch: transposed copies at the chain's ends plus the
@@ -676,18 +736,24 @@ static int chain_walk(bool run, const void* input, const void* const* values, vo
                       const void* bias, void* workspace, size_t inter_bytes, void* scratch,
                       size_t scratch_bytes, int no_alloc, int64_t batch, int nfactors,
                       const int32_t* patterns, int dtype, int bs_last, int out_bs_last, int activation,
-                      cudaStream_t stream, size_t* scratch_max, int allow_switch, const void* residual) {
+                      cudaStream_t stream, size_t* scratch_max, int allow_switch, int pad, const void* residual) {
   if (nfactors > ChainPlan::kMax)
     return set_error(KSMM_ERR_UNSUPPORTED, "chains of more than %d factors", ChainPlan::kMax);
   ChainPlan plan;
-  plan_chain(nfactors, patterns, batch, dtype, bs_last, out_bs_last, allow_switch != 0, &plan);
+  plan_chain(nfactors, patterns, batch, dtype, bs_last, out_bs_last, allow_switch != 0, pad != 0, &plan);
   const size_t es = dtype_size(dtype);
   const int32_t* p0 = patterns;
   const int32_t* pl = patterns + 4 * (nfactors - 1);
   const int64_t in_feats = static_cast<int64_t>(p0[0]) * p0[2] * p0[3];
   const int64_t out_feats = static_cast<int64_t>(pl[0]) * pl[1] * pl[3];
-  const size_t pre_bytes = plan.pre_transpose ? align_up(static_cast<size_t>(in_feats) * batch * es, 256) : 0;
-  const size_t post_bytes = plan.post_transpose ? align_up(static_cast<size_t>(out_feats) * batch * es, 256) : 0;
+  // row stride of the batch-last tensors between the chain's ends
+  const int64_t ld = pad ? padded_ld(batch, static_cast<int>(es)) : batch;
+  // a batch-last chain input with rows that no tensor map can address is copied into padded rows
+  // (blocks that the tensor kernels do not take read it as it is)
+  const bool pad_in = ld != batch && bs_last && !plan.pre_transpose && p0[1] >= 32 && p0[2] >= 16;
+  const size_t pre_bytes =
+      plan.pre_transpose || pad_in ? align_up(static_cast<size_t>(in_feats) * ld * es, 256) : 0;
+  const size_t post_bytes = plan.post_transpose ? align_up(static_cast<size_t>(out_feats) * ld * es, 256) : 0;
   const size_t half = nfactors == 2 ? inter_bytes : inter_bytes / 2;
   const void* cur = input;
   bool cur_regrouped = false;  // the intermediate in `cur` is regrouped by the blocks of factor f
@@ -710,7 +776,7 @@ static int chain_walk(bool run, const void* input, const void* const* values, vo
     size_t total = 0;
     int stp = chain_walk(false, nullptr, nullptr, nullptr, nullptr, nullptr, inter_bytes, nullptr, 0, 0, batch,
                          nfactors, patterns, dtype, bs_last, out_bs_last, activation, nullptr, &total,
-                         allow_switch);
+                         allow_switch, pad);
     if (stp != KSMM_OK) return stp;
     if (total > 0) {
       Problem sp;
@@ -728,7 +794,12 @@ static int chain_walk(bool run, const void* input, const void* const* values, vo
   if (plan.pre_transpose && run && batch > 0) {
     // (batch, features) -> (features, batch) or back
     int st = bs_last ? launch_transpose(input, t_pre, in_feats, batch, static_cast<int>(es), stream)
-                     : launch_transpose(input, t_pre, batch, in_feats, static_cast<int>(es), stream);
+                     : launch_transpose(input, t_pre, batch, in_feats, static_cast<int>(es), stream, ld);
+    if (st != KSMM_OK) return st;
+    cur = t_pre;
+  }
+  if (pad_in && run && batch > 0) {
+    int st = launch_copy_rows(input, batch, t_pre, ld, in_feats, batch, static_cast<int>(es), stream);
     if (st != KSMM_OK) return st;
     cur = t_pre;
   }
@@ -743,6 +814,9 @@ static int chain_walk(bool run, const void* input, const void* const* values, vo
     p.in_dtype = dtype; p.out_dtype = dtype; p.alpha = 1.f;
     p.bs_last = plan.in_last[f];
     p.out_bs_last = plan.out_last[f] == plan.in_last[f] ? -1 : plan.out_last[f];
+    if (plan.in_last[f]) p.in_ld = f > 0 || plan.pre_transpose || pad_in ? ld : batch;
+    if (plan.out_last[f]) p.out_ld = !last || plan.post_transpose ? ld : batch;
+    p.no_pad = !pad;
     p.activation = last ? activation : 0;
     // the residual has the chain output's layout: it can join the last factor's epilogue only when
     // that factor writes the final layout itself
@@ -799,7 +873,7 @@ static int chain_walk(bool run, const void* input, const void* const* values, vo
   if (plan.post_transpose && run && batch > 0) {
     // the last factor wrote the other layout into t_post
     const int last_layout = plan.out_last[nfactors - 1];
-    int st = last_layout ? launch_transpose(t_post, output, out_feats, batch, static_cast<int>(es), stream)
+    int st = last_layout ? launch_transpose(t_post, output, out_feats, batch, static_cast<int>(es), stream, 0, ld)
                          : launch_transpose(t_post, output, batch, out_feats, static_cast<int>(es), stream);
     if (st != KSMM_OK) return st;
     if (residual != nullptr) {
@@ -812,6 +886,17 @@ static int chain_walk(bool run, const void* input, const void* const* values, vo
   }
   if (scratch_max) *scratch_max = pre_bytes + post_bytes + factor_scratch_max;
   return KSMM_OK;
+}
+
+// intermediates and scratch of one form of a chain; -1 where it cannot run
+static size_t chain_need(int nfactors, const int32_t* patterns, int64_t batch, int dtype, int bs_last, int out_bs_last,
+                         int allow_switch, int pad) {
+  const size_t inter = chain_intermediate_bytes(nfactors, patterns, batch, dtype, pad);
+  size_t scratch = 0;
+  if (chain_walk(false, nullptr, nullptr, nullptr, nullptr, nullptr, inter, nullptr, 0, 0, batch, nfactors, patterns,
+                 dtype, bs_last, out_bs_last, 0, nullptr, &scratch, allow_switch, pad) != KSMM_OK)
+    return static_cast<size_t>(-1);
+  return inter + scratch;
 }
 
 static int check_chain(int nfactors, const int32_t* patterns, const void* const* values, int dtype,
@@ -852,18 +937,15 @@ size_t ksmm_cu_chain_workspace_bytes_layouts(int nfactors, const int32_t* patter
   if (nfactors <= 0 || !patterns || batch <= 0) return 0;
   const void* dummy = nullptr;
   if (check_chain(nfactors, patterns, &dummy, dtype, 0) != KSMM_OK) return 0;
-  const size_t inter = chain_intermediate_bytes(nfactors, patterns, batch, dtype);
-  // the larger of the two plans: with layout-changing factors (every pointer 16-byte aligned) and
-  // without them, so that the size holds whatever the pointers of the call turn out to be
-  size_t scratch = 0;
-  for (int allow = 0; allow < 2; ++allow) {
-    size_t need = 0;
-    if (chain_walk(false, nullptr, nullptr, nullptr, nullptr, nullptr, inter, nullptr, 0, 0, batch, nfactors,
-                   patterns, dtype, bs_last ? 1 : 0, out_bs_last ? 1 : 0, 0, nullptr, &need, allow) != KSMM_OK)
-      return 0;
-    if (need > scratch) scratch = need;
+  // the largest of the plans: with layout-changing factors (every pointer 16-byte aligned) and
+  // without them, with padded rows and without, so that the size holds whatever the call turns out to be
+  size_t most = 0;
+  for (int mode = 0; mode < 4; ++mode) {
+    const size_t need = chain_need(nfactors, patterns, batch, dtype, bs_last ? 1 : 0, out_bs_last ? 1 : 0, mode & 1, mode >> 1);
+    if (need == static_cast<size_t>(-1)) return 0;
+    if (need > most) most = need;
   }
-  return inter + scratch;
+  return most;
 }
 
 int ksmm_cu_chain_forward(const void* input, const void* const* values, void* output,
@@ -887,7 +969,16 @@ static int chain_forward_impl(const void* input, const void* const* values, void
   if (out_bs_last != 0 && out_bs_last != 1)
     return set_error(KSMM_ERR_BAD_ARGUMENT, "the output layout must be 0 (batch-first) or 1 (batch-last)");
   if (batch < 0) return set_error(KSMM_ERR_BAD_ARGUMENT, "negative batch");
-  const size_t inter = chain_intermediate_bytes(nfactors, patterns, batch, dtype);
+  // layout-changing factors go through TMA on both sides: every buffer has to be 16-byte aligned
+  auto al16 = [](const void* q) { return reinterpret_cast<uintptr_t>(q) % 16 == 0; };
+  int allow_switch = al16(input) && al16(output) && al16(workspace) && al16(residual) ? 1 : 0;
+  for (int f = 0; f < nfactors; ++f) allow_switch &= al16(values[f]) ? 1 : 0;
+  // Padded rows where the batch needs them and the workspace has room for that form and its copies;
+  // the form without needs no more than it did.
+  int pad = 0;
+  if (batch > 0 && padded_ld(batch, dtype_size(dtype)) != batch && workspace && al16(workspace))
+    pad = workspace_bytes >= chain_need(nfactors, patterns, batch, dtype, bs_last, out_bs_last, allow_switch, 1);
+  const size_t inter = chain_intermediate_bytes(nfactors, patterns, batch, dtype, pad);
   if (inter > 0 && (!workspace || workspace_bytes < inter))
     return set_error(KSMM_ERR_WORKSPACE, "chain workspace: need %zu bytes, got %zu", inter,
                      workspace_bytes);
@@ -897,15 +988,11 @@ static int chain_forward_impl(const void* input, const void* const* values, void
     scratch = static_cast<char*>(workspace) + inter;
     scratch_bytes = workspace_bytes - inter;
   }
-  // layout-changing factors go through TMA on both sides: every buffer has to be 16-byte aligned
-  auto al16 = [](const void* q) { return reinterpret_cast<uintptr_t>(q) % 16 == 0; };
-  int allow_switch = al16(input) && al16(output) && al16(workspace) && al16(residual) ? 1 : 0;
-  for (int f = 0; f < nfactors; ++f) allow_switch &= al16(values[f]) ? 1 : 0;
   if (no_alloc) {
     // refuse before the first launch, not half-way through the chain
     size_t need = 0;
     st = chain_walk(false, nullptr, nullptr, nullptr, nullptr, nullptr, inter, nullptr, 0, 0, batch,
-                    nfactors, patterns, dtype, bs_last, out_bs_last, activation, nullptr, &need, allow_switch);
+                    nfactors, patterns, dtype, bs_last, out_bs_last, activation, nullptr, &need, allow_switch, pad);
     if (st != KSMM_OK) return st;
     if (need > scratch_bytes)
       return set_error(KSMM_ERR_WORKSPACE,
@@ -915,7 +1002,7 @@ static int chain_forward_impl(const void* input, const void* const* values, void
   }
   return chain_walk(true, input, values, output, bias, workspace, inter, scratch, scratch_bytes, no_alloc,
                     batch, nfactors, patterns, dtype, bs_last, out_bs_last, activation, stream, nullptr,
-                    allow_switch, residual);
+                    allow_switch, pad, residual);
 }
 
 int ksmm_cu_chain_forward_act(const void* input, const void* const* values, void* output,
@@ -1002,7 +1089,7 @@ int ksmm_cu_grouped_chain_forward(const void* input, const void* const* values, 
   if (batch < 0) return set_error(KSMM_ERR_BAD_ARGUMENT, "negative batch");
   // per group: the intermediates of one chain; whatever follows the groups' intermediates is
   // layout scratch for the factors that run group by group
-  const size_t inter1 = chain_intermediate_bytes(nfactors, patterns, batch, dtype);
+  const size_t inter1 = chain_intermediate_bytes(nfactors, patterns, batch, dtype, 0);
   const size_t inter = inter1 * groups;
   if (inter > 0 && (!workspace || workspace_bytes < inter))
     return set_error(KSMM_ERR_WORKSPACE, "grouped chain workspace: need %zu bytes, got %zu", inter,
@@ -1105,7 +1192,14 @@ int ksmm_cu_chain_forward_static(const void* input, const void* const* values, v
   if (st != KSMM_OK) return st;
   // intermediates and, for batch-first factors that run through a layout conversion, their
   // transposed copies: all of it has to fit into the array
-  const size_t need = ksmm_cu_chain_workspace_bytes_ex(nfactors, patterns, batch, dtype, bs_last);
+  // (a ragged batch fits in the form without padded rows at least)
+  size_t need = ksmm_cu_chain_workspace_bytes_ex(nfactors, patterns, batch, dtype, bs_last);
+  if (need > static_cast<size_t>(KSMM_CU_STATIC_SCRATCH_BYTES)) {
+    const int last = bs_last ? 1 : 0;
+    const size_t plain = std::max(chain_need(nfactors, patterns, batch, dtype, last, last, 0, 0),
+                                  chain_need(nfactors, patterns, batch, dtype, last, last, 1, 0));
+    if (plain < need) need = plain;
+  }
   if (need > static_cast<size_t>(KSMM_CU_STATIC_SCRATCH_BYTES))
     return set_error(KSMM_ERR_WORKSPACE,
                      "the chain needs %zu bytes of scratch but the built-in scratch holds %zu: use "
@@ -1490,9 +1584,14 @@ int ksmm_cu_default_choice(const ksmm_forward_desc_t* desc, int* algo, int* conf
   if (ch.algo == KSMM_ALGO_CONVERT) {
     // report the kernel of the batch-last problem that the conversion path dispatches
     conv = 1;
+    ch = auto_choice(batch_last_twin(p));
+  } else if (ch.algo == kAlgoPadRows) {
+    // the kernel behind the padded copy
+    conv = 1;
     Problem q = p;
-    q.bs_last = 1;
-    q.in = q.out = reinterpret_cast<void*>(256);
+    q.in = reinterpret_cast<void*>(256);
+    q.in_ld = padded_ld(p.batch, dtype_size(p.in_dtype));
+    q.out_ld = p.batch;
     ch = auto_choice(q);
   }
   al = ch.algo;

@@ -18,6 +18,10 @@ int encode_map(CUtensorMap* tm, int dt, int rank, const void* base, const uint64
 // Device address of the per-device status word (0 = no device-side timeout).
 int* status_word();
 int num_sms();
+// true if a tensor map can address rows of `ld` elements of `es` bytes at `ptr`
+inline bool rows_addressable(const void* ptr, int64_t ld, int es) {
+  return (ld * es) % 16 == 0 && reinterpret_cast<uintptr_t>(ptr) % 16 == 0;
+}
 // false when the environment variable KSMM_NO_PDL is set (read once): launches are then plain ones
 bool pdl_enabled();
 

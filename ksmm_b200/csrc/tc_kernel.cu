@@ -81,6 +81,10 @@ struct Params {
   int groups, gx;
   int tiles_jg;    // tiles_j * groups
   const void* residual;  // added after the activation; output's layout and type; or nullptr
+  // Batch-last output whose rows no tensor map can address (y_direct): base pointer and row stride
+  void* y;
+  int64_t y_ld;
+  int y_direct;
 };
 
 // WRES = true  ("weight-stationary"): the CTA's weight tile (all NWC k chunks of
@@ -483,6 +487,51 @@ __global__ void __launch_bounds__(kThreads, Cfg<IN_LAST, OUT_LAST, ES, OS, NT, K
                            : "memory");
             }
           }
+          if (BS_LAST && P.y_direct) {
+            // Rows that start anywhere: the warp writes the staging tile one output row at a time, 32
+            // words per store instruction.  A 16-bit row that starts on an odd element takes its
+            // words from two neighbouring lanes and its two ends as single elements.  Sixteen rows are
+            // read ahead of their stores.
+            __syncwarp();
+            const int cols = col_limit - cbi * C::CB;                      // columns of this tile that exist
+            const int rows_here = min(32, row_limit - q * 32);
+            uint8_t* yrow = static_cast<uint8_t*>(P.y) +
+                            (((static_cast<int64_t>(i + yi0) * P.b + j0 + q * 32) * d + l) * P.y_ld + n0 + cbi * C::CB) * OS;
+            const int64_t ystep = static_cast<int64_t>(d) * P.y_ld * OS;
+#pragma unroll
+            for (int r0 = 0; r0 < 32; r0 += 16) {
+              uint32_t w[16], prev[16];
+#pragma unroll
+              for (int rr = 0; rr < 16; ++rr)
+                asm volatile("ld.shared.b32 %0, [%1];"
+                             : "=r"(w[rr])
+                             : "r"(stg + (r0 + rr) * 128 + (((lane >> 2) ^ (rr & 7)) << 4) + ((lane & 3) << 2)));
+              if constexpr (OS == 2) {
+#pragma unroll
+                for (int rr = 0; rr < 16; ++rr) prev[rr] = __shfl_up_sync(0xffffffffu, w[rr], 1);
+              }
+#pragma unroll
+              for (int rr = 0; rr < 16; ++rr, yrow += ystep) {
+                if (r0 + rr >= rows_here) break;
+                if constexpr (OS == 4) {
+                  if (lane < cols) reinterpret_cast<uint32_t*>(yrow)[lane] = w[rr];
+                } else {
+                  uint16_t* y16 = reinterpret_cast<uint16_t*>(yrow);
+                  if ((reinterpret_cast<uintptr_t>(yrow) & 2) == 0) {
+                    if (2 * lane + 1 < cols) reinterpret_cast<uint32_t*>(yrow)[lane] = w[rr];
+                    else if (2 * lane < cols) y16[2 * lane] = static_cast<uint16_t>(w[rr]);
+                  } else {
+                    // word of elements 2 lane - 1 and 2 lane
+                    if (lane == 0) y16[0] = static_cast<uint16_t>(w[rr]);
+                    else if (2 * lane < cols) *reinterpret_cast<uint32_t*>(y16 + 2 * lane - 1) = (prev[rr] >> 16) | (w[rr] << 16);
+                    else if (2 * lane - 1 < cols) y16[2 * lane - 1] = static_cast<uint16_t>(prev[rr] >> 16);
+                    if (lane == 31 && cols > 63) y16[63] = static_cast<uint16_t>(w[rr] >> 16);
+                  }
+                }
+              }
+            }
+            continue;  // (the next tile's writes come after the __syncwarp at the top of the loop)
+          }
           fence_proxy_async();
           __syncwarp();
           if (tron) KSMM_TRACE(trole, 25);
@@ -659,6 +708,9 @@ static int launch_one(const Problem& p, cudaStream_t stream) {
   P.groups = static_cast<int>(G);
   P.gx = GX > 1 ? 1 : 0;
   P.residual = p.residual;
+  P.y = p.out;
+  P.y_ld = out_stride(p);
+  P.y_direct = OUT_LAST && !rows_addressable(p.out, out_stride(p), OS);
   P.status = status_word();
   if (!P.status) return set_error(KSMM_ERR_CUDA, "cannot resolve the device status word");
   const uint32_t fmt = p.in_dtype == KSMM_BF16 ? 1u : 0u;  // f16 / e4m3 = 0, bf16 = 1
@@ -679,7 +731,9 @@ static int launch_one(const Problem& p, cudaStream_t stream) {
     const uint32_t xb[3] = {static_cast<uint32_t>(KC), 1, static_cast<uint32_t>(C::XN)};
     if ((st = encode_map(&tmX, p.in_dtype, 3, p.in, xd, xs, xb)) != KSMM_OK) return st;
   }
-  if (OUT_LAST) {
+  if (P.y_direct) {
+    tmY = tmX;  // unused: the epilogue stores rows with ordinary stores
+  } else if (OUT_LAST) {
     const uint64_t yd[4] = {B, d, b, G * a};
     const uint64_t L = out_stride(p);
     const uint64_t ys[4] = {1, L, d * L, b * d * L};
@@ -814,9 +868,9 @@ bool tc_config_supported(const Problem& p, int config, bool check_pointers) {
     if ((p.in_dtype != KSMM_F16 && p.in_dtype != KSMM_BF16) || p.out_dtype != p.in_dtype) return false;
     if (p.batch <= 0 || p.batch > 0x7fffffffLL) return false;
     if (p.b % 8 != 0 || p.c % 8 != 0) return false;   // 16-byte strides on both sides
-    if ((p.bs_last ? in_stride(p) : out_stride(p)) % 8 != 0) return false;
+    if (p.bs_last && in_stride(p) % 8 != 0) return false;
     if (check_pointers && (reinterpret_cast<uintptr_t>(p.in) % 16 || reinterpret_cast<uintptr_t>(p.w) % 16 ||
-                           reinterpret_cast<uintptr_t>(p.out) % 16))
+                           reinterpret_cast<uintptr_t>(p.out) % (out_last ? 2 : 16)))
       return false;
     return true;
   }
@@ -837,7 +891,7 @@ bool tc_config_supported(const Problem& p, int config, bool check_pointers) {
   // tensor-map rules: every global stride is a multiple of 16 bytes
   if ((static_cast<int64_t>(p.b) * es) % 16 != 0) return false;
   if (p.bs_last) {
-    if ((in_stride(p) * es) % 16 != 0 || (out_stride(p) * os) % 16 != 0) return false;
+    if ((in_stride(p) * es) % 16 != 0) return false;  // (output rows may start anywhere)
   } else {
     if (p.d != 1) return false;
     if ((static_cast<int64_t>(p.c) * es) % 16 != 0) return false;
@@ -845,7 +899,7 @@ bool tc_config_supported(const Problem& p, int config, bool check_pointers) {
   }
   if (check_pointers) {
     if (reinterpret_cast<uintptr_t>(p.in) % 16 || reinterpret_cast<uintptr_t>(p.w) % 16 ||
-        reinterpret_cast<uintptr_t>(p.out) % 16)
+        reinterpret_cast<uintptr_t>(p.out) % (p.bs_last ? os : 16))
       return false;
   }
   return true;
@@ -868,6 +922,8 @@ bool tc_fuses_residual(const Problem& p) {
   const bool out_last = p.out_bs_last < 0 ? p.bs_last != 0 : p.out_bs_last != 0;
   if (out_last == (p.bs_last != 0) && !p.bs_last && p.d != 1) return false;
   if (p.groups > 1 || p.out_regroup_d || has_padded_rows(p)) return false;
+  // (the epilogue reads the residual in 16-byte pieces of a row)
+  if (out_last && (p.batch * dtype_size(p.out_dtype)) % 16 != 0) return false;
   return reinterpret_cast<uintptr_t>(p.residual) % 16 == 0;
 }
 

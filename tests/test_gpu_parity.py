@@ -1290,3 +1290,54 @@ def test_weight_gradient_fp32_error(pattern, bs_last):
         err = torch.linalg.norm(dw.double() - ref.reshape(a * d * c, b)) / torch.linalg.norm(ref)
         assert err.item() < 4.8e-7, (batch, err.item())
     kb.check_device()
+
+
+# ---------------------------------------------------------------------------
+# batch-last tensors whose rows are no 16-byte multiples: padded copies inside, rows stored where they are
+# ---------------------------------------------------------------------------
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16, torch.float8_e4m3fn])
+@pytest.mark.parametrize("pattern", [(2, 48, 72, 3), (1, 192, 64, 4), (1, 144, 336, 2), (3, 64, 64, 1)])
+def test_ragged_rows_single_factor(pattern, dtype):
+    """Batches around the store tiles of 64 entries, an output that starts on an odd element, and nothing
+    written beyond it.  Tolerances: the fp32 sums of the general kernel differ in order only; a 16-bit
+    result may land on the neighbouring value (one rounding step relative to the result's norm)."""
+    a, b, c, d = pattern
+    fp8 = dtype == torch.float8_e4m3fn
+    outs = [torch.bfloat16, torch.float32] if fp8 else [dtype]
+    for batch in (1, 7, 63, 65, 197, 1001):
+        x, w = _inputs(pattern, batch, torch.float32 if fp8 else dtype, True, seed=batch)
+        xg, wk = x.to(DEV), kb.generate_factor(*pattern, "kernel", w, w.dtype, DEV)
+        if fp8:
+            xg, wk = xg.to(dtype), (wk * 4).to(dtype)
+        for od in outs:
+            n = a * b * d * batch
+            tol = {torch.float32: 1e-6, torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}[od]
+            ref = kb.forward_ex(xg, wk, True, a, b, c, d, out_dtype=od, algo=_lib.KSMM_ALGO_SIMT)
+            buf = torch.full((n + 130,), 7.0, dtype=od, device=DEV)
+            out = buf[1:1 + n].view(a * b * d, batch)
+            kb.forward_ex(xg, wk, True, a, b, c, d, out_dtype=od, out=out)
+            err = (torch.linalg.norm(out.double() - ref.double()) / torch.linalg.norm(ref.double())).item()
+            assert err < tol, (batch, od, err)
+            assert buf[0].item() == 7.0 and bool((buf[1 + n:] == 7.0).all()), batch
+    kb.check_device()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("patterns", [[(4, 48, 48, 1), (1, 192, 48, 4)], [(1, 96, 192, 4), (4, 64, 96, 1)],
+                                      [(1, 64, 64, 16), (4, 64, 64, 4), (16, 64, 64, 1)]])
+@pytest.mark.parametrize("bs_last,out_last", [(False, False), (False, True), (True, True), (True, False)])
+def test_ragged_chains(patterns, dtype, bs_last, out_last):
+    """Chains over every pair of end layouts at ragged batches against the fp64 product."""
+    rng = np.random.RandomState(3)
+    layer = kb.KSLinear(patterns, weights=[torch.from_numpy(w) for w in make_weights(patterns, rng)], bias=True,
+                        dtype=dtype, bs_last=bs_last, out_bs_last=out_last, device=DEV, activation="relu")
+    ws = [kb.from_kernel_format_to_abcd(f.data, p).float().cpu().numpy() for f, p in zip(layer.factors, patterns)]
+    for batch in (3, 66, 197, 1001):
+        x = rng.standard_normal((layer.in_size, batch) if bs_last else (batch, layer.in_size)).astype(np.float32)
+        xt = torch.from_numpy(x).to(dtype)
+        y = layer(xt.to(DEV)).float().cpu().numpy()
+        ref = ko.chain_apply(xt.float().numpy(), ws, bs_last)
+        ref = ref if bs_last else ref.T
+        ref = np.maximum(ref + layer.bias.detach().float().cpu().numpy().reshape(-1, 1), 0)
+        assert ko.rel_fro_error(y if out_last else y.T, ref) < TOL[dtype], batch
+    kb.check_device()
