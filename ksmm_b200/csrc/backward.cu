@@ -343,7 +343,8 @@ __global__ void __launch_bounds__(kThreadsW, 1)
 // elements per thread (elems is a multiple of 4 in the vector form), four splits in flight.
 template <typename T, int V>
 __global__ void __launch_bounds__(256)
-    wgrad_reduce_kernel(const float* __restrict__ part, T* __restrict__ dw, int64_t elems, int splits) {
+    wgrad_reduce_kernel(const float* part, T* dw, int64_t elems, int splits) {
+  // (no read-only loads in this kernel: the compiler may move those above the wait)
   grid_dep_wait();
   grid_dep_launch();
   const int64_t n = elems / V;
@@ -353,7 +354,12 @@ __global__ void __launch_bounds__(256)
 #pragma unroll 4
     for (int q = 0; q < splits; ++q) {
       float v[V];
-      load_vec<float, V>(part + q * elems + e * V, v);
+      if constexpr (V == 4) {
+        const float4 f = *reinterpret_cast<const float4*>(part + q * elems + e * V);
+        v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+      } else {
+        v[0] = part[q * elems + e];
+      }
 #pragma unroll
       for (int u = 0; u < V; ++u) s[u] += v[u];
     }
