@@ -132,8 +132,25 @@ KSMM_API int ksmm_cu_forward(const void* input, const void* values, void* output
 KSMM_API int ksmm_cu_forward_ex(const ksmm_forward_desc_t* desc, void* stream);
 
 /*
+ * A chain in fp8-e4m3 with activations in fp32, fp16 or bf16 (in_dtype) and a
+ * bf16 result: the input of every factor is quantised with its own per-tensor
+ * scale (amax / 448), which is computed and stays on the device.  `values` are
+ * the factors quantised by the caller, weight_scales[f] (host memory) their
+ * scales; bias: bf16, added by the last factor.  The workspace is aligned to
+ * 256 bytes.  (The reference's fp8 branch is empty, kernel.cu:66-82.)
+ */
+KSMM_API size_t ksmm_cu_chain_fp8_workspace_bytes(int nfactors, const int32_t* patterns, int64_t batch,
+                                         int in_dtype, int bs_last);
+KSMM_API int ksmm_cu_chain_forward_fp8(const void* input, int in_dtype, const void* const* values,
+                              const float* weight_scales, void* output, const void* bias,
+                              void* workspace, size_t workspace_bytes, int64_t batch, int nfactors,
+                              const int32_t* patterns, int bs_last, void* stream);
+
+/*
  * Device memory (bytes) that ksmm_cu_forward_ex needs beside input, weights
  * and output for this problem under the current dispatch: non-zero only for
+ * batch-last factors whose rows are no 16-byte multiples (copied into padded
+ * rows; without that scratch they run on the register-staged kernel) and for
  * batch-first factors with d > 1 that run through a layout conversion or a
  * regrouping pass (the reference's kernels index such inputs directly with
  * strided scalar accesses, template_kernels_half.cuh:402-413, and need none).

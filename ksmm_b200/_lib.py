@@ -41,6 +41,7 @@ EXPORTS = (
     "ksmm_cu_chain_workspace_bytes_layouts", "ksmm_cu_chain_forward_layouts", "ksmm_cu_chain_forward_desc",
     "ksmm_cu_backward_input_workspace_bytes", "ksmm_cu_backward_input",
     "ksmm_cu_backward_weights_workspace_bytes", "ksmm_cu_backward_weights",
+    "ksmm_cu_chain_fp8_workspace_bytes", "ksmm_cu_chain_forward_fp8",
 )
 
 
@@ -135,6 +136,11 @@ def load():
         fn = getattr(lib, name)
         fn.restype = i32
         fn.argtypes = [vp, vp, vp, vp, ctypes.c_size_t, i64, i32, i32, i32, i32, i32, i32, vp]
+    lib.ksmm_cu_chain_fp8_workspace_bytes.restype = ctypes.c_size_t
+    lib.ksmm_cu_chain_fp8_workspace_bytes.argtypes = [i32, ctypes.POINTER(ctypes.c_int32), i64, i32, i32]
+    lib.ksmm_cu_chain_forward_fp8.restype = i32
+    lib.ksmm_cu_chain_forward_fp8.argtypes = [vp, i32, ctypes.POINTER(vp), ctypes.POINTER(ctypes.c_float), vp, vp, vp,
+                                              ctypes.c_size_t, i64, i32, ctypes.POINTER(ctypes.c_int32), i32, vp]
     lib.ksmm_cu_host_wait.restype = i32
     lib.ksmm_cu_host_wait.argtypes = [ctypes.c_uint64]
     lib.ksmm_cu_num_configs.restype = i32

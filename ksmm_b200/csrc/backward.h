@@ -1,4 +1,5 @@
-// Host interface of the backward kernels (backward.cu, tc_wgrad_f32.cu).
+// Host interface of the backward kernels (backward.cu, tc_wgrad_f32.cu) and of the kernels that copy or
+// convert whole tensors (transpose.cu, quantize.cu).
 #pragma once
 
 #include "common.cuh"
@@ -32,5 +33,11 @@ int launch_transpose(const void* in, void* out, int64_t rows, int64_t cols, int 
 // are aligned to 16 bytes
 int launch_copy_rows(const void* in, int64_t in_ld, void* out, int64_t out_ld, int64_t rows, int64_t cols, int es,
                      cudaStream_t stream);
+
+// Per-tensor e4m3 quantisation of (rows, cols) with row stride in_ld: out has the same order (row stride
+// out_ld) or, with transpose (in_ld = cols), is (cols, rows).  `parts` holds quantize_parts_bytes().
+size_t quantize_parts_bytes();
+int launch_quantize(const void* in, int dtype, int64_t in_ld, void* out, int64_t out_ld, int64_t rows, int64_t cols,
+                    bool transpose, void* parts, float* scale, cudaStream_t stream);
 
 }  // namespace ksmm

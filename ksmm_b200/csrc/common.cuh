@@ -140,6 +140,7 @@ struct Problem {
   int64_t in_ld = 0, out_ld = 0;
   int no_pad = 0;  // 1: copies and intermediates keep rows of exactly the batch (what fits without padding)
   float alpha;
+  const float* alpha_dev = nullptr;  // fp8: a factor of alpha that a kernel earlier in the stream computes
   // Chains only.  out_regroup_d > 0: store the output regrouped by the blocks of the next factor
   // (c = out_regroup_c, d = out_regroup_d): feature (i2*c + k)*d + l goes to (i2*d + l)*c + k.
   // in_regrouped: the input already has that order for this factor's own (c, d).
@@ -174,6 +175,10 @@ inline bool has_padded_rows(const Problem& p) {
 // Row stride of the library's own batch-last copies and intermediates: the batch where its rows are
 // whole 16-byte pieces, else the next multiple of 64 entries.
 inline int64_t padded_ld(int64_t batch, int es) { return (batch * es) % 16 == 0 ? batch : (batch + 63) / 64 * 64; }
+
+__device__ __forceinline__ float scaled_alpha(float alpha, const float* alpha_dev) {
+  return alpha_dev ? static_cast<float>(static_cast<double>(*alpha_dev) * static_cast<double>(alpha)) : alpha;
+}
 
 // element-wise epilogue function (ksmm_activation_t)
 // erf by the rational approximation 7.1.26 of Abramowitz and Stegun (absolute error below

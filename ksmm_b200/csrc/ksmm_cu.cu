@@ -1034,6 +1034,109 @@ int ksmm_cu_chain_forward_layouts(const void* input, const void* const* values, 
                             static_cast<cudaStream_t>(stream));
 }
 
+// ---------------------------------------------------------------------------
+// fp8 chains: every factor's input is quantised per tensor on the device (quantize.cu) and the scale
+// stays there.  The activations turn batch-last, inside a quantisation, at the first factor that no
+// batch-first kernel covers, and stay so; a batch-first output is transposed once at the end.
+// ---------------------------------------------------------------------------
+struct Fp8Buffers {
+  size_t q = 0, y = 0;  // bytes of the quantised input, of one of the two bf16 intermediates
+  size_t parts() const { return align_up(quantize_parts_bytes(), 256); }
+  size_t total() const { return 256 + parts() + q + 2 * y; }  // (scales first)
+};
+
+static int chain_fp8_walk(bool run, const void* input, int in_dtype, const void* const* values, const float* wscales,
+                          void* output, const void* bias, char* ws, Fp8Buffers* buf, int64_t batch, int nfactors,
+                          const int32_t* patterns, int bs_last, cudaStream_t stream) {
+  if (nfactors > 64) return set_error(KSMM_ERR_UNSUPPORTED, "fp8 chains of more than 64 factors");
+  char* const plan = reinterpret_cast<char*>(static_cast<uintptr_t>(1) << 20);  // a plausible address
+  float* scales = reinterpret_cast<float*>(run ? ws : plan);
+  char* parts = reinterpret_cast<char*>(scales) + 256;
+  char* qbuf = parts + buf->parts();
+  char* ybuf = qbuf + buf->q;
+  const void* cur = input;
+  int cur_dtype = in_dtype, layout = bs_last;
+  int64_t cur_ld = bs_last ? batch : static_cast<int64_t>(patterns[0]) * patterns[2] * patterns[3];
+  for (int f = 0; f < nfactors; ++f) {
+    const int32_t* pt = patterns + 4 * f;
+    const bool last = f + 1 == nfactors;
+    const int64_t n_in = static_cast<int64_t>(pt[0]) * pt[2] * pt[3], n_out = static_cast<int64_t>(pt[0]) * pt[1] * pt[3];
+    Problem p;
+    p.in = qbuf; p.w = run ? values[f] : plan; p.bias = last ? bias : nullptr;
+    p.batch = batch; p.a = pt[0]; p.b = pt[1]; p.c = pt[2]; p.d = pt[3];
+    p.in_dtype = KSMM_F8E4M3; p.out_dtype = KSMM_BF16;
+    p.alpha = run ? wscales[f] : 1.f;
+    p.alpha_dev = scales + f;
+    p.no_alloc = 1;
+    p.bs_last = layout;
+    p.out = ybuf;
+    const bool turn = !layout && auto_choice(p).algo == KSMM_ALGO_CONVERT;
+    if (turn) p.bs_last = 1;
+    const int64_t q_ld = p.bs_last ? padded_ld(batch, 1) : n_in;
+    const int64_t y_ld = p.bs_last ? padded_ld(batch, 2) : n_out;
+    const bool to_output = last && p.bs_last == bs_last;
+    if (p.bs_last) {
+      p.in_ld = q_ld;
+      p.out_ld = to_output ? batch : y_ld;
+    }
+    p.out = to_output ? output : ybuf + (f & 1) * buf->y;
+    if (run) {
+      const int64_t rows = layout ? n_in : batch, cols = layout ? batch : n_in;
+      int st = launch_quantize(cur, cur_dtype, cur_ld, qbuf, q_ld, rows, cols, turn, parts, scales + f, stream);
+      if (st == KSMM_OK) st = dispatch(p, KSMM_ALGO_AUTO, -1, stream);
+      if (st != KSMM_OK) return st;
+      if (last && !to_output) return launch_transpose(p.out, output, n_out, batch, 2, stream, 0, y_ld);
+    } else {
+      buf->q = std::max(buf->q, align_up(static_cast<size_t>(p.bs_last ? n_in : batch) * q_ld, 256));
+      if (!to_output) buf->y = std::max(buf->y, align_up(static_cast<size_t>(p.bs_last ? n_out : batch) * y_ld * 2, 256));
+    }
+    cur = p.out;
+    cur_dtype = KSMM_BF16;
+    layout = p.bs_last;
+    cur_ld = y_ld;
+  }
+  return KSMM_OK;
+}
+
+static int check_chain_fp8(int nfactors, const int32_t* patterns, const void* const* values, int64_t batch, int in_dtype,
+                           int bs_last) {
+  int st = check_chain(nfactors, patterns, values, KSMM_BF16, 0);
+  if (st != KSMM_OK) return st;
+  if (in_dtype != KSMM_F32 && in_dtype != KSMM_F16 && in_dtype != KSMM_BF16)
+    return set_error(KSMM_ERR_BAD_ARGUMENT, "an fp8 chain takes fp32, fp16 or bf16 activations");
+  if (bs_last != 0 && bs_last != 1) return set_error(KSMM_ERR_BAD_ARGUMENT, "bs_last must be 0 or 1");
+  if (batch < 0) return set_error(KSMM_ERR_BAD_ARGUMENT, "negative batch");
+  return KSMM_OK;
+}
+
+size_t ksmm_cu_chain_fp8_workspace_bytes(int nfactors, const int32_t* patterns, int64_t batch, int in_dtype, int bs_last) {
+  const void* dummy = nullptr;
+  Fp8Buffers buf;
+  if (batch <= 0 || check_chain_fp8(nfactors, patterns, &dummy, batch, in_dtype, bs_last) != KSMM_OK) return 0;
+  if (chain_fp8_walk(false, nullptr, in_dtype, nullptr, nullptr, nullptr, nullptr, nullptr, &buf, batch, nfactors,
+                     patterns, bs_last, nullptr) != KSMM_OK)
+    return 0;
+  return buf.total();
+}
+
+int ksmm_cu_chain_forward_fp8(const void* input, int in_dtype, const void* const* values, const float* weight_scales,
+                              void* output, const void* bias, void* workspace, size_t workspace_bytes, int64_t batch,
+                              int nfactors, const int32_t* patterns, int bs_last, void* stream) {
+  int st = check_chain_fp8(nfactors, patterns, values, batch, in_dtype, bs_last);
+  if (st != KSMM_OK) return st;
+  if (batch == 0) return KSMM_OK;
+  if (!input || !output || !weight_scales) return set_error(KSMM_ERR_BAD_ARGUMENT, "null pointer");
+  Fp8Buffers buf;
+  st = chain_fp8_walk(false, nullptr, in_dtype, nullptr, nullptr, nullptr, nullptr, nullptr, &buf, batch, nfactors,
+                      patterns, bs_last, nullptr);
+  if (st != KSMM_OK) return st;
+  if (!workspace || reinterpret_cast<uintptr_t>(workspace) % 256 || workspace_bytes < buf.total())
+    return set_error(KSMM_ERR_WORKSPACE, "fp8 chain workspace: need %zu bytes aligned to 256, got %zu", buf.total(),
+                     workspace_bytes);
+  return chain_fp8_walk(true, input, in_dtype, values, weight_scales, output, bias, static_cast<char*>(workspace), &buf,
+                        batch, nfactors, patterns, bs_last, static_cast<cudaStream_t>(stream));
+}
+
 // One factor for `groups` stacked problems: one grouped launch where a kernel has that form,
 // else one dispatch per group.
 static int grouped_factor(Problem p, int groups, int shared_input, cudaStream_t stream) {

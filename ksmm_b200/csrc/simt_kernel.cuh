@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(WJ* WN * 32, 512 / (WJ * WN * 32))
   // ---- epilogue: alpha, bias, conversion, vector stores ---------------------
   TOut* __restrict__ Y = static_cast<TOut*>(p.out);
   const TOut* __restrict__ bias = static_cast<const TOut*>(p.bias);
-  const float alpha = p.alpha;
+  const float alpha = scaled_alpha(p.alpha, p.alpha_dev);
 
   if constexpr (BS_LAST) {
 #pragma unroll

@@ -70,6 +70,7 @@ struct Params {
   int nk;
   uint32_t idesc;
   float alpha;
+  const float* alpha_dev;
   const void* bias;
   int out_dtype;
   int* status;
@@ -327,7 +328,8 @@ __global__ void __launch_bounds__(kThreads, Cfg<IN_LAST, OUT_LAST, ES, OS, NT, K
     const int q = warp & 3;
     const int grp = ew >> 2;
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
-    const bool plain = (P.alpha == 1.f) && (P.bias == nullptr) && (P.act == 0);
+    const float alpha = ES == 1 ? scaled_alpha(P.alpha, P.alpha_dev) : P.alpha;
+    const bool plain = (alpha == 1.f) && (P.bias == nullptr) && (P.act == 0);
     const uint32_t stg_base = stg0 + ew * C::STG_WARP_BYTES;
     uint32_t ut = 0, sti = 0;
     KSMM_TRACE_DECL;
@@ -403,7 +405,7 @@ __global__ void __launch_bounds__(kThreads, Cfg<IN_LAST, OUT_LAST, ES, OS, NT, K
                   bv = __uint_as_float(__shfl_sync(0xffffffffu, braw, e));
                 }
               }
-              r[e] = __float_as_uint(fmaf(P.alpha, __uint_as_float(r[e]), bv));
+              r[e] = __float_as_uint(fmaf(alpha, __uint_as_float(r[e]), bv));
             }
             if (P.act == KSMM_ACT_GELU) {
 #pragma unroll
@@ -700,6 +702,7 @@ static int launch_one(const Problem& p, cudaStream_t stream) {
   P.batch = p.batch;
   P.nk = (p.c + KC - 1) / KC;
   P.alpha = p.alpha;
+  P.alpha_dev = p.alpha_dev;
   P.bias = p.bias;
   P.out_dtype = p.out_dtype;
   P.act = p.activation;
@@ -952,7 +955,8 @@ int tc_default_config(const Problem& p) {
   // 24.1 against 26.5 us batch-first for the 16-block patterns)
   const bool small16 = p.in_dtype != KSMM_F8E4M3 && p.b <= 64 && p.c <= 64 && p.batch >= 4096;
   if (out_last) return small16 ? 5 : (p.batch >= 256 * 148 / 2 || p.batch >= 4096 ? 0 : 1);
-  return p.b > 128 ? 0 : (p.b > 64 ? 1 : (small16 ? 5 : 4));
+  // (configuration 4 is narrower than a 128-byte box row of 8-bit weights)
+  return p.b > 128 ? 0 : (p.b > 64 || p.in_dtype == KSMM_F8E4M3 ? 1 : (small16 ? 5 : 4));
 }
 
 int tc_launch(const Problem& p, int config, cudaStream_t stream) {

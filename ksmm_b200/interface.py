@@ -133,12 +133,17 @@ class KSLinear(nn.Module):
     def _forward_2d(self, x, residual=None):
         bias = None if self.bias is None else self.bias.reshape(-1)
         if self.is_fp8:
-            y = x
-            for idx, (p, (wq, sw)) in enumerate(zip(self.patterns, self._fp8_factors())):
-                xq, sx = _k.quantize_e4m3(y)
-                last = idx + 1 == self.num_mat
-                y = _k.forward_fp8(xq, wq, self.bs_last, *p, sx, sw, out_dtype=torch.bfloat16,
-                                   bias=bias if last else None)
+            quantised = self._fp8_factors()
+            if x.is_cuda and x.numel() and x.dtype in (torch.bfloat16, torch.float16, torch.float32):
+                y = _k.chain_forward_fp8(x.detach(), [w for w, _ in quantised], [s for _, s in quantised],
+                                         self.patterns, self.bs_last, bias=bias)
+            else:
+                y = x
+                for idx, (p, (wq, sw)) in enumerate(zip(self.patterns, quantised)):
+                    xq, sx = _k.quantize_e4m3(y)
+                    last = idx + 1 == self.num_mat
+                    y = _k.forward_fp8(xq, wq, self.bs_last, *p, sx, sw, out_dtype=torch.bfloat16,
+                                       bias=bias if last else None)
             if self.activation == "gelu":
                 y = torch.nn.functional.gelu(y)
             elif self.activation == "relu":

@@ -208,6 +208,39 @@ def chain_forward(input, factors, patterns, bs_last, bias=None, workspace=None, 
     return out
 
 
+def chain_forward_fp8(input, factors, scales, patterns, bs_last, bias=None):
+    """All factors of an fp8 KSLinear in one library call (``ksmm_cu_chain_forward_fp8``): ``factors[f]`` and
+    ``scales[f]`` come from ``quantize_e4m3``; every factor's input is quantised on the device the way
+    ``quantize_e4m3`` does it.  ``input``: fp32, fp16 or bf16; the result and ``bias`` are bf16."""
+    lib = _lib.load()
+    bs_last = int(bool(bs_last))
+    nf = len(patterns)
+    feats = input.shape[0] if bs_last else input.shape[1]
+    for (a, b, c, d), w in zip(patterns, factors):
+        if feats != a * c * d:
+            raise ValueError(f"input has {feats} features, pattern ({a},{b},{c},{d}) expects {a * c * d}")
+        if tuple(w.shape) != (a * d * c, b) or w.dtype != torch.float8_e4m3fn or not w.is_contiguous():
+            raise ValueError(f"factor must be a contiguous ({a * d * c}, {b}) tensor of float8_e4m3fn")
+        if w.device != input.device:
+            raise ValueError("input and factor live on different devices")
+        feats = a * b * d
+    if bias is not None and (bias.numel() != feats or bias.dtype != torch.bfloat16 or not bias.is_contiguous()):
+        raise ValueError("bias must hold a*b*d contiguous elements of the output dtype")
+    batch = input.shape[1] if bs_last else input.shape[0]
+    out = torch.empty((feats, batch) if bs_last else (batch, feats), dtype=torch.bfloat16, device=input.device)
+    pat = _lib.int32_array([int(v) for p in patterns for v in p])
+    code = dtype_code(input.dtype)
+    need = lib.ksmm_cu_chain_fp8_workspace_bytes(nf, pat, batch, code, bs_last)
+    ws = torch.empty(max(need, 1), dtype=torch.uint8, device=input.device)
+    vals = (ctypes.c_void_p * nf)(*[w.data_ptr() for w in factors])
+    with torch.cuda.device(input.device):
+        _lib.check(lib.ksmm_cu_chain_forward_fp8(
+            input.data_ptr(), code, vals, (ctypes.c_float * nf)(*scales), out.data_ptr(),
+            bias.data_ptr() if bias is not None else None, ws.data_ptr(), need, batch, nf, pat, bs_last,
+            _stream_ptr(input.device)))
+    return out
+
+
 def grouped_chain_forward(input, stacked_factors, patterns, bs_last, groups, bias=None):
     """``groups`` chains with the same ``patterns`` on one shared input (``ksmm_cu_grouped_chain_forward``):
     ``stacked_factors[f]`` is the (groups * a*d*c, b) concatenation of the groups' kernel-format

@@ -1341,3 +1341,34 @@ def test_ragged_chains(patterns, dtype, bs_last, out_last):
         ref = np.maximum(ref + layer.bias.detach().float().cpu().numpy().reshape(-1, 1), 0)
         assert ko.rel_fro_error(y if out_last else y.T, ref) < TOL[dtype], batch
     kb.check_device()
+
+
+# ---------------------------------------------------------------------------
+# fp8 chains with the quantisation on the device
+# ---------------------------------------------------------------------------
+@pytest.mark.parametrize("in_dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("patterns", [[(4, 48, 48, 1), (1, 192, 48, 4)], [(1, 96, 192, 4), (4, 64, 96, 1)],
+                                      [(2, 40, 24, 3), (3, 24, 40, 2)], [(3, 64, 64, 1)]])
+@pytest.mark.parametrize("bs_last", [False, True])
+def test_fp8_chain_quantises_as_quantize_e4m3(patterns, bs_last, in_dtype):
+    """Against the factors one by one, quantised by torch on the same values.  The sums of a factor may
+    differ in order, so a bf16 intermediate can land on a neighbouring value and its e4m3 value on the
+    next one (2^-4) for a few per thousand of the entries: 2^-8 of the result's norm."""
+    layer = kb.KSLinear(patterns, dtype=torch.float8_e4m3fn, bs_last=bs_last, device=DEV)
+    for batch in (1, 40, 197, 1000):
+        gen = torch.Generator(device=DEV).manual_seed(batch)
+        shape = (layer.in_size, batch) if bs_last else (batch, layer.in_size)
+        for x in (torch.randn(shape, device=DEV, generator=gen).to(in_dtype), torch.zeros(shape, device=DEV, dtype=in_dtype)):
+            y = layer(x)
+            ref = x
+            for f, (p, (wq, sw)) in enumerate(zip(patterns, layer._fp8_factors())):
+                q, sx = kb.quantize_e4m3(ref)
+                ref = kb.forward_fp8(q, wq, bs_last, *p, sx, sw,
+                                     bias=layer.bias.reshape(-1) if f + 1 == len(patterns) else None)
+            assert y.dtype == ref.dtype and y.shape == ref.shape
+            err = torch.linalg.norm(y.double() - ref.double()) / torch.linalg.norm(ref.double())
+            assert err.item() < 2.0 ** -8, (batch, err.item())
+    x = torch.randn(layer.in_size, 64, device=DEV).t().contiguous() if not bs_last else torch.randn(layer.in_size, 64, device=DEV)
+    x.view(-1)[5] = float("nan")
+    assert bool(torch.isnan(layer(x.to(in_dtype))).any())
+    kb.check_device()
