@@ -266,6 +266,31 @@ KSMM_API int ksmm_cu_grouped_chain_forward(const void* input, const void* const*
                                            int dtype, int bs_last, int groups, void* stream);
 
 /*
+ * A chain with its backward (the reference's backward is a stub, kernel.py:323-329).
+ * ksmm_cu_chain_train_bytes gives the sizes of the three buffers: what the
+ * forward keeps for the backward (`saved`), its scratch, and the backward's
+ * workspace; all aligned to 256 bytes.  The forward writes the intermediates
+ * into `saved` and says in layouts[0 .. nfactors - 2] how each is stored (0
+ * batch-first, 1 batch-last, 2 batch-first in the block order of the next
+ * factor).  The backward computes whichever of grad_input, grad_values[f]
+ * (kernel format) and grad_bias is not NULL; its input and grad_output are
+ * aligned to 16 bytes.  fp32, fp16 and bf16; results have the input's type.
+ */
+KSMM_API int ksmm_cu_chain_train_bytes(int nfactors, const int32_t* patterns, int64_t batch, int dtype,
+                              int bs_last, size_t* saved_bytes, size_t* forward_bytes,
+                              size_t* backward_bytes);
+KSMM_API int ksmm_cu_chain_train_forward(const void* input, const void* const* values, void* output,
+                                const void* bias, void* saved, size_t saved_bytes, void* scratch,
+                                size_t scratch_bytes, int64_t batch, int nfactors,
+                                const int32_t* patterns, int dtype, int bs_last,
+                                int32_t* layouts, void* stream);
+KSMM_API int ksmm_cu_chain_backward(const void* input, const void* const* values, const void* saved,
+                           const int32_t* layouts, const void* grad_output, void* grad_input,
+                           void* const* grad_values, void* grad_bias, void* workspace,
+                           size_t workspace_bytes, int64_t batch, int nfactors,
+                           const int32_t* patterns, int dtype, int bs_last, void* stream);
+
+/*
  * Backward of one factor.  The reference has none: Kernel.backward is a stub
  * that calls an undefined kernel.backward
  * (src/ksmm_py/layer/kronecker_sparse/kernel.py:323-329).

@@ -41,6 +41,7 @@ EXPORTS = (
     "ksmm_cu_chain_workspace_bytes_layouts", "ksmm_cu_chain_forward_layouts", "ksmm_cu_chain_forward_desc",
     "ksmm_cu_backward_input_workspace_bytes", "ksmm_cu_backward_input",
     "ksmm_cu_backward_weights_workspace_bytes", "ksmm_cu_backward_weights",
+    "ksmm_cu_chain_train_bytes", "ksmm_cu_chain_train_forward", "ksmm_cu_chain_backward",
     "ksmm_cu_chain_fp8_workspace_bytes", "ksmm_cu_chain_forward_fp8",
 )
 
@@ -136,6 +137,15 @@ def load():
         fn = getattr(lib, name)
         fn.restype = i32
         fn.argtypes = [vp, vp, vp, vp, ctypes.c_size_t, i64, i32, i32, i32, i32, i32, i32, vp]
+    psz, pvp, pi32 = ctypes.POINTER(ctypes.c_size_t), ctypes.POINTER(vp), ctypes.POINTER(ctypes.c_int32)
+    lib.ksmm_cu_chain_train_bytes.restype = i32
+    lib.ksmm_cu_chain_train_bytes.argtypes = [i32, pi32, i64, i32, i32, psz, psz, psz]
+    lib.ksmm_cu_chain_train_forward.restype = i32
+    lib.ksmm_cu_chain_train_forward.argtypes = [vp, pvp, vp, vp, vp, ctypes.c_size_t, vp, ctypes.c_size_t, i64, i32, pi32,
+                                                i32, i32, pi32, vp]
+    lib.ksmm_cu_chain_backward.restype = i32
+    lib.ksmm_cu_chain_backward.argtypes = [vp, pvp, vp, pi32, vp, vp, pvp, vp, vp, ctypes.c_size_t, i64, i32, pi32, i32, i32,
+                                           vp]
     lib.ksmm_cu_chain_fp8_workspace_bytes.restype = ctypes.c_size_t
     lib.ksmm_cu_chain_fp8_workspace_bytes.argtypes = [i32, ctypes.POINTER(ctypes.c_int32), i64, i32, i32]
     lib.ksmm_cu_chain_forward_fp8.restype = i32

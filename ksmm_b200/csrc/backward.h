@@ -12,6 +12,7 @@ struct WgradOperand {
   const void* ptr;
   int last;    // 1: (features, batch), 0: (batch, features)
   int64_t ld;
+  int regrouped = 0;  // batch-first rows in block order (i, l, k) instead of (i, k, l)
 };
 
 // block transposes of kernel-format weights: (nblk, c, b) -> (nblk, b, c)
@@ -22,6 +23,13 @@ int launch_transpose_blocks(const void* in, void* out, int64_t nblk, int c, int 
 size_t wgrad_workspace_bytes(const Problem& p, const WgradOperand& x, const WgradOperand& g);
 int wgrad_launch(const Problem& p, WgradOperand x, WgradOperand g, void* workspace, size_t workspace_bytes,
                  cudaStream_t stream);
+// Gradient of a bias: the sum over the batch of a gradient of `feats` features, in fp32, stored as `dtype`.
+// The workspace holds bias_grad_workspace_bytes(feats) for a batch-first gradient.
+size_t bias_grad_workspace_bytes(int64_t feats);
+int launch_bias_grad(const void* g, int last, int64_t ld, void* out, void* workspace, int64_t batch, int64_t feats,
+                     int dtype, cudaStream_t stream);
+// the weight gradient of such a factor runs on the tensor cores for every pair of operand layouts
+bool wgrad_any_layout(const Problem& p);
 // the fp32 tensor-core kernel: partial tiles (splits, a*d, c, b) into `part`; nt = 64 or 128 columns
 int wgrad_f32_launch(const Problem& p, const WgradOperand& x, const WgradOperand& g, float* part, int nt, int splits,
                      cudaStream_t stream);

@@ -727,8 +727,12 @@ static int chain_walk(bool run, const void* input, const void* const* values, vo
                       size_t scratch_bytes, int no_alloc, int64_t batch, int nfactors,
                       const int32_t* patterns, int dtype, int bs_last, int out_bs_last, int activation,
                       cudaStream_t stream, size_t* scratch_max, int allow_switch,
-                      int pad, const void* residual = nullptr);
+                      int pad, const void* residual = nullptr, int keep = 0, int32_t* layouts = nullptr);
 
+// `pad`: 0 every batch-last tensor has rows of exactly the batch, 1 those inside the chain are padded where
+// the batch is no multiple of 16 bytes, 2 as 0, but a factor may copy its own input into padded rows and
+// nothing is regrouped.  `keep`: every intermediate has its own buffer, and layouts[f] says how factor f's
+// output is stored (0 batch-first, 1 batch-last, 2 batch-first in the next factor's block order).
 // One pass over a chain: either plans it (run == false: returns through *scratch_max the layout
 // scratch it needs under the current dispatch: transposed copies at the chain's ends plus the
 // largest scratch of any factor) or runs it.
@@ -736,25 +740,28 @@ static int chain_walk(bool run, const void* input, const void* const* values, vo
                       const void* bias, void* workspace, size_t inter_bytes, void* scratch,
                       size_t scratch_bytes, int no_alloc, int64_t batch, int nfactors,
                       const int32_t* patterns, int dtype, int bs_last, int out_bs_last, int activation,
-                      cudaStream_t stream, size_t* scratch_max, int allow_switch, int pad, const void* residual) {
+                      cudaStream_t stream, size_t* scratch_max, int allow_switch, int pad, const void* residual,
+                      int keep, int32_t* layouts) {
   if (nfactors > ChainPlan::kMax)
     return set_error(KSMM_ERR_UNSUPPORTED, "chains of more than %d factors", ChainPlan::kMax);
   ChainPlan plan;
-  plan_chain(nfactors, patterns, batch, dtype, bs_last, out_bs_last, allow_switch != 0, pad != 0, &plan);
+  plan_chain(nfactors, patterns, batch, dtype, bs_last, out_bs_last, allow_switch != 0, pad == 1, &plan);
   const size_t es = dtype_size(dtype);
   const int32_t* p0 = patterns;
   const int32_t* pl = patterns + 4 * (nfactors - 1);
   const int64_t in_feats = static_cast<int64_t>(p0[0]) * p0[2] * p0[3];
   const int64_t out_feats = static_cast<int64_t>(pl[0]) * pl[1] * pl[3];
   // row stride of the batch-last tensors between the chain's ends
-  const int64_t ld = pad ? padded_ld(batch, static_cast<int>(es)) : batch;
+  const int64_t ld = pad == 1 ? padded_ld(batch, static_cast<int>(es)) : batch;
   // a batch-last chain input with rows that no tensor map can address is copied into padded rows
   // (blocks that the tensor kernels do not take read it as it is)
   const bool pad_in = ld != batch && bs_last && !plan.pre_transpose && p0[1] >= 32 && p0[2] >= 16;
   const size_t pre_bytes =
       plan.pre_transpose || pad_in ? align_up(static_cast<size_t>(in_feats) * ld * es, 256) : 0;
   const size_t post_bytes = plan.post_transpose ? align_up(static_cast<size_t>(out_feats) * ld * es, 256) : 0;
-  const size_t half = nfactors == 2 ? inter_bytes : inter_bytes / 2;
+  // one buffer per intermediate, or two that alternate
+  const size_t half = keep ? inter_bytes / std::max(1, nfactors - 1) : (nfactors == 2 ? inter_bytes : inter_bytes / 2);
+  auto inter_at = [&](int f) { return static_cast<size_t>(keep ? f : f & 1) * half; };
   const void* cur = input;
   bool cur_regrouped = false;  // the intermediate in `cur` is regrouped by the blocks of factor f
   char* ws = static_cast<char*>(workspace);
@@ -776,7 +783,7 @@ static int chain_walk(bool run, const void* input, const void* const* values, vo
     size_t total = 0;
     int stp = chain_walk(false, nullptr, nullptr, nullptr, nullptr, nullptr, inter_bytes, nullptr, 0, 0, batch,
                          nfactors, patterns, dtype, bs_last, out_bs_last, activation, nullptr, &total,
-                         allow_switch, pad);
+                         allow_switch, pad, nullptr, keep);
     if (stp != KSMM_OK) return stp;
     if (total > 0) {
       Problem sp;
@@ -807,16 +814,17 @@ static int chain_walk(bool run, const void* input, const void* const* values, vo
   for (int f = 0; f < nfactors; ++f) {
     const int32_t* q = patterns + 4 * f;
     const bool last = (f + 1 == nfactors);
-    void* dst = last ? (plan.post_transpose && run ? static_cast<void*>(t_post) : output) : ws + (f & 1) * half;
+    void* dst = last ? (plan.post_transpose && run ? static_cast<void*>(t_post) : output) : ws + inter_at(f);
     Problem p;
     p.in = cur; p.w = run ? values[f] : ws; p.out = dst; p.bias = last ? bias : nullptr;
     p.batch = batch; p.a = q[0]; p.b = q[1]; p.c = q[2]; p.d = q[3];
     p.in_dtype = dtype; p.out_dtype = dtype; p.alpha = 1.f;
     p.bs_last = plan.in_last[f];
     p.out_bs_last = plan.out_last[f] == plan.in_last[f] ? -1 : plan.out_last[f];
-    if (plan.in_last[f]) p.in_ld = f > 0 || plan.pre_transpose || pad_in ? ld : batch;
-    if (plan.out_last[f]) p.out_ld = !last || plan.post_transpose ? ld : batch;
-    p.no_pad = !pad;
+    // (0 = the batch)
+    if (plan.in_last[f] && ld != batch) p.in_ld = f > 0 || plan.pre_transpose || pad_in ? ld : batch;
+    if (plan.out_last[f] && ld != batch) p.out_ld = !last || plan.post_transpose ? ld : batch;
+    p.no_pad = pad == 0;
     p.activation = last ? activation : 0;
     // the residual has the chain output's layout: it can join the last factor's epilogue only when
     // that factor writes the final layout itself
@@ -828,12 +836,12 @@ static int chain_walk(bool run, const void* input, const void* const* values, vo
     // written in that order and the next factor runs the kernel without the transposer stage
     // (and without a regrouping pass).
     bool next_regrouped = false;
-    if (!last && same_first && !plan.in_last[f + 1] && !plan.out_last[f + 1]) {
+    if (!last && same_first && !plan.in_last[f + 1] && !plan.out_last[f + 1] && pad != 2) {
       const int32_t* r = patterns + 4 * (f + 1);
       Problem nx = p;
       // the next factor reads this factor's destination and writes its own one
       nx.in = dst;
-      nx.out = (f + 2 == nfactors) ? output : ws + ((f + 1) & 1) * half;
+      nx.out = (f + 2 == nfactors) ? output : ws + inter_at(f + 1);
       nx.w = run ? values[f + 1] : ws; nx.bias = nullptr;
       nx.a = r[0]; nx.b = r[1]; nx.c = r[2]; nx.d = r[3];
       p.out_regroup_c = r[2];
@@ -869,6 +877,7 @@ static int chain_walk(bool run, const void* input, const void* const* values, vo
     if (st != KSMM_OK) return st;
     cur = dst;
     cur_regrouped = next_regrouped;
+    if (layouts && !last) layouts[f] = next_regrouped ? 2 : plan.out_last[f];
   }
   if (plan.post_transpose && run && batch > 0) {
     // the last factor wrote the other layout into t_post
@@ -1286,6 +1295,283 @@ int ksmm_cu_backward_weights(const void* input, const void* grad_output, void* g
   if (st != KSMM_OK) return st;
   return wgrad_launch(p, WgradOperand{input, bs_last, batch}, WgradOperand{grad_output, bs_last, batch}, workspace,
                       workspace_bytes, static_cast<cudaStream_t>(stream));
+}
+
+// ---------------------------------------------------------------------------
+// A chain with its backward.  The forward keeps every intermediate in the layout that its plan gives it.
+// The backward plans the gradients' layouts the same way, over the transposed factors in reverse, with
+// the copy of a weight gradient's operand (batch-first with d > 1 cannot be addressed) among the costs:
+// a batch-first gradient of a factor with d > 1 is transposed once, for both of its uses.  Input and
+// gradient of a factor may lie in different layouts; where a weight gradient has no tensor-core form
+// for that (tiny blocks, short fp32 batches) the whole call keeps the layout of its ends.
+// ---------------------------------------------------------------------------
+static bool train_one_layout(int nfactors, const int32_t* patterns, int64_t batch, int dtype, int bs_last) {
+  for (int f = 0; f < nfactors; ++f) {
+    const int32_t* q = patterns + 4 * f;
+    if (!wgrad_any_layout(backward_problem(nullptr, nullptr, nullptr, batch, q[0], q[1], q[2], q[3], dtype, bs_last)))
+      return true;
+  }
+  return nfactors > 8;
+}
+
+// bytes of one intermediate's buffer
+static size_t train_buffer_bytes(int nfactors, const int32_t* patterns, int64_t batch, int dtype) {
+  size_t mx = 0;
+  for (int f = 0; f + 1 < nfactors; ++f) {
+    const int32_t* q = patterns + 4 * f;
+    mx = std::max(mx, static_cast<size_t>(q[0]) * q[1] * q[3]);
+  }
+  return align_up(mx * padded_ld(batch, dtype_size(dtype)) * dtype_size(dtype), 256);
+}
+
+struct BackwardPlan {
+  bool pre = false;                   // a transposed copy of the output's gradient
+  int in_last[ChainPlan::kMax], out_last[ChainPlan::kMax];  // of the input-gradient multiplication of factor f
+};
+
+// copy of a weight gradient's operand that the kernels cannot address: a transpose
+static double wgrad_copy_cost(const int32_t* q, int64_t batch, int dtype, int last) {
+  if (last || q[3] == 1) return 0.0;
+  return 1.5 * dtype_size(dtype) * q[0] * q[1] * q[3] * static_cast<double>(batch);
+}
+
+static void plan_backward(int nfactors, const int32_t* patterns, int64_t batch, int dtype, int bs_last, bool need_input,
+                          bool allow_switch, BackwardPlan* plan) {
+  for (int f = 0; f < nfactors; ++f) plan->in_last[f] = plan->out_last[f] = bs_last;
+  plan->pre = false;
+  if (!allow_switch) return;
+  const int32_t* pl = patterns + 4 * (nfactors - 1);
+  const double kTranspose = 0.75 * 2.0, es = dtype_size(dtype);
+  const double out_bytes = es * pl[0] * pl[1] * pl[3] * batch;
+  const double in_bytes = es * patterns[0] * patterns[2] * patterns[3] * batch;
+  double best = -1.0;
+  for (int pre = 0; pre < 2; ++pre) {
+    for (unsigned mask = 0; mask < (1u << nfactors); ++mask) {
+      int state = pre ? !bs_last : bs_last;
+      double cost = pre ? kTranspose * out_bytes : 0.0;
+      bool ok = true;
+      for (int f = nfactors - 1; f >= 0 && ok; --f) {
+        const int32_t* q = patterns + 4 * f;
+        cost += wgrad_copy_cost(q, batch, dtype, state || (f == nfactors - 1 && (pre || bs_last)));
+        const int o = (mask >> f) & 1;
+        if (f == 0 && !need_input) {
+          if (o != state) ok = false;  // nothing is multiplied
+          break;
+        }
+        const int32_t t[4] = {q[0], q[2], q[1], q[3]};  // the transposed factor
+        const double c = step_cost(t, batch, dtype, state, o, true);
+        if (c < 0) ok = false;
+        cost += c;
+        state = o;
+      }
+      if (!ok) continue;
+      if (need_input && state != bs_last) cost += kTranspose * in_bytes;
+      if (best < 0 || cost < best * 0.999) {
+        best = cost;
+        plan->pre = pre != 0;
+        int s2 = pre ? !bs_last : bs_last;
+        for (int f = nfactors - 1; f >= 0; --f) {
+          plan->in_last[f] = s2;
+          plan->out_last[f] = s2 = (mask >> f) & 1;
+        }
+      }
+    }
+  }
+}
+
+// Plans (run == false: the workspace's bytes through *need) or runs the backward of a chain.
+static int chain_backward_walk(bool run, const void* input, const void* const* values, const void* saved,
+                               const int32_t* layouts, const void* grad_output, void* grad_input,
+                               void* const* grad_values, void* grad_bias, char* ws, int64_t batch, int nfactors,
+                               const int32_t* patterns, int dtype, int bs_last, bool need_input, bool allow_switch,
+                               bool one_layout, cudaStream_t stream, size_t* need) {
+  const int es = dtype_size(dtype);
+  const int64_t ld = one_layout ? batch : padded_ld(batch, es);
+  BackwardPlan plan;
+  plan_backward(nfactors, patterns, batch, dtype, bs_last, need_input, allow_switch && !one_layout, &plan);
+  const int32_t* pl = patterns + 4 * (nfactors - 1);
+  const int64_t n_out = static_cast<int64_t>(pl[0]) * pl[1] * pl[3];
+  const int64_t n_in = static_cast<int64_t>(patterns[0]) * patterns[2] * patterns[3];
+  const size_t one = train_buffer_bytes(nfactors, patterns, batch, dtype);
+  // a second version of the output's gradient: the other layout, or padded rows
+  const bool pad_copy = !plan.pre && bs_last && ld != batch;
+  const size_t second_bytes = plan.pre || pad_copy ? align_up(static_cast<size_t>(n_out) * ld * es, 256) : 0;
+  const bool post = need_input && plan.out_last[0] != bs_last;
+  const size_t post_bytes = post ? align_up(static_cast<size_t>(n_in) * ld * es, 256) : 0;
+  char* const dummy = reinterpret_cast<char*>(static_cast<uintptr_t>(1) << 20);
+  if (!run) ws = dummy;
+  char* second = ws;
+  char* gbuf = second + second_bytes;       // gradients of the intermediates, two alternating buffers
+  char* g0 = gbuf + 2 * one;                // the input's gradient before its transpose
+  char* tail = g0 + post_bytes;             // what one launch sequence needs for itself
+  size_t tail_bytes = 0;
+
+  // versions of the output's gradient
+  WgradOperand dy{run ? grad_output : dummy, bs_last, batch}, dy2 = dy;
+  if (plan.pre) dy2 = WgradOperand{second, !bs_last, !bs_last ? ld : 0};
+  if (pad_copy) dy2 = WgradOperand{second, 1, ld};
+  int st = KSMM_OK;
+  if (run && plan.pre)
+    st = bs_last ? launch_transpose(grad_output, second, n_out, batch, es, stream)
+                 : launch_transpose(grad_output, second, batch, n_out, es, stream, ld);
+  if (run && pad_copy) st = launch_copy_rows(grad_output, batch, second, ld, n_out, batch, es, stream);
+  if (st != KSMM_OK) return st;
+  if (grad_bias || !run) {
+    const WgradOperand& b = dy2.last ? dy2 : dy;  // row sums need no second launch
+    if (!b.last) tail_bytes = std::max(tail_bytes, bias_grad_workspace_bytes(n_out));
+    if (run) st = launch_bias_grad(b.ptr, b.last, b.last ? b.ld : 0, grad_bias, tail, batch, n_out, dtype, stream);
+    if (st != KSMM_OK) return st;
+  }
+  WgradOperand g = dy2;  // gradient of the current factor's output
+  for (int f = nfactors - 1; f >= 0; --f) {
+    const int32_t* q = patterns + 4 * f;
+    if (!run || grad_values[f]) {
+      Problem p = backward_problem(nullptr, nullptr, run ? grad_values[f] : dummy, batch, q[0], q[1], q[2], q[3], dtype, bs_last);
+      WgradOperand x{run ? input : dummy, bs_last, batch};
+      if (f > 0) {
+        x.ptr = run ? static_cast<const char*>(saved) + static_cast<size_t>(f - 1) * one : dummy;
+        x.last = layouts[f - 1] == 1;
+        x.ld = x.last ? ld : 0;
+        x.regrouped = layouts[f - 1] == 2;
+      }
+      WgradOperand gw = f == nfactors - 1 && dy.last && !pad_copy ? dy : g;
+      const size_t wneed = wgrad_workspace_bytes(p, x, gw);
+      tail_bytes = std::max(tail_bytes, wneed);
+      if (run) st = wgrad_launch(p, x, gw, tail, wneed, stream);
+      if (st != KSMM_OK) return st;
+    }
+    if (f == 0 && !need_input) break;
+    const size_t wt = align_up(static_cast<size_t>(q[0]) * q[1] * q[2] * q[3] * es, 256);
+    const bool to_input = f == 0 && !post;
+    const int64_t own_ld = plan.out_last[f] ? (to_input ? batch : ld) : 0;
+    void* dst = to_input ? (run ? grad_input : dummy) : (f == 0 ? g0 : gbuf + (f & 1) * one);
+    Problem p = backward_problem(g.ptr, tail, dst, batch, q[0], q[2], q[1], q[3], dtype, plan.in_last[f]);
+    if (plan.in_last[f] && g.ld != batch) p.in_ld = g.ld;
+    if (plan.out_last[f] && own_ld != batch) p.out_ld = own_ld;
+    if (p.in_ld && !p.out_ld && plan.out_last[f]) p.out_ld = batch;
+    p.no_alloc = 1;
+    const bool turns = plan.in_last[f] != plan.out_last[f];
+    if (turns) p.out_bs_last = plan.out_last[f];
+    const size_t sneed = turns ? 0 : scratch_need(p, auto_choice(p));
+    tail_bytes = std::max(tail_bytes, wt + sneed);
+    if (run) {
+      st = launch_transpose_blocks(values[f], tail, static_cast<int64_t>(q[0]) * q[3], q[2], q[1], es, stream);
+      if (st != KSMM_OK) return st;
+      if (sneed) {
+        p.scratch = tail + wt;
+        p.scratch_bytes = sneed;
+      }
+      st = turns ? run_family(p, KSMM_ALGO_TC, -1, stream) : dispatch(p, KSMM_ALGO_AUTO, -1, stream);
+      if (st != KSMM_OK) return st;
+    }
+    g = WgradOperand{dst, plan.out_last[f], own_ld};
+  }
+  if (run && post)
+    st = bs_last ? launch_transpose(g0, grad_input, batch, n_in, es, stream)
+                 : launch_transpose(g0, grad_input, n_in, batch, es, stream, 0, ld);
+  if (need) *need = second_bytes + 2 * one + post_bytes + align_up(tail_bytes, 256);
+  return st;
+}
+
+static int check_train(int nfactors, const int32_t* patterns, const void* const* values, int64_t batch, int dtype, int bs_last) {
+  int st = check_chain(nfactors, patterns, values, dtype, 0);
+  if (st != KSMM_OK) return st;
+  if (nfactors > ChainPlan::kMax)
+    return set_error(KSMM_ERR_UNSUPPORTED, "chains of more than %d factors", ChainPlan::kMax);
+  if (bs_last != 0 && bs_last != 1) return set_error(KSMM_ERR_BAD_ARGUMENT, "bs_last must be 0 or 1");
+  if (batch < 0) return set_error(KSMM_ERR_BAD_ARGUMENT, "negative batch");
+  return KSMM_OK;
+}
+
+static bool aligned16(const void* q) { return reinterpret_cast<uintptr_t>(q) % 16 == 0; }
+
+int ksmm_cu_chain_train_bytes(int nfactors, const int32_t* patterns, int64_t batch, int dtype, int bs_last,
+                              size_t* saved_bytes, size_t* forward_bytes, size_t* backward_bytes) {
+  const void* dummy = nullptr;
+  int st = check_train(nfactors, patterns, &dummy, batch, dtype, bs_last);
+  if (st != KSMM_OK) return st;
+  if (!saved_bytes || !forward_bytes || !backward_bytes) return set_error(KSMM_ERR_BAD_ARGUMENT, "null pointer");
+  *saved_bytes = *forward_bytes = *backward_bytes = 0;
+  if (batch == 0) return KSMM_OK;
+  const bool one_layout = train_one_layout(nfactors, patterns, batch, dtype, bs_last);
+  *saved_bytes = train_buffer_bytes(nfactors, patterns, batch, dtype) * (nfactors - 1);
+  for (int allow = 0; allow < (one_layout ? 1 : 2); ++allow) {
+    size_t need = 0;
+    int32_t layouts[ChainPlan::kMax] = {};
+    st = chain_walk(false, nullptr, nullptr, nullptr, nullptr, nullptr, *saved_bytes, nullptr, 0, 0, batch, nfactors, patterns,
+                    dtype, bs_last, bs_last, 0, nullptr, &need, allow, one_layout ? 2 : 1, nullptr, 1, layouts);
+    if (st != KSMM_OK) return st;
+    *forward_bytes = std::max(*forward_bytes, need);
+    // the intermediates' layouts decide which weight gradients copy: every one of them
+    for (int kind = 0; kind < 2; ++kind) {
+      for (int f = 0; f + 1 < nfactors && kind == 1; ++f) layouts[f] = one_layout ? bs_last : 0;
+      for (int need_input = 0; need_input < 2; ++need_input) {
+        st = chain_backward_walk(false, nullptr, nullptr, nullptr, layouts, nullptr, nullptr, nullptr, nullptr, nullptr, batch,
+                                 nfactors, patterns, dtype, bs_last, need_input != 0, allow != 0, one_layout, nullptr, &need);
+        if (st != KSMM_OK) return st;
+        *backward_bytes = std::max(*backward_bytes, need);
+      }
+    }
+  }
+  return KSMM_OK;
+}
+
+int ksmm_cu_chain_train_forward(const void* input, const void* const* values, void* output, const void* bias, void* saved,
+                                size_t saved_bytes, void* scratch, size_t scratch_bytes, int64_t batch, int nfactors,
+                                const int32_t* patterns, int dtype, int bs_last, int32_t* layouts, void* stream) {
+  size_t want[3];
+  int st = ksmm_cu_chain_train_bytes(nfactors, patterns, batch, dtype, bs_last, &want[0], &want[1], &want[2]);
+  if (st != KSMM_OK) return st;
+  if (batch == 0) return KSMM_OK;
+  if ((want[0] && (!saved || reinterpret_cast<uintptr_t>(saved) % 256 || saved_bytes < want[0])) ||
+      (want[1] && (!scratch || reinterpret_cast<uintptr_t>(scratch) % 256 || scratch_bytes < want[1])))
+    return set_error(KSMM_ERR_WORKSPACE, "training forward: need %zu bytes kept and %zu of scratch, aligned to 256", want[0],
+                     want[1]);
+  if (!layouts && nfactors > 1) return set_error(KSMM_ERR_BAD_ARGUMENT, "null layouts");
+  if (!input || !output) return set_error(KSMM_ERR_BAD_ARGUMENT, "null pointer");
+  const bool one_layout = train_one_layout(nfactors, patterns, batch, dtype, bs_last);
+  int allow = !one_layout && aligned16(input) && aligned16(output) ? 1 : 0;
+  for (int f = 0; f < nfactors; ++f) allow &= aligned16(values[f]) ? 1 : 0;
+  return chain_walk(true, input, values, output, bias, saved, want[0], scratch, scratch_bytes, /*no_alloc=*/1, batch, nfactors,
+                    patterns, dtype, bs_last, bs_last, 0, static_cast<cudaStream_t>(stream), nullptr, allow,
+                    one_layout ? 2 : 1, nullptr, /*keep=*/1, layouts);
+}
+
+int ksmm_cu_chain_backward(const void* input, const void* const* values, const void* saved, const int32_t* layouts,
+                           const void* grad_output, void* grad_input, void* const* grad_values, void* grad_bias,
+                           void* workspace, size_t workspace_bytes, int64_t batch, int nfactors, const int32_t* patterns,
+                           int dtype, int bs_last, void* stream) {
+  int st = check_train(nfactors, patterns, values, batch, dtype, bs_last);
+  if (st != KSMM_OK) return st;
+  if (!grad_values || (nfactors > 1 && !layouts)) return set_error(KSMM_ERR_BAD_ARGUMENT, "null pointer");
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (batch == 0) {
+    // sums over nothing
+    const int es = dtype_size(dtype);
+    const int32_t* pl = patterns + 4 * (nfactors - 1);
+    for (int f = 0; f < nfactors; ++f) {
+      const int32_t* q = patterns + 4 * f;
+      if (grad_values[f]) KSMM_CUDA_OK(cudaMemsetAsync(grad_values[f], 0, static_cast<size_t>(q[0]) * q[1] * q[2] * q[3] * es, s));
+    }
+    if (grad_bias) KSMM_CUDA_OK(cudaMemsetAsync(grad_bias, 0, static_cast<size_t>(pl[0]) * pl[1] * pl[3] * es, s));
+    return KSMM_OK;
+  }
+  if (!input || !grad_output || (nfactors > 1 && !saved)) return set_error(KSMM_ERR_BAD_ARGUMENT, "null pointer");
+  if (!aligned16(input) || !aligned16(grad_output))
+    return set_error(KSMM_ERR_BAD_ARGUMENT, "the backward of a chain takes an input and a gradient aligned to 16 bytes");
+  const bool one_layout = train_one_layout(nfactors, patterns, batch, dtype, bs_last);
+  bool allow = aligned16(grad_input);
+  for (int f = 0; f < nfactors; ++f) allow = allow && aligned16(values[f]);
+  size_t need = 0;
+  for (int run = 0; run < 2; ++run) {
+    st = chain_backward_walk(run != 0, input, values, saved, layouts, grad_output, grad_input, grad_values, grad_bias,
+                             static_cast<char*>(workspace), batch, nfactors, patterns, dtype, bs_last, grad_input != nullptr,
+                             allow, one_layout, s, run ? nullptr : &need);
+    if (st != KSMM_OK) return st;
+    if (!run && need && (!workspace || reinterpret_cast<uintptr_t>(workspace) % 256 || workspace_bytes < need))
+      return set_error(KSMM_ERR_WORKSPACE, "chain backward: need %zu bytes aligned to 256, got %zu", need, workspace_bytes);
+  }
+  return KSMM_OK;
 }
 
 int ksmm_cu_chain_forward_static(const void* input, const void* const* values, void* output,

@@ -64,8 +64,8 @@ class KSLinear(nn.Module):
                  requires_grad: bool = False, out_bs_last=None):
         super().__init__()
         # `requires_grad` is an addition as well: the reference's kernel path is inference-only (its
-        # backward is a stub).  With trainable factors the forward runs factor by factor through
-        # autograd (FactorFunction: dX and dW kernels of the library)
+        # backward is a stub).  With trainable factors the forward runs through autograd (ChainFunction:
+        # the dX, dW and bias-gradient kernels of the library)
         # `activation` (None, "gelu", "relu") is an addition to the reference's signature: it is applied
         # after the bias inside the last factor's epilogue instead of as a separate kernel
         if activation not in (None, "gelu", "relu"):
@@ -152,12 +152,16 @@ class KSLinear(nn.Module):
         if residual is None and torch.is_grad_enabled() and (
                 x.requires_grad or any(f.requires_grad for f in self.factors)
                 or (self.bias is not None and self.bias.requires_grad)):
-            # differentiable path: one autograd node per factor; bias and activation are torch ops
-            y = x
-            for p, f in zip(self.patterns, self.factors):
-                y = _k.FactorFunction.apply(y, f, self.bs_last, *p)
-            if self.bias is not None:
-                y = y + (self.bias.reshape(-1, 1) if self.bs_last else self.bias.reshape(1, -1))
+            # differentiable path: one autograd node for the factors and the bias (one per factor for very
+            # long chains); the activation is a torch op
+            if self.num_mat <= 16:
+                y = _k.ChainFunction.apply(x, self.bias, self.bs_last, self.patterns, *self.factors)
+            else:
+                y = x
+                for p, f in zip(self.patterns, self.factors):
+                    y = _k.FactorFunction.apply(y, f, self.bs_last, *p)
+                if self.bias is not None:
+                    y = y + (self.bias.reshape(-1, 1) if self.bs_last else self.bias.reshape(1, -1))
             if self.out_bs_last != bool(self.bs_last):
                 y = y.t().contiguous()
             if self.activation == "gelu":

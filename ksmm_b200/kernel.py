@@ -151,6 +151,23 @@ def forward(input, factor, bs_last, a, b, c, d, dtype, vsize=4):
     return Kernel.forward(input, factor, bool(bs_last), a, b, c, d, dtype, vsize)
 
 
+def _check_chain(input, factors, patterns, bs_last):
+    if not patterns or len(factors) != len(patterns):
+        raise ValueError("need one factor per pattern")
+    for f, (p, w) in enumerate(zip(patterns, factors)):
+        a, b, c, d = p
+        if f == 0:
+            _check_inputs(input, w, bs_last, a, b, c, d)
+        elif tuple(w.shape) != (a * d * c, b) or w.dtype != input.dtype or not w.is_contiguous() \
+                or w.device != input.device:
+            raise ValueError(f"factor {f} must be a contiguous ({a * d * c}, {b}) tensor of {input.dtype}")
+
+
+def _aligned(t):
+    """``t``, or a copy of it where it starts between two 16-byte pieces."""
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def chain_forward(input, factors, patterns, bs_last, bias=None, workspace=None, out=None,
                   activation=None, out_bs_last=None, residual=None):
     """All factors of one KSLinear in one library call (``ksmm_cu_chain_forward_layouts``).
@@ -166,15 +183,7 @@ def chain_forward(input, factors, patterns, bs_last, bias=None, workspace=None, 
     bs_last = int(bool(bs_last))
     out_last = bs_last if out_bs_last is None else int(bool(out_bs_last))
     nf = len(patterns)
-    if nf == 0 or len(factors) != nf:
-        raise ValueError("need one factor per pattern")
-    for f, (p, w) in enumerate(zip(patterns, factors)):
-        a, b, c, d = p
-        if f == 0:
-            _check_inputs(input, w, bs_last, a, b, c, d)
-        elif tuple(w.shape) != (a * d * c, b) or w.dtype != input.dtype or not w.is_contiguous() \
-                or w.device != input.device:
-            raise ValueError(f"factor {f} must be a contiguous ({a * d * c}, {b}) tensor of {input.dtype}")
+    _check_chain(input, factors, patterns, bs_last)
     batch = input.shape[1] if bs_last else input.shape[0]
     la, lb, lc, ld = patterns[-1]
     n_out = la * lb * ld
@@ -359,6 +368,59 @@ class FactorFunction(torch.autograd.Function):
         if ctx.needs_input_grad[1]:
             grad_factor = backward_weights(input.detach(), grad_output, bs_last, a, b, c, d)
         return grad_input, grad_factor, None, None, None, None, None
+
+
+class ChainFunction(torch.autograd.Function):
+    """All factors of a layer and its bias as one differentiable operation: one library call forward
+    (``ksmm_cu_chain_train_forward``, which keeps the intermediates in the layouts it plans) and one backward
+    (``ksmm_cu_chain_backward``)."""
+
+    @staticmethod
+    def forward(ctx, input, bias, bs_last, patterns, *factors):
+        lib = _lib.load()
+        bs_last = int(bool(bs_last))
+        _check_chain(input, factors, patterns, bs_last)
+        input = _aligned(input)
+        nf = len(patterns)
+        batch = input.shape[1] if bs_last else input.shape[0]
+        n_out = patterns[-1][0] * patterns[-1][1] * patterns[-1][3]
+        if bias is not None and (bias.numel() != n_out or bias.dtype != input.dtype or not bias.is_contiguous()
+                                 or bias.device != input.device):
+            raise ValueError("bias must hold out_size contiguous elements of the input dtype")
+        pat = _lib.int32_array([v for p in patterns for v in p])
+        code = dtype_code(input.dtype)
+        sizes = (ctypes.c_size_t * 3)()
+        at = [ctypes.cast(ctypes.byref(sizes, 8 * q), ctypes.POINTER(ctypes.c_size_t)) for q in range(3)]
+        _lib.check(lib.ksmm_cu_chain_train_bytes(nf, pat, batch, code, bs_last, *at))
+        out = torch.empty((n_out, batch) if bs_last else (batch, n_out), dtype=input.dtype, device=input.device)
+        saved = torch.empty(sizes[0], dtype=torch.uint8, device=input.device)
+        scratch = torch.empty(sizes[1], dtype=torch.uint8, device=input.device)
+        layouts = (ctypes.c_int32 * max(nf - 1, 1))()
+        vals = (ctypes.c_void_p * nf)(*[w.data_ptr() for w in factors])
+        with torch.cuda.device(input.device):
+            _lib.check(lib.ksmm_cu_chain_train_forward(
+                input.data_ptr(), vals, out.data_ptr(), bias.data_ptr() if bias is not None else None, saved.data_ptr(),
+                sizes[0], scratch.data_ptr(), sizes[1], batch, nf, pat, code, bs_last, layouts, _stream_ptr(input.device)))
+        ctx.save_for_backward(input, saved, *factors)
+        ctx.chain = (bs_last, nf, pat, batch, code, layouts, int(sizes[2]), bias.shape if bias is not None else None)
+        return out
+
+    @staticmethod
+    def backward(ctx, grad_output):
+        input, saved, *factors = ctx.saved_tensors
+        bs_last, nf, pat, batch, code, layouts, need, bias_shape = ctx.chain
+        grad_output = _aligned(grad_output.contiguous())
+        grad_input = torch.empty_like(input) if ctx.needs_input_grad[0] else None
+        grad_bias = torch.empty(bias_shape, dtype=input.dtype, device=input.device) if ctx.needs_input_grad[1] else None
+        grads = [torch.empty_like(w) if n else None for w, n in zip(factors, ctx.needs_input_grad[4:])]
+        ws = torch.empty(need, dtype=torch.uint8, device=input.device)
+        ptr = [None if t is None else t.data_ptr() for t in (grad_input, grad_bias, *grads)]
+        with torch.cuda.device(input.device):
+            _lib.check(_lib.load().ksmm_cu_chain_backward(
+                input.data_ptr(), (ctypes.c_void_p * nf)(*[w.data_ptr() for w in factors]), saved.data_ptr(), layouts,
+                grad_output.data_ptr(), ptr[0], (ctypes.c_void_p * nf)(*ptr[2:]), ptr[1], ws.data_ptr(), need, batch, nf,
+                pat, code, bs_last, _stream_ptr(input.device)))
+        return grad_input, grad_bias, None, None, *grads
 
 
 def quantize_e4m3(t):

@@ -1372,3 +1372,68 @@ def test_fp8_chain_quantises_as_quantize_e4m3(patterns, bs_last, in_dtype):
     x.view(-1)[5] = float("nan")
     assert bool(torch.isnan(layer(x.to(in_dtype))).any())
     kb.check_device()
+
+
+# ---------------------------------------------------------------------------
+# a layer's forward and backward as one chain: layouts, ragged batches, what is asked for
+# ---------------------------------------------------------------------------
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("patterns", [[(6, 64, 64, 1), (1, 96, 192, 2)], [(4, 48, 48, 1), (1, 192, 48, 4)],
+                                      [(1, 96, 192, 4), (4, 64, 96, 1)], [(1, 64, 64, 16), (4, 64, 64, 4), (16, 64, 64, 1)],
+                                      [(2, 24, 10, 3), (1, 12, 48, 3)], [(1, 130, 70, 2)]])
+@pytest.mark.parametrize("bs_last", [False, True])
+def test_chain_gradients(patterns, bs_last, dtype):
+    """Against fp64 autograd on dense matrices of the same values.  16-bit intermediates are rounded
+    between the factors: one rounding step each way."""
+    tol = {torch.float32: 1e-5, torch.float16: 4e-3, torch.bfloat16: 3e-2}[dtype]
+    layer = kb.KSLinear(patterns, dtype=dtype, bs_last=bs_last, device=DEV, requires_grad=True)
+    dense = [kb.from_kernel_format_to_dense(f.data.double(), p) for f, p in zip(layer.factors, patterns)]
+    for batch in (1, 40, 197, 640):
+        gen = torch.Generator(device=DEV).manual_seed(batch)
+        x = torch.randn((layer.in_size, batch) if bs_last else (batch, layer.in_size), device=DEV, generator=gen).to(dtype)
+        g = torch.randn((layer.out_size, batch) if bs_last else (batch, layer.out_size), device=DEV, generator=gen).to(dtype)
+        # what autograd gives from one factor at a time
+        xr = x.clone().requires_grad_(True)
+        fr = [f.detach().clone().requires_grad_(True) for f in layer.factors]
+        y = xr
+        for p, f in zip(patterns, fr):
+            y = kb.FactorFunction.apply(y, f, bs_last, *p)
+        y.backward(g)
+        for want_x in (True, False):
+            layer.zero_grad(set_to_none=True)
+            xi = x.clone().requires_grad_(want_x)
+            out = layer(xi)
+            out.backward(g)
+            h = (x if bs_last else x.t()).double()
+            for m in dense:
+                h = m @ h
+            ref = h + layer.bias.detach().double().reshape(-1, 1)
+            got = [("y", out.detach() if bs_last else out.detach().t(), ref),
+                   ("bias", layer.bias.grad.reshape(-1), (g if bs_last else g.t()).double().sum(1))]
+            if want_x:
+                gx = (g if bs_last else g.t()).double()
+                for m in reversed(dense):
+                    gx = m.t() @ gx
+                got.append(("x", xi.grad if bs_last else xi.grad.t(), gx))
+            got += [(f"w{q}", f.grad, r.grad.double()) for q, (f, r) in enumerate(zip(layer.factors, fr))]
+            for name, v, r in got:
+                err = (torch.linalg.norm(v.double() - r) / torch.linalg.norm(r)).item()
+                assert err < tol, (name, batch, want_x, err)
+    kb.check_device()
+
+
+def test_chain_gradients_of_frozen_parts():
+    """Only what is asked for is computed; an empty batch has zero gradients."""
+    layer = kb.KSLinear([(4, 48, 48, 1), (1, 192, 48, 4)], dtype=torch.float16, device=DEV, requires_grad=True)
+    layer.factors[1].requires_grad_(False)
+    layer.bias.requires_grad_(False)
+    x = torch.randn(70, layer.in_size, device=DEV, dtype=torch.float16)
+    layer(x).sum().backward()
+    assert layer.factors[0].grad is not None and layer.factors[1].grad is None and layer.bias.grad is None
+    layer.zero_grad(set_to_none=True)
+    layer(x[:0]).sum().backward()
+    assert not layer.factors[0].grad.any()
+    shifted = torch.randn(70 * layer.in_size + 1, device=DEV, dtype=torch.float16)[1:].view(70, -1).requires_grad_(True)
+    layer(shifted).sum().backward()   # starts between two 16-byte pieces
+    assert shifted.grad.shape == shifted.shape
+    kb.check_device()
