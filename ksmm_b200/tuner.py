@@ -271,6 +271,8 @@ def load_default():
     Set KSMM_NO_TUNED_TABLE=1 to start from the heuristic alone."""
     if _os.environ.get("KSMM_NO_TUNED_TABLE") or not _os.path.exists(DEFAULT_TABLE):
         return 0
+    if not _os.path.exists(_lib.LIB_PATH):
+        return 0  # nothing to push it into yet: the package is being built
     return load(DEFAULT_TABLE)
 
 
