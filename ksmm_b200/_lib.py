@@ -46,6 +46,23 @@ EXPORTS = (
 )
 
 
+def _load_native():
+    """The extension module that ``build.build_torch_extension`` compiles (csrc/torch_ext.cpp), or None where it
+    has not been built: every call then goes through ctypes, to the same library, with more host time."""
+    if not os.path.exists(LIB_PATH):
+        return None
+    try:
+        import torch  # noqa: F401  (libtorch must be loaded before the module)
+
+        from . import ksmm_torch_ext
+    except ImportError:
+        return None
+    return ksmm_torch_ext if hasattr(ksmm_torch_ext, "layer_train") else None
+
+
+native = _load_native()
+
+
 class ForwardDesc(ctypes.Structure):
     """Mirror of ksmm_forward_desc_t."""
     _fields_ = [

@@ -21,6 +21,7 @@ import math
 import torch
 from torch import nn
 
+from . import _lib
 from . import kernel as _k
 
 
@@ -131,6 +132,12 @@ class KSLinear(nn.Module):
         return self._fp8_cache
 
     def _forward_2d(self, x, residual=None):
+        if _lib.native is not None and not self.is_fp8 and (self.fuse_chain or self.num_mat == 1):
+            # one call of the extension module; None where it is not for it (gradients, a wrong argument)
+            y = _lib.native.layer_forward(x, list(self.factors), self.patterns, bool(self.bs_last),
+                                          self.out_bs_last, self.bias, _lib.ACTIVATIONS[self.activation], residual)
+            if y is not None:
+                return _k._result(y)
         bias = None if self.bias is None else self.bias.reshape(-1)
         if self.is_fp8:
             quantised = self._fp8_factors()
@@ -155,7 +162,7 @@ class KSLinear(nn.Module):
             # differentiable path: one autograd node for the factors and the bias (one per factor for very
             # long chains); the activation is a torch op
             if self.num_mat <= 16:
-                y = _k.ChainFunction.apply(x, self.bias, self.bs_last, self.patterns, *self.factors)
+                y = _k.chain_train(x, list(self.factors), self.patterns, self.bs_last, self.bias)
             else:
                 y = x
                 for p, f in zip(self.patterns, self.factors):
@@ -184,7 +191,6 @@ class KSLinear(nn.Module):
         return y
 
     def _ensure_workspace(self, x):
-        from . import _lib
         lib = _lib.load()
         batch = x.shape[1] if self.bs_last else x.shape[0]
         flat = [v for p in self.patterns for v in p]

@@ -22,6 +22,7 @@ import ctypes
 import torch
 
 from . import _lib
+from ._lib import native as _native
 from ._lib import ForwardDesc, KsmmError  # noqa: F401
 
 _DTYPE_CODE = {
@@ -143,7 +144,18 @@ class Kernel:
             code = dtype_code(dtype)
             if code != dtype_code(input.dtype):
                 raise TypeError(f"dtype argument {dtype} does not match the input's {input.dtype}")
+        if _native is not None and isinstance(input, torch.Tensor) and isinstance(factor, torch.Tensor):
+            out = _native.factor_forward(input, factor, bool(bs_last), a, b, c, d)
+            if out is not None:
+                return _result(out)
         return forward_ex(input, factor, bs_last, a, b, c, d)
+
+
+def _result(out):
+    """What a call of the extension module gave: a tensor, or a status of the library."""
+    if isinstance(out, int):
+        _lib.check(out)
+    return out
 
 
 def forward(input, factor, bs_last, a, b, c, d, dtype, vsize=4):
@@ -221,6 +233,10 @@ def chain_forward_fp8(input, factors, scales, patterns, bs_last, bias=None):
     """All factors of an fp8 KSLinear in one library call (``ksmm_cu_chain_forward_fp8``): ``factors[f]`` and
     ``scales[f]`` come from ``quantize_e4m3``; every factor's input is quantised on the device the way
     ``quantize_e4m3`` does it.  ``input``: fp32, fp16 or bf16; the result and ``bias`` are bf16."""
+    if _native is not None:
+        out = _native.fp8_forward(input, factors, scales, patterns, bool(bs_last), bias)
+        if out is not None:
+            return _result(out)
     lib = _lib.load()
     bs_last = int(bool(bs_last))
     nf = len(patterns)
@@ -255,6 +271,10 @@ def grouped_chain_forward(input, stacked_factors, patterns, bs_last, groups, bia
     ``stacked_factors[f]`` is the (groups * a*d*c, b) concatenation of the groups' kernel-format
     factors f.  Returns the stacked output (groups, out, batch) / (groups, batch, out); ``out[g]`` is
     group g's result, a contiguous tensor."""
+    if _native is not None and isinstance(groups, int):
+        out = _native.grouped_forward(input, list(stacked_factors), patterns, bool(bs_last), groups, bias)
+        if out is not None:
+            return _result(out)
     lib = _lib.load()
     bs_last = int(bool(bs_last))
     nf = len(patterns)
@@ -421,6 +441,15 @@ class ChainFunction(torch.autograd.Function):
                 grad_output.data_ptr(), ptr[0], (ctypes.c_void_p * nf)(*ptr[2:]), ptr[1], ws.data_ptr(), need, batch, nf,
                 pat, code, bs_last, _stream_ptr(input.device)))
         return grad_input, grad_bias, None, None, *grads
+
+
+def chain_train(input, factors, patterns, bs_last, bias=None):
+    """The factors and the bias of a trainable layer as one autograd node."""
+    if _native is not None:
+        out = _native.layer_train(input, factors, patterns, bool(bs_last), bias)
+        if out is not None:
+            return out
+    return ChainFunction.apply(input, bias, bs_last, patterns, *factors)
 
 
 def quantize_e4m3(t):

@@ -1437,3 +1437,53 @@ def test_chain_gradients_of_frozen_parts():
     layer(shifted).sum().backward()   # starts between two 16-byte pieces
     assert shifted.grad.shape == shifted.shape
     kb.check_device()
+
+
+# ---------------------------------------------------------------------------
+# the extension module's calls against the same calls through ctypes
+# ---------------------------------------------------------------------------
+@pytest.mark.parametrize("bs_last", [False, True])
+def test_extension_calls_match_ctypes(bs_last, monkeypatch):
+    """The same library calls: the same bits.  Arguments that do not fit raise what they raised."""
+    from ksmm_b200 import kernel as kk
+    assert _lib.native is not None, "ksmm_torch_ext has not been built"
+    pats = [(4, 48, 48, 1), (1, 192, 48, 4)]
+    gen = torch.Generator(device=DEV).manual_seed(5)
+
+    def make(batch, feats, dtype):
+        return torch.randn((feats, batch) if bs_last else (batch, feats), device=DEV, generator=gen).to(dtype)
+
+    layer = kb.KSLinear(pats, dtype=torch.float16, bs_last=bs_last, device=DEV, activation="gelu")
+    train = kb.KSLinear(pats, dtype=torch.float16, bs_last=bs_last, device=DEV, requires_grad=True)
+    fp8 = kb.KSLinear(pats, dtype=torch.float8_e4m3fn, bs_last=bs_last, device=DEV)
+    group = kb.KSLinearGroup([kb.KSLinear(pats, dtype=torch.float16, bs_last=bs_last, device=DEV) for _ in range(3)])
+
+    def results(batch):
+        gen.manual_seed(batch)
+        x = make(batch, 192, torch.float16)
+        res = make(batch, 768, torch.float16)
+        out = [layer(x), layer(x, residual=res), fp8(x.bfloat16()), *group(x),
+               kb.Kernel.forward(x, layer.factors[0], bs_last, *pats[0], "torch.float16")]
+        train.zero_grad(set_to_none=True)
+        xg = x.clone().requires_grad_(True)
+        y = train(xg)
+        y.backward(res)
+        return out + [y.detach(), xg.grad, train.bias.grad] + [f.grad for f in train.factors]
+
+    for batch in (1, 96, 197):
+        fast = results(batch)
+        with monkeypatch.context() as m:
+            m.setattr(_lib, "native", None)
+            m.setattr(kk, "_native", None)
+            slow = results(batch)
+        for a, b in zip(fast, slow):
+            assert a.shape == b.shape and a.dtype == b.dtype and torch.equal(a, b), batch
+    with pytest.raises(ValueError):
+        kb.Kernel.forward(make(8, 100, torch.float16), layer.factors[0], bs_last, *pats[0], "torch.float16")
+    with pytest.raises(ValueError):
+        layer(make(8, 100, torch.float16))
+    with pytest.raises(TypeError):
+        layer(make(8, 192, torch.float32))
+    with pytest.raises(ValueError):
+        layer(make(8, 192, torch.float16).cpu())
+    kb.check_device()
