@@ -24,7 +24,7 @@
 // dimension, so each epilogue thread owns a run of consecutive output
 // elements: it converts them, writes 16-byte chunks into a 128-byte-swizzled
 // staging tile, and one thread issues a TMA store of the tile.  The epilogue
-// applies alpha, the bias (one coalesced load per tile, broadcast by shuffles) and
+// applies alpha, the bias (batch-first: staged once per tile, see tc_epilogue.cuh) and
 // an optional activation; in a chain it can store a batch-first 16-bit output
 // regrouped by the blocks of the next factor (see tc_bsfirst_dp.cu).
 //
@@ -51,6 +51,7 @@
 
 #include <mutex>
 
+#include "tc_epilogue.cuh"
 #include "tc_kernel.h"
 #include "tc_host.h"
 #include "tc_ptx.cuh"
@@ -373,47 +374,25 @@ __global__ void __launch_bounds__(kThreads, Cfg<IN_LAST, OUT_LAST, ES, OS, NT, K
           tmem_ld_wait();
           if (tron) KSMM_TRACE(trole, 23);
           if (!plain) {
-            // batch-first: the bias of the tile's columns comes through one coalesced load per lane
-            // and shuffles (16-bit: columns 2 lane, 2 lane + 1; fp32: column lane);
-            // batch-last: one value per accumulator row
-            uint32_t braw = 0;
+            auto val = [&](int e) -> uint32_t& { return r[e]; };
             if (!BS_LAST && P.bias != nullptr) {
-              const int col = cbi * C::CB + (OS == 2 ? 2 * lane : lane);
-              if (col < col_limit) {
-                const int64_t e0 = bias0 + static_cast<int64_t>(i) * P.b + j0 + col;
-                if constexpr (OS == 2) {
-                  // (col_limit is even for 16-bit outputs: b * 2 bytes is a multiple of 16)
-                  const uint16_t* bp = static_cast<const uint16_t*>(P.bias) + e0;
-                  braw = (reinterpret_cast<uintptr_t>(bp) & 3) == 0
-                             ? *reinterpret_cast<const uint32_t*>(bp)
-                             : (static_cast<uint32_t>(bp[0]) | (static_cast<uint32_t>(bp[1]) << 16));
-                } else {
-                  braw = static_cast<const uint32_t*>(P.bias)[e0];
-                }
+              // the columns' bias passes through the staging tile, which is free here
+              const int64_t e0 = bias0 + static_cast<int64_t>(i) * P.b + j0 + cbi * C::CB;
+              const int exist = col_limit - cbi * C::CB;
+              if constexpr (OS == 2) {
+                // (an even number of columns exists: b * 2 bytes is a multiple of 16)
+                stage_bias_16<1>(P.bias, e0, 2 * lane < exist, P.out_dtype, stg, lane);
+              } else {
+                const float bv = lane < exist ? static_cast<const float*>(P.bias)[e0 + lane] : 0.f;
+                asm volatile("st.shared.f32 [%0], %1;" ::"r"(stg + lane * 4), "f"(bv) : "memory");
               }
+              __syncwarp();
+              scale_and_bias<C::CB>(val, alpha, stg);
+              __syncwarp();
+            } else {
+              scale_and_add<C::CB>(val, alpha, bias_row);
             }
-#pragma unroll
-            for (int e = 0; e < C::CB; ++e) {
-              float bv = bias_row;
-              if (!BS_LAST) {
-                if constexpr (OS == 2) {
-                  const uint32_t pr = __shfl_sync(0xffffffffu, braw, e >> 1);
-                  const uint16_t hv = static_cast<uint16_t>((e & 1) ? (pr >> 16) : (pr & 0xffffu));
-                  bv = P.out_dtype == KSMM_BF16 ? __uint_as_float(static_cast<uint32_t>(hv) << 16)
-                                                : __half2float(__ushort_as_half(hv));
-                } else {
-                  bv = __uint_as_float(__shfl_sync(0xffffffffu, braw, e));
-                }
-              }
-              r[e] = __float_as_uint(fmaf(alpha, __uint_as_float(r[e]), bv));
-            }
-            if (P.act == KSMM_ACT_GELU) {
-#pragma unroll
-              for (int e = 0; e < C::CB; ++e) r[e] = __float_as_uint(OS == 2 ? gelu_16bit(__uint_as_float(r[e])) : apply_activation(__uint_as_float(r[e]), 1));
-            } else if (P.act == KSMM_ACT_RELU) {
-#pragma unroll
-              for (int e = 0; e < C::CB; ++e) r[e] = __float_as_uint(fmaxf(__uint_as_float(r[e]), 0.f));
-            }
+            activate<C::CB, OS == 2>(val, P.act);
           }
           if (P.residual != nullptr && q * 32 + lane < row_limit) {
             // this thread's CB outputs are consecutive in memory (128 bytes): eight 16-byte loads
