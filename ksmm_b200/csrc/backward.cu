@@ -625,12 +625,12 @@ __global__ void __launch_bounds__(256)
   }
 }
 template <typename T>
-__global__ void __launch_bounds__(256) bias_grad_sum_kernel(const float* __restrict__ part, T* __restrict__ out, int64_t feats) {
+__global__ void __launch_bounds__(256) bias_grad_sum_kernel(const float* __restrict__ part, int slices, T* __restrict__ out, int64_t feats) {
   const int64_t f = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
   if (f >= feats) return;
   float s = 0.f;
 #pragma unroll 8
-  for (int q = 0; q < kBiasSlices; ++q) s += part[q * feats + f];
+  for (int q = 0; q < slices; ++q) s += part[q * feats + f];
   out[f] = ElemTraits<T>::from_float(s);
 }
 
@@ -651,7 +651,7 @@ int bias_grad_typed(const T* g, int last, int64_t ld, T* out, float* part, int64
     if (vec) bias_grad_cols_kernel<T, V><<<grid, 256, 0, stream>>>(g, part, batch, feats);
     else bias_grad_cols_kernel<T, 1><<<grid, 256, 0, stream>>>(g, part, batch, feats);
     count_launch();
-    bias_grad_sum_kernel<T><<<static_cast<unsigned>((feats + 255) / 256), 256, 0, stream>>>(part, out, feats);
+    bias_grad_sum_kernel<T><<<static_cast<unsigned>((feats + 255) / 256), 256, 0, stream>>>(part, kBiasSlices, out, feats);
   }
   count_launch();
   cudaError_t err = cudaGetLastError();
@@ -672,6 +672,17 @@ int launch_bias_grad(const void* g, int last, int64_t ld, void* out, void* works
     return bias_grad_typed(static_cast<const __half*>(g), last, ld, static_cast<__half*>(out), part, batch, feats, stream);
   return bias_grad_typed(static_cast<const __nv_bfloat16*>(g), last, ld, static_cast<__nv_bfloat16*>(out), part, batch,
                          feats, stream);
+}
+
+int launch_bias_sum(const float* part, int slices, void* out, int64_t feats, int dtype, cudaStream_t stream) {
+  const unsigned grid = static_cast<unsigned>((feats + 255) / 256);
+  if (dtype == KSMM_F32) bias_grad_sum_kernel<<<grid, 256, 0, stream>>>(part, slices, static_cast<float*>(out), feats);
+  else if (dtype == KSMM_F16) bias_grad_sum_kernel<<<grid, 256, 0, stream>>>(part, slices, static_cast<__half*>(out), feats);
+  else bias_grad_sum_kernel<<<grid, 256, 0, stream>>>(part, slices, static_cast<__nv_bfloat16*>(out), feats);
+  count_launch();
+  cudaError_t err = cudaGetLastError();
+  if (err != cudaSuccess) return set_error(KSMM_ERR_CUDA, "bias-gradient launch failed: %s", cudaGetErrorString(err));
+  return KSMM_OK;
 }
 
 size_t wgrad_workspace_bytes(const Problem& p, const WgradOperand& x, const WgradOperand& g) {

@@ -28,6 +28,8 @@ int wgrad_launch(const Problem& p, WgradOperand x, WgradOperand g, void* workspa
 size_t bias_grad_workspace_bytes(int64_t feats);
 int launch_bias_grad(const void* g, int last, int64_t ld, void* out, void* workspace, int64_t batch, int64_t feats,
                      int dtype, cudaStream_t stream);
+// the same from fp32 partial sums (slices, feats)
+int launch_bias_sum(const float* part, int slices, void* out, int64_t feats, int dtype, cudaStream_t stream);
 // the weight gradient of such a factor runs on the tensor cores for every pair of operand layouts
 bool wgrad_any_layout(const Problem& p);
 // the fp32 tensor-core kernel: partial tiles (splits, a*d, c, b) into `part`; nt = 64 or 128 columns
@@ -36,7 +38,9 @@ int wgrad_f32_launch(const Problem& p, const WgradOperand& x, const WgradOperand
 
 // in: rows x cols with row stride in_ld (0 = cols), out: cols x rows with row stride out_ld (0 = rows)
 int launch_transpose(const void* in, void* out, int64_t rows, int64_t cols, int es, cudaStream_t stream,
-                     int64_t out_ld = 0, int64_t in_ld = 0);
+                     int64_t out_ld = 0, int64_t in_ld = 0, float* sums = nullptr, int sum_dtype = 0);
+// with `sums` (elements of sum_dtype): sums[t][col] over the rows of row tile t, fp32
+int transpose_row_tiles(int64_t rows, int es);
 // rows x cols from row stride in_ld to row stride out_ld (elements of es bytes); rows of the destination
 // are aligned to 16 bytes
 int launch_copy_rows(const void* in, int64_t in_ld, void* out, int64_t out_ld, int64_t rows, int64_t cols, int es,

@@ -1411,12 +1411,21 @@ static int chain_backward_walk(bool run, const void* input, const void* const* v
   if (plan.pre) dy2 = WgradOperand{second, !bs_last, !bs_last ? ld : 0};
   if (pad_copy) dy2 = WgradOperand{second, 1, ld};
   int st = KSMM_OK;
+  // the transpose of a batch-first gradient sums its columns on the way (12 us for 12544 x 3072 fp16 as a
+  // pass of its own)
+  const bool sum_on_way = plan.pre && !bs_last && (grad_bias || !run);
   if (run && plan.pre)
     st = bs_last ? launch_transpose(grad_output, second, n_out, batch, es, stream)
-                 : launch_transpose(grad_output, second, batch, n_out, es, stream, ld);
+                 : launch_transpose(grad_output, second, batch, n_out, es, stream, ld, 0,
+                                    sum_on_way ? reinterpret_cast<float*>(tail) : nullptr, dtype);
   if (run && pad_copy) st = launch_copy_rows(grad_output, batch, second, ld, n_out, batch, es, stream);
   if (st != KSMM_OK) return st;
-  if (grad_bias || !run) {
+  if (sum_on_way) {
+    const int slices = transpose_row_tiles(batch, es);
+    tail_bytes = std::max(tail_bytes, static_cast<size_t>(slices) * n_out * sizeof(float));
+    if (run) st = launch_bias_sum(reinterpret_cast<float*>(tail), slices, grad_bias, n_out, dtype, stream);
+    if (st != KSMM_OK) return st;
+  } else if (grad_bias || !run) {
     const WgradOperand& b = dy2.last ? dy2 : dy;  // row sums need no second launch
     if (!b.last) tail_bytes = std::max(tail_bytes, bias_grad_workspace_bytes(n_out));
     if (run) st = launch_bias_grad(b.ptr, b.last, b.last ? b.ld : 0, grad_bias, tail, batch, n_out, dtype, stream);
