@@ -14,6 +14,7 @@
 
 #include "backward.h"
 #include "common.cuh"
+#include "tc_host.h"
 #include "tc_kernel.h"
 
 namespace ksmm {
@@ -1209,22 +1210,61 @@ int ksmm_cu_grouped_chain_forward(const void* input, const void* const* values, 
   const size_t half1 = nfactors == 2 ? inter1 : inter1 / 2;  // one buffer of one group
   char* ws = static_cast<char*>(workspace);
   const void* cur = input;
+  bool regrouped = false;  // the intermediate in `cur` is in the block order of factor f
   for (int f = 0; f < nfactors; ++f) {
-    const int32_t* q = patterns + 4 * f;
     const bool last = (f + 1 == nfactors);
-    // the groups' copies of intermediate buffer (f & 1) are contiguous: a stacked tensor
-    void* dst = last ? output : ws + static_cast<size_t>(f & 1) * half1 * groups;
-    Problem p;
-    p.in = cur; p.w = values[f]; p.out = dst; p.bias = last ? bias : nullptr;
-    p.batch = batch; p.a = q[0]; p.b = q[1]; p.c = q[2]; p.d = q[3];
-    p.in_dtype = dtype; p.out_dtype = dtype; p.bs_last = bs_last; p.alpha = 1.f;
-    if (workspace && workspace_bytes > inter) {
-      p.scratch = ws + inter;
-      p.scratch_bytes = workspace_bytes - inter;
+    auto problem = [&](int g) {
+      const int32_t* q = patterns + 4 * g;
+      Problem p;
+      // the groups' copies of intermediate buffer (g & 1) are contiguous: a stacked tensor
+      p.in = g == f ? cur : ws + static_cast<size_t>((g - 1) & 1) * half1 * groups;
+      p.w = values[g];
+      p.out = g + 1 == nfactors ? output : ws + static_cast<size_t>(g & 1) * half1 * groups;
+      p.bias = g + 1 == nfactors ? bias : nullptr;
+      p.batch = batch; p.a = q[0]; p.b = q[1]; p.c = q[2]; p.d = q[3];
+      p.in_dtype = dtype; p.out_dtype = dtype; p.bs_last = bs_last; p.alpha = 1.f;
+      return p;
+    };
+    Problem p = problem(f);
+    // Two batch-first factors of which the second has interleaved blocks: the first stores its output in the
+    // block order of the second, which then needs no split in the kernel and runs the groups in one
+    // launch (the q, k and v projections of 12608 rows, 768 -> 768 bf16: 81 us group by group -> 39 us).
+    bool next_regrouped = false;
+    if (!last && !bs_last && !regrouped && groups > 1 && batch > 0 && patterns[4 * f + 3] == 1 &&
+        (patterns[4 * (f + 1) + 3] == 2 || patterns[4 * (f + 1) + 3] == 4)) {
+      Problem nx = problem(f + 1);
+      Choice ch;
+      const bool pinned = lookup_choice(p, &ch) || lookup_choice(nx, &ch);  // a tuned choice wins
+      Problem g = p;
+      g.groups = nx.groups = groups;
+      g.group_shared_input = f == 0 ? 1 : 0;
+      nx.group_shared_input = 0;
+      nx.in_regrouped = 1;
+      g.out_regroup_c = nx.c;
+      g.out_regroup_d = nx.d;
+      const int cfg = pinned || nx.b < 32 || nx.c < 16 || groups * ((nx.b + 63) / 64) > tc::num_sms() || !tc_can_regroup_output(g) || !tc_config_supported(nx, 1, true)
+                          ? -1
+                          : tc_default_config(g);
+      if (cfg >= 0) {
+        next_regrouped = true;
+        st = tc_launch(g, cfg, static_cast<cudaStream_t>(stream));
+      }
     }
-    st = grouped_factor(p, groups, f == 0 ? 1 : 0, static_cast<cudaStream_t>(stream));
+    if (regrouped) {
+      p.groups = groups;
+      p.group_shared_input = 0;
+      p.in_regrouped = 1;
+      st = tc_launch(p, 1, static_cast<cudaStream_t>(stream));
+    } else if (!next_regrouped) {
+      if (workspace && workspace_bytes > inter) {
+        p.scratch = ws + inter;
+        p.scratch_bytes = workspace_bytes - inter;
+      }
+      st = grouped_factor(p, groups, f == 0 ? 1 : 0, static_cast<cudaStream_t>(stream));
+    }
     if (st != KSMM_OK) return st;
-    cur = dst;
+    cur = p.out;
+    regrouped = next_regrouped;
   }
   return KSMM_OK;
 }

@@ -50,6 +50,7 @@ struct ParamsP {
   const void* bias;
   int out_dtype;
   int act;  // ksmm_activation_t
+  int groups;  // problems of this pattern, inputs, weights and outputs stacked (see tc_kernel.cu)
   int* status;
 };
 
@@ -136,8 +137,9 @@ __global__ void __launch_bounds__(kThreadsP, 1)
   grid_dep_launch();
 
   const int nkc = P.nkc;
-  const int tj = static_cast<int>(blockIdx.x % P.tiles_j);
-  const uint32_t rc = blockIdx.x / P.tiles_j;
+  const int tjg = static_cast<int>(blockIdx.x % (P.tiles_j * P.groups));
+  const int tj = tjg % P.tiles_j, grp_id = tjg / P.tiles_j;
+  const uint32_t rc = blockIdx.x / (P.tiles_j * P.groups);
   const uint32_t row_begin = static_cast<uint32_t>(static_cast<uint64_t>(rc) * P.rows / P.row_groups);
   const uint32_t row_end = static_cast<uint32_t>(static_cast<uint64_t>(rc + 1) * P.rows / P.row_groups);
   const int j0 = tj * C::NJ;
@@ -155,13 +157,13 @@ __global__ void __launch_bounds__(kThreadsP, 1)
             if (!mbar_wait<64>(free_bar(si), sph ^ 1u, abort_flag, P.status, 51)) { ok = false; break; }
             const uint32_t sb = stage0 + si * C::STAGE_BYTES;
             mbar_expect_tx(full_bar(si), C::STAGE_BYTES);
-            // regrouped input seen as (k, n, l, i): two tiles of 128 rows x 64 k
-            tma_load_4d(sb, &tmX, full_bar(si), kc * 64, n0, lp * 2, i);
+            // regrouped input seen as (k, n, l, i, group): two tiles of 128 rows x 64 k
+            tma_load_5d(sb, &tmX, full_bar(si), kc * 64, n0, lp * 2, i, grp_id);
             // weights (a*d*c, b) seen as (b, c, a*d): per 64 columns, two blocks of 64 k rows
 #pragma unroll
             for (int jb = 0; jb < C::NJ / 64; ++jb)
               tma_load_3d(sb + C::A_BYTES + jb * C::WJB_BYTES, &tmW, full_bar(si), j0 + jb * 64, kc * 64,
-                          i * D + lp * 2);
+                          (grp_id * P.a + i) * D + lp * 2);
             if (++si == ST) { si = 0; sph ^= 1u; }
           }
         }
@@ -262,7 +264,7 @@ __global__ void __launch_bounds__(kThreadsP, 1)
           // the bias of the tile's 64 columns passes through the staging tile, in the order of the accumulators
           auto val = [&](int e) -> uint32_t& { return r[e / JB][e % JB]; };
           if (P.bias != nullptr) {
-            stage_bias_16<D>(P.bias, (static_cast<int64_t>(i) * P.b + j0 + jj0) * D, j0 + jj0 + (2 * lane) / D < P.b, P.out_dtype,
+            stage_bias_16<D>(P.bias, ((static_cast<int64_t>(grp_id) * P.a + i) * P.b + j0 + jj0) * D, j0 + jj0 + (2 * lane) / D < P.b, P.out_dtype,
                           tile, lane);
             __syncwarp();
             scale_and_bias<64>(val, P.alpha, tile);
@@ -292,7 +294,7 @@ __global__ void __launch_bounds__(kThreadsP, 1)
         fence_proxy_async();
         __syncwarp();
         if (lane == 0) {
-          tma_store_3d(&tmY, tile, (j0 + jj0) * D, i, n0 + q * 32);
+          tma_store_4d(&tmY, tile, (j0 + jj0) * D, i, n0 + q * 32, grp_id);
           bulk_commit();
         }
         if (STGN > 1) sti = (sti + 1 == STGN) ? 0u : sti + 1;
@@ -337,29 +339,29 @@ static int launch_p(const Problem& p, const void* regrouped, cudaStream_t stream
                        C::SMEM_BYTES, cudaGetErrorString(e));
     attr_set[dev] = true;
   }
-  const uint64_t a = p.a, b = p.b, c = p.c, d = p.d, B = p.batch;
+  const uint64_t a = p.a, b = p.b, c = p.c, d = p.d, B = p.batch, G = p.groups;
   CUtensorMap tmX, tmW, tmY;
   int st;
   {
-    // regrouped input [n][i][l][k] seen as (k, n, l, i): box = two tiles of 128 rows x 64 k
-    const uint64_t dims[4] = {c, B, d, a};
-    const uint64_t str[4] = {1, a * c * d, c, c * d};
-    const uint32_t box[4] = {64, 128, 2, 1};
-    if ((st = encode_map(&tmX, p.in_dtype, 4, regrouped, dims, str, box, true)) != KSMM_OK) return st;
+    // regrouped input [group][n][i][l][k] seen as (k, n, l, i, group): box = two tiles of 128 rows x 64 k
+    const uint64_t dims[5] = {c, B, d, a, G};
+    const uint64_t str[5] = {1, a * c * d, c, c * d, B * a * c * d};
+    const uint32_t box[5] = {64, 128, 2, 1, 1};
+    if ((st = encode_map(&tmX, p.in_dtype, 5, regrouped, dims, str, box, true)) != KSMM_OK) return st;
   }
   {
     // weights (a*d*c, b) row-major seen as (b, c, a*d); box = 64 j x 64 k rows x two blocks
-    const uint64_t dims[3] = {b, c, a * d};
+    const uint64_t dims[3] = {b, c, G * a * d};
     const uint64_t str[3] = {1, b, c * b};
     const uint32_t box[3] = {64, 64, 2};
     if ((st = encode_map(&tmW, p.in_dtype, 3, p.w, dims, str, box, true)) != KSMM_OK) return st;
   }
   {
     // output rows: (b*d, a, batch); one epilogue warp stores 64 elements x 32 rows
-    const uint64_t dims[3] = {b * d, a, B};
-    const uint64_t str[3] = {1, b * d, a * b * d};
-    const uint32_t box[3] = {64, 1, 32};
-    if ((st = encode_map(&tmY, p.out_dtype, 3, p.out, dims, str, box, true)) != KSMM_OK) return st;
+    const uint64_t dims[4] = {b * d, a, B, G};
+    const uint64_t str[4] = {1, b * d, a * b * d, B * a * b * d};
+    const uint32_t box[4] = {64, 1, 32, 1};
+    if ((st = encode_map(&tmY, p.out_dtype, 4, p.out, dims, str, box, true)) != KSMM_OK) return st;
   }
   ParamsP P;
   P.a = p.a; P.b = p.b; P.c = p.c; P.d = p.d;
@@ -371,6 +373,7 @@ static int launch_p(const Problem& p, const void* regrouped, cudaStream_t stream
   P.bias = p.bias;
   P.out_dtype = p.out_dtype;
   P.act = p.activation;
+  P.groups = p.groups;
   P.status = status_word();
   if (!P.status) return set_error(KSMM_ERR_CUDA, "cannot resolve the device status word");
   const uint32_t fmt = p.in_dtype == KSMM_BF16 ? 1u : 0u;
@@ -380,13 +383,14 @@ static int launch_p(const Problem& p, const void* regrouped, cudaStream_t stream
   const int sms = num_sms();
   if (sms <= 0) return set_error(KSMM_ERR_NO_DEVICE, "no CUDA device");
   const int64_t rows = static_cast<int64_t>(P.tiles_n) * p.a;
-  if (rows <= 0 || rows > 0x7fffffffLL || P.tiles_j > sms)
+  const int tiles_jg = P.tiles_j * p.groups;
+  if (rows <= 0 || rows > 0x7fffffffLL || tiles_jg > sms)
     return set_error(KSMM_ERR_UNSUPPORTED, "tensor-core family: work-split limits exceeded");
   P.rows = static_cast<uint32_t>(rows);
-  int64_t groups = sms / P.tiles_j;
+  int64_t groups = sms / tiles_jg;
   if (groups > rows) groups = rows;
   P.row_groups = static_cast<uint32_t>(groups);
-  const unsigned grid = static_cast<unsigned>(groups * P.tiles_j);
+  const unsigned grid = static_cast<unsigned>(groups * tiles_jg);
   cudaError_t err = launch_pdl(kern, grid, kThreadsP, C::SMEM_BYTES, stream, tmX, tmW, tmY, P);
   count_launch();
   if (err == cudaSuccess) err = cudaGetLastError();

@@ -205,11 +205,12 @@ __global__ void __launch_bounds__(kThreads, Cfg<IN_LAST, OUT_LAST, ES, OS, NT, K
   const uint32_t row_end = static_cast<uint32_t>(static_cast<uint64_t>(rc + 1) * P.rows / P.row_groups);
   const int j0 = tj * (BS_LAST ? 128 : NT);
   // offsets of this CTA's group in the stacked tensors: weight blocks, block rows of a batch-last
-  // input / output, batch rows of a batch-first input / output, bias elements
+  // input / output, batch rows of a batch-first input (a batch-first output has the group as a
+  // dimension of its map, so that its last rows are clipped at the group's end), bias elements
   const int wblk0 = grp_id * P.a * P.d;
   const int xi0 = P.gx ? grp_id * P.a : 0, yi0 = grp_id * P.a;
-  const int xn0 = P.gx ? grp_id * static_cast<int>(P.batch) : 0, yn0 = grp_id * static_cast<int>(P.batch);
-  (void)xi0; (void)xn0; (void)yi0; (void)yn0;
+  const int xn0 = P.gx ? grp_id * static_cast<int>(P.batch) : 0;
+  (void)xi0; (void)xn0; (void)yi0;
   const int64_t bias0 = static_cast<int64_t>(grp_id) * P.a * P.b * P.d;
 
   if (warp == 0) {
@@ -522,9 +523,9 @@ __global__ void __launch_bounds__(kThreads, Cfg<IN_LAST, OUT_LAST, ES, OS, NT, K
             } else if (P.rg_d != 0) {
               // output seen as (k2, l2, i2, n): the tile starts at feature m0 = i*b + j0 + 64*cbi
               const int m0 = i * P.b + j0 + cbi * C::CB, seg = P.rg_c * P.rg_d;
-              tma_store_4d(&tmY, stg, (m0 % seg) / P.rg_d, 0, m0 / seg, n0 + q * 32);
+              tma_store_5d(&tmY, stg, (m0 % seg) / P.rg_d, 0, m0 / seg, n0 + q * 32, grp_id);
             } else {
-              tma_store_3d(&tmY, stg, j0 + cbi * C::CB, i, n0 + q * 32 + yn0);
+              tma_store_4d(&tmY, stg, j0 + cbi * C::CB, i, n0 + q * 32, grp_id);
             }
             bulk_commit();
           }
@@ -724,15 +725,15 @@ static int launch_one(const Problem& p, cudaStream_t stream) {
   } else if (p.out_regroup_d > 0 && OS == 2) {
     // regrouped output (k2, l2, i2, n): a staging tile of 64 features is d2 runs of 64 / d2
     const uint64_t c2 = p.out_regroup_c, d2 = p.out_regroup_d;
-    const uint64_t yd[4] = {c2, d2, a * b / (c2 * d2), B};
-    const uint64_t ys[4] = {1, c2, c2 * d2, a * b};
-    const uint32_t yb[4] = {static_cast<uint32_t>(C::CB / d2), static_cast<uint32_t>(d2), 1, 32};
-    if ((st = encode_map(&tmY, p.out_dtype, 4, p.out, yd, ys, yb, false)) != KSMM_OK) return st;
+    const uint64_t yd[5] = {c2, d2, a * b / (c2 * d2), B, G};
+    const uint64_t ys[5] = {1, c2, c2 * d2, a * b, a * b * B};
+    const uint32_t yb[5] = {static_cast<uint32_t>(C::CB / d2), static_cast<uint32_t>(d2), 1, 32, 1};
+    if ((st = encode_map(&tmY, p.out_dtype, 5, p.out, yd, ys, yb, false)) != KSMM_OK) return st;
   } else {
-    const uint64_t yd[3] = {b, a, G * B};
-    const uint64_t ys[3] = {1, b, a * b};
-    const uint32_t yb[3] = {static_cast<uint32_t>(C::CB), 1, 32};
-    if ((st = encode_map(&tmY, p.out_dtype, 3, p.out, yd, ys, yb)) != KSMM_OK) return st;
+    const uint64_t yd[4] = {b, a, B, G};
+    const uint64_t ys[4] = {1, b, a * b, a * b * B};
+    const uint32_t yb[4] = {static_cast<uint32_t>(C::CB), 1, 32, 1};
+    if ((st = encode_map(&tmY, p.out_dtype, 4, p.out, yd, ys, yb)) != KSMM_OK) return st;
   }
   P.tiles_n = static_cast<int>((B + C::XN - 1) / C::XN);
   P.tiles_j = static_cast<int>((b + C::WJ - 1) / C::WJ);
@@ -812,16 +813,18 @@ static int launch_cfg(const Problem& p, int config, cudaStream_t stream) {
 }
 
 // Layout-changing factors (d = 1, 16-bit): the tile shapes of the output's layout, configurations
-// 0, 1 and 4 of it (the other two differ only in ring depth).
+// 0, 1, 4 and 5 of it (the others differ only in ring depth).  Configuration 5, two CTAs per SM for blocks
+// of up to 64 x 64, has 64 columns where those are the weights'.
 template <bool IN_LAST>
 static int launch_mixed(const Problem& p, int config, cudaStream_t stream) {
   constexpr bool OUT_LAST = !IN_LAST;
   if (config == 2 || config == 6 || config == 7) config = 0;
-  if (config == 3 || config == 5) config = 1;
+  if (config == 3) config = 1;
   switch (config) {
     case 0: return launch_flavour<IN_LAST, OUT_LAST, 2, 2, 256, 128, 3, OUT_LAST ? 4 : 6, 4>(p, stream);
     case 1: return launch_flavour<IN_LAST, OUT_LAST, 2, 2, 128, 128, 6, 6, 6>(p, stream);
     case 4: return launch_flavour<IN_LAST, OUT_LAST, 2, 2, 64, 128, 6, 8, 8>(p, stream);
+    case 5: return launch_flavour<IN_LAST, OUT_LAST, 2, 2, OUT_LAST ? 128 : 64, 128, 1, OUT_LAST ? 3 : 4, OUT_LAST ? 2 : 3>(p, stream);
   }
   return set_error(KSMM_ERR_BAD_ARGUMENT, "tensor-core family: no configuration %d", config);
 }
@@ -833,11 +836,11 @@ int tc_num_configs() { return tc::kNumConfigs; }
 bool tc_config_supported(const Problem& p, int config, bool check_pointers) {
   if (config < 0 || config >= tc::kNumConfigs) return false;
   if (p.groups > 1) {
-    // grouped launches exist in the 16-bit / 8-bit kernel of this file only; batch-first outputs of
-    // the groups follow one another row-wise, so a partly filled last store box would spill into
-    // the next group: the batch has to be a whole number of 32-row boxes
-    if (p.in_dtype == KSMM_F32 || (!p.bs_last && (p.d != 1 || p.batch % 32 != 0))) return false;
-    if (p.out_regroup_d || p.in_regrouped) return false;
+    // grouped launches exist in the 16-bit / 8-bit kernel of this file, and in the kernel for block-ordered
+    // inputs (stacked ones)
+    if (p.in_dtype == KSMM_F32) return false;
+    if (p.in_regrouped ? (p.bs_last || p.d == 1 || config != 1 || p.group_shared_input) : (!p.bs_last && p.d != 1))
+      return false;
     if (static_cast<int64_t>(p.groups) * p.batch > 0x7fffffffLL ||
         static_cast<int64_t>(p.groups) * p.a * p.d > 0x7fffffffLL)
       return false;

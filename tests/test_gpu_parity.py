@@ -1487,3 +1487,36 @@ def test_extension_calls_match_ctypes(bs_last, monkeypatch):
     with pytest.raises(ValueError):
         layer(make(8, 192, torch.float16).cpu())
     kb.check_device()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("patterns", [[(4, 48, 48, 1), (1, 72, 48, 4)], [(2, 64, 40, 1), (1, 136, 64, 2)], [(2, 192, 64, 1)]])
+def test_grouped_batch_first_groups_end_inside_a_tile(patterns, dtype):
+    """Three groups whose batch is no multiple of the 32-row store boxes, through the block-ordered
+    intermediate where there is one: each group as its own layer computes it."""
+    gen = torch.Generator(device=DEV).manual_seed(1)
+    group = kb.KSLinearGroup([kb.KSLinear(patterns, dtype=dtype, device=DEV) for _ in range(3)])
+    for batch in (1, 31, 130, 1000):
+        x = torch.randn(batch, group.layers[0].in_size, device=DEV, generator=gen).to(dtype)
+        for y, layer in zip(group(x), group.layers):
+            ws = [kb.from_kernel_format_to_abcd(f.data, p).float().cpu().numpy() for f, p in zip(layer.factors, patterns)]
+            ref = ko.chain_apply(x.float().cpu().numpy(), ws, False) + layer.bias.float().cpu().numpy()
+            assert ko.rel_fro_error(y.float().cpu().numpy(), ref) < TOL[dtype], batch
+    kb.check_device()
+
+
+@pytest.mark.parametrize("patterns", [[(1, 64, 64, 16), (16, 64, 64, 1)], [(16, 56, 64, 1), (1, 64, 56, 16)]])
+@pytest.mark.parametrize("bs_last", [False, True])
+def test_layout_changing_small_blocks(patterns, bs_last):
+    """Blocks of up to 64 x 64 that change the layout, from the batch at which two CTAs share an SM."""
+    for batch in (4095, 4096, 4232, 8200):
+        layer = kb.KSLinear(patterns, dtype=torch.float16, bs_last=bs_last, out_bs_last=not bs_last, device=DEV)
+        x = torch.randn((layer.in_size, batch) if bs_last else (batch, layer.in_size), device=DEV, dtype=torch.float16)
+        h = (x if bs_last else x.t()).float()
+        for f, p in zip(layer.factors, patterns):
+            h = (kb.from_kernel_format_to_dense(f.data.float(), p) @ h).half().float()
+        ref = h + layer.bias.detach().float().reshape(-1, 1)
+        y = layer(x).float()
+        y = y.t() if bs_last else y
+        assert (torch.linalg.norm(y - ref) / torch.linalg.norm(ref)).item() < 2e-3, batch
+    kb.check_device()
