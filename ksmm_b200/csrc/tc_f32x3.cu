@@ -83,7 +83,6 @@ namespace tc {
 struct ParamsF {
   int a, b, c, d;
   int64_t batch;
-  int64_t out_ld;       // row stride of a batch-last output
   int tiles_n, tiles_j;
   uint32_t rows;        // blocks * tiles_n: (block, batch tile) pairs
   uint32_t row_groups;  // CTAs per j tile
@@ -502,8 +501,8 @@ __global__ void __launch_bounds__(kThreadsF, 1)
       const bool warp_active = n0 + q * 32 < P.batch;
       // direct stores: row (i*b + j0)*d + l of the output, this lane's batch entry
       const int64_t n_row = static_cast<int64_t>(n0) + q * 32 + lane;
-      const int64_t jstride = static_cast<int64_t>(P.d) * P.out_ld;
-      float* row_out = P.out + ((static_cast<int64_t>(blk / P.d) * P.b + j0) * P.d + blk % P.d) * P.out_ld + n_row;
+      const int64_t jstride = static_cast<int64_t>(P.d) * P.batch;
+      float* row_out = P.out + ((static_cast<int64_t>(blk / P.d) * P.b + j0) * P.d + blk % P.d) * P.batch + n_row;
       (void)n_row; (void)jstride; (void)row_out;
       int jlim = P.b - j0;
       if (jlim > C::NJ) jlim = C::NJ;
@@ -640,11 +639,8 @@ static int launch_f(const Problem& p, cudaStream_t stream) {
   if (IN_LAST) {
     // input (a*c*d, batch), row (i*c + k)*d + l, seen as (n % 32, k, n / 32, l, i): one box is the
     // four atoms (32 batch entries x 32 k rows) of an MN-major operand tile
-    // (rows are whole atoms: where the batch ends inside one, its tail feeds accumulator rows that are
-    // never stored)
-    const uint64_t L = in_stride(p);
-    const uint64_t dims[5] = {32, c, (B + 31) / 32, d, a};
-    const uint64_t str[5] = {1, d * L, 32, L, c * d * L};
+    const uint64_t dims[5] = {32, c, B / 32, d, a};
+    const uint64_t str[5] = {1, d * B, 32, B, c * d * B};
     const uint32_t box[5] = {32, kKC, 4, 1, 1};
     if ((st = encode_map(&tmX, KSMM_F32, 5, p.in, dims, str, box, true, true)) != KSMM_OK) return st;
   } else {
@@ -666,8 +662,7 @@ static int launch_f(const Problem& p, cudaStream_t stream) {
   } else if (BS_LAST) {
     // output (a*b*d, batch): row (i*b + j)*d + l; store = 32 j x 32 batch entries
     const uint64_t dims[4] = {B, d, b, a};
-    const uint64_t L = out_stride(p);
-    const uint64_t str[4] = {1, L, d * L, b * d * L};
+    const uint64_t str[4] = {1, B, d * B, b * d * B};
     const uint32_t box[4] = {32, 1, 32, 1};
     if ((st = encode_map(&tmY, KSMM_F32, 4, p.out, dims, str, box, false)) != KSMM_OK) return st;
   } else {
@@ -680,7 +675,6 @@ static int launch_f(const Problem& p, cudaStream_t stream) {
   ParamsF P;
   P.a = p.a; P.b = p.b; P.c = p.c; P.d = p.d;
   P.batch = p.batch;
-  P.out_ld = out_stride(p);
   P.tiles_n = static_cast<int>((B + 127) / 128);
   P.tiles_j = static_cast<int>((b + C::NJ - 1) / C::NJ);
   P.nchunks = (p.c + kKC - 1) / kKC;
@@ -718,16 +712,19 @@ static int launch_f(const Problem& p, cudaStream_t stream) {
 
 bool tc_f32x3_supported(const Problem& p, bool check_pointers) {
   if (p.in_dtype != KSMM_F32 || p.out_dtype != KSMM_F32) return false;
+  // Rows are addressed with the batch as their stride.  (Batches of partial atoms stay on the FFMA kernels
+  // also where a copy could pad their rows: those sum in full fp32, and this kernel's error is two to six
+  // times theirs.  Rounding the hi parts instead of cutting them off does not close that: the accumulator
+  // truncates once per 8 k, 4.9e-7 against 2.5e-7 at c = 192, 2.7e-7 against 1.8e-7 at c = 96.)
+  if (has_padded_rows(p)) return false;
   if (p.batch <= 0 || p.batch > 0x7fffffffLL) return false;
   // the operand tiles are addressed in atoms of 32 columns; global strides are multiples of 16 bytes
   if (p.b % 32 != 0) return false;
-  const bool out_last = out_is_last(p);
+  const bool out_last = p.out_bs_last < 0 ? p.bs_last != 0 : p.out_bs_last != 0;
   if (out_last != (p.bs_last != 0) && (p.d != 1 || p.groups > 1)) return false;  // layout-changing factors
-  // (Batches of partial atoms stay on the FFMA kernels also where rows are padded: those sum in full fp32,
-  // this kernel's error is two to six times theirs, 5e-7 to 2e-6.)
-  if ((p.bs_last || out_last) && p.batch % 32 != 0) return false;
-  if (p.bs_last && in_stride(p) % 32 != 0) return false;
-  if (out_last && out_stride(p) % 32 != 0) return false;
+  if (p.bs_last || out_last) {
+    if (p.batch % 32 != 0) return false;
+  }
   if (!p.bs_last) {
     if (p.d != 1 || p.c % 4 != 0) return false;
   }
