@@ -473,7 +473,9 @@ __global__ void __launch_bounds__(kThreads, Cfg<IN_LAST, OUT_LAST, ES, OS, NT, K
             // Rows that start anywhere: the warp writes the staging tile one output row at a time, 32
             // words per store instruction.  A 16-bit row that starts on an odd element takes its
             // words from two neighbouring lanes and its two ends as single elements.  Sixteen rows are
-            // read ahead of their stores.
+            // read ahead of their stores; the stores are what it costs, about 11 cycles each per SM:
+            // (1,768,192,2) fp16 13 us at 6504 columns, 22 at 6502, 30 at 6501.  (Runs of 128 entries whose
+            // pieces meet on 128-byte lines, three shorter stores a row, measured 34 and 48 us.)
             __syncwarp();
             const int cols = col_limit - cbi * C::CB;                      // columns of this tile that exist
             const int rows_here = min(32, row_limit - q * 32);
@@ -504,6 +506,13 @@ __global__ void __launch_bounds__(kThreads, Cfg<IN_LAST, OUT_LAST, ES, OS, NT, K
                     else if (2 * lane < cols) y16[2 * lane] = static_cast<uint16_t>(w[rr]);
                   } else {
                     // word of elements 2 lane - 1 and 2 lane
+                    if (cols >= 64) {
+                      // a whole box: the words in one store, both ends in another
+                      const uint16_t end = static_cast<uint16_t>(lane == 0 ? w[rr] : w[rr] >> 16);
+                      if (lane != 0) *reinterpret_cast<uint32_t*>(y16 + 2 * lane - 1) = (prev[rr] >> 16) | (w[rr] << 16);
+                      if (lane == 0 || lane == 31) y16[lane == 0 ? 0 : 63] = end;
+                      continue;
+                    }
                     if (lane == 0) y16[0] = static_cast<uint16_t>(w[rr]);
                     else if (2 * lane < cols) *reinterpret_cast<uint32_t*>(y16 + 2 * lane - 1) = (prev[rr] >> 16) | (w[rr] << 16);
                     else if (2 * lane - 1 < cols) y16[2 * lane - 1] = static_cast<uint16_t>(prev[rr] >> 16);
