@@ -116,7 +116,8 @@ def forward_ex(input, factor, bs_last, a, b, c, d, *, out_dtype=None, alpha=1.0,
 def default_choice(pattern, batch, dtype, bs_last, out_dtype=None):
     """What the automatic dispatch runs for one factor: ``(family, config, via_transpose)`` with
     family ``"ffma"`` or ``"tensor"``; ``via_transpose`` is true when the call goes through the
-    layout-conversion path (transpose, batch-last kernel, transpose)."""
+    layout-conversion path (transpose, batch-last kernel, transpose) or through a copy of a batch-last
+    input into padded rows."""
     lib = _lib.load()
     a, b, c, d = (int(v) for v in pattern)
     out_dtype = dtype if out_dtype is None else out_dtype
