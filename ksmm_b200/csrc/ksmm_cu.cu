@@ -323,6 +323,7 @@ static size_t pad_rows_scratch_bytes(const Problem& p) {
   return align_up(static_cast<size_t>(p.a) * p.c * p.d * padded_ld(p.batch, es) * es, 256);
 }
 
+static size_t scratch_need(const Problem& p, const Choice& ch);
 static int run_family(const Problem& p, int algo, int config, cudaStream_t stream);
 static int dispatch(const Problem& p, int algo, int config, cudaStream_t stream);
 
@@ -416,10 +417,13 @@ static int dispatch(const Problem& p, int algo, int config, cudaStream_t stream)
   if (st != KSMM_OK) return st;
   if (p.batch == 0) return KSMM_OK;  // empty batch: nothing to write
   if (algo == KSMM_ALGO_AUTO) {
-    Choice ch = auto_choice(p);
-    // the padded copy lives in scratch that the caller passed, or not at all
-    if (ch.algo == kAlgoPadRows && (p.scratch == nullptr || reinterpret_cast<uintptr_t>(p.scratch) % 16 ||
-                                    p.scratch_bytes < pad_rows_scratch_bytes(p)))
+    Choice ch = auto_choice(p), pin;
+    // Padded copies live in scratch that the caller passed, or not at all (no allocation and no refusal
+    // inside a stream capture for calls that never needed scratch); a tuned conversion takes what it takes.
+    const Problem twin = batch_last_twin(p);
+    const bool padded = ch.algo == kAlgoPadRows ||
+                        (ch.algo == KSMM_ALGO_CONVERT && has_padded_rows(twin) && !lookup_choice(p, &pin));
+    if (padded && (p.scratch == nullptr || reinterpret_cast<uintptr_t>(p.scratch) % 16 || p.scratch_bytes < scratch_need(p, ch)))
       ch = Choice{KSMM_ALGO_SIMT, -1};
     return run_family(p, ch.algo, ch.config, stream);
   }

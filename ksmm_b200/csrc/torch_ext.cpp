@@ -55,10 +55,24 @@ torch::Tensor forward(torch::Tensor input, torch::Tensor factor, int64_t bs_last
   const int64_t batch = input.size(bs_last ? 1 : 0);
   auto out = bs_last ? torch::empty({a * b * d, batch}, input.options())
                      : torch::empty({batch, a * b * d}, input.options());
-  check_status(ksmm_cu_forward(input.data_ptr(), factor.data_ptr(), out.data_ptr(), batch,
-                               static_cast<int>(a), static_cast<int>(b), static_cast<int>(c),
-                               static_cast<int>(d), dtype_code(input), bs_last ? 1 : 0,
-                               at::cuda::getCurrentCUDAStream().stream()));
+  ksmm_forward_desc_t f = {};
+  f.input = input.data_ptr();
+  f.values = factor.data_ptr();
+  f.output = out.data_ptr();
+  f.batch = batch;
+  f.a = static_cast<int>(a); f.b = static_cast<int>(b); f.c = static_cast<int>(c); f.d = static_cast<int>(d);
+  f.in_dtype = f.out_dtype = dtype_code(input);
+  f.bs_last = bs_last ? 1 : 0;
+  f.algo = KSMM_ALGO_AUTO;
+  f.config = -1;
+  f.alpha = 1.f;
+  torch::Tensor scratch;
+  if (const size_t need = ksmm_cu_layout_scratch_bytes(&f)) {
+    scratch = torch::empty({static_cast<int64_t>(need)}, input.options().dtype(at::kByte));
+    f.scratch = scratch.data_ptr();
+    f.scratch_bytes = need;
+  }
+  check_status(ksmm_cu_forward_ex(&f, at::cuda::getCurrentCUDAStream().stream()));
   return out;
 }
 

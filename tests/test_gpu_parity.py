@@ -1520,3 +1520,50 @@ def test_layout_changing_small_blocks(patterns, bs_last):
         y = y.t() if bs_last else y
         assert (torch.linalg.norm(y - ref) / torch.linalg.norm(ref)).item() < 2e-3, batch
     kb.check_device()
+
+
+@pytest.mark.parametrize("pattern,bs_last", [((1, 64, 64, 16), False), ((1, 96, 64, 12), False), ((1, 96, 64, 2), True)])
+def test_ragged_calls_without_scratch(pattern, bs_last):
+    """The plain C call takes no scratch: at a ragged batch it allocates nothing, can be captured, and
+    computes what the call with scratch does (the sums differ in order: one rounding step)."""
+    a, b, c, d = pattern
+    batch = 203
+    lib = _lib.load()
+    x, w = _inputs(pattern, batch, torch.float16, bs_last, seed=4)
+    xg, wk = x.to(DEV), kb.generate_factor(*pattern, "kernel", w, w.dtype, DEV)
+    ref = kb.forward_ex(xg, wk, bs_last, a, b, c, d)
+    out = torch.zeros_like(ref)
+    stream = torch.cuda.Stream()
+    before = kb.alloc_count()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        _lib.check(lib.ksmm_cu_forward(xg.data_ptr(), wk.data_ptr(), out.data_ptr(), batch, a, b, c, d, _lib.KSMM_F16,
+                                       int(bs_last), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert kb.alloc_count() == before
+    err = torch.linalg.norm(out.double() - ref.double()) / torch.linalg.norm(ref.double())
+    assert err.item() < 2.0 ** -11
+    kb.check_device()
+
+
+@pytest.mark.parametrize("bs_last", [False, True])
+def test_ragged_chain_takes_the_older_workspace(bs_last):
+    """A workspace of the size without padded rows still serves; the result is that of the larger one."""
+    pats = [(4, 48, 48, 1), (1, 192, 48, 4)]
+    batch = 333
+    lib = _lib.load()
+    layer = kb.KSLinear(pats, dtype=torch.float16, bs_last=bs_last, bias=False, device=DEV)
+    x = torch.randn((192, batch) if bs_last else (batch, 192), device=DEV, dtype=torch.float16)
+    ref = layer(x)
+    out = torch.zeros_like(ref)
+    ws = torch.empty((192 * batch * 2 + 255) // 256 * 256, dtype=torch.uint8, device=DEV)
+    vals = (ctypes.c_void_p * 2)(*[f.data_ptr() for f in layer.factors])
+    _lib.check(lib.ksmm_cu_chain_forward(x.data_ptr(), vals, out.data_ptr(), None, ws.data_ptr(), ws.numel(), batch, 2,
+                                         _lib.int32_array([v for p in pats for v in p]), _lib.KSMM_F16, int(bs_last),
+                                         ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    torch.cuda.synchronize()
+    err = torch.linalg.norm(out.double() - ref.double()) / torch.linalg.norm(ref.double())
+    assert err.item() < 2.0 ** -10   # two factors, one rounding step each
+    kb.check_device()
