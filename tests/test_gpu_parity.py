@@ -1567,3 +1567,27 @@ def test_ragged_chain_takes_the_older_workspace(bs_last):
     err = torch.linalg.norm(out.double() - ref.double()) / torch.linalg.norm(ref.double())
     assert err.item() < 2.0 ** -10   # two factors, one rounding step each
     kb.check_device()
+
+
+def test_chain_gradients_without_bias(monkeypatch):
+    """No bias among the node's inputs: the factors' gradients are those of the layer with a bias."""
+    from ksmm_b200 import kernel as kk
+    pats = [(4, 48, 48, 1), (1, 192, 48, 4)]
+    layer = kb.KSLinear(pats, dtype=torch.float16, device=DEV, requires_grad=True)
+    plain = kb.KSLinear(pats, dtype=torch.float16, device=DEV, requires_grad=True, bias=False,
+                        weights=[kb.from_kernel_format_to_abcd(f.detach(), p) for f, p in zip(layer.factors, pats)])
+    x = torch.randn(140, 192, device=DEV, dtype=torch.float16)
+    g = torch.randn(140, 768, device=DEV, dtype=torch.float16)
+    layer(x).backward(g)
+    for native in (kk._native, None):
+        monkeypatch.setattr(kk, "_native", native)
+        for frozen in (None, 0, 1):
+            plain.zero_grad(set_to_none=True)
+            for q, f in enumerate(plain.factors):
+                f.requires_grad_(q != frozen)
+            xg = x.clone().requires_grad_(True)
+            plain(xg).backward(g)
+            assert xg.grad.shape == x.shape
+            for q, (a, b) in enumerate(zip(plain.factors, layer.factors)):
+                assert (a.grad is None) if q == frozen else torch.equal(a.grad, b.grad)
+    kb.check_device()
