@@ -274,7 +274,11 @@ KSMM_API int ksmm_cu_grouped_chain_forward(const void* input, const void* const*
  * batch-first, 1 batch-last, 2 batch-first in the block order of the next
  * factor).  The backward computes whichever of grad_input, grad_values[f]
  * (kernel format) and grad_bias is not NULL; its input and grad_output are
- * aligned to 16 bytes.  fp32, fp16 and bf16; results have the input's type.
+ * aligned to 16 bytes, its results may start at any element (a grad_input that
+ * is not aligned to 16 bytes runs on a slower kernel where the aligned one's
+ * workspace has no room for a faster one).  The forward refuses an unaligned
+ * input or output (KSMM_ERR_WORKSPACE) where it would need more scratch than
+ * for aligned ones.  fp32, fp16 and bf16; results have the input's type.
  */
 KSMM_API int ksmm_cu_chain_train_bytes(int nfactors, const int32_t* patterns, int64_t batch, int dtype,
                               int bs_last, size_t* saved_bytes, size_t* forward_bytes,

@@ -1423,12 +1423,14 @@ static void plan_backward(int nfactors, const int32_t* patterns, int64_t batch, 
   }
 }
 
-// Plans (run == false: the workspace's bytes through *need) or runs the backward of a chain.
+// Plans (run == false: the workspace's bytes through *need) or runs the backward of a chain.  The plan knows
+// neither the alignment of grad_input nor what is tuned by the time of the run, so the run takes no more
+// than `ws_bytes`: a factor whose scratch is not there runs on the register-staged kernel, which needs none.
 static int chain_backward_walk(bool run, const void* input, const void* const* values, const void* saved,
                                const int32_t* layouts, const void* grad_output, void* grad_input,
-                               void* const* grad_values, void* grad_bias, char* ws, int64_t batch, int nfactors,
-                               const int32_t* patterns, int dtype, int bs_last, bool need_input, bool allow_switch,
-                               bool one_layout, cudaStream_t stream, size_t* need) {
+                               void* const* grad_values, void* grad_bias, char* ws, size_t ws_bytes, int64_t batch,
+                               int nfactors, const int32_t* patterns, int dtype, int bs_last, bool need_input,
+                               bool allow_switch, bool one_layout, cudaStream_t stream, size_t* need) {
   const int es = dtype_size(dtype);
   const int64_t ld = one_layout ? batch : padded_ld(batch, es);
   BackwardPlan plan;
@@ -1448,6 +1450,7 @@ static int chain_backward_walk(bool run, const void* input, const void* const* v
   char* gbuf = second + second_bytes;       // gradients of the intermediates, two alternating buffers
   char* g0 = gbuf + 2 * one;                // the input's gradient before its transpose
   char* tail = g0 + post_bytes;             // what one launch sequence needs for itself
+  const size_t tail_room = ws_bytes - static_cast<size_t>(tail - ws);
   size_t tail_bytes = 0;
 
   // versions of the output's gradient
@@ -1490,7 +1493,7 @@ static int chain_backward_walk(bool run, const void* input, const void* const* v
       WgradOperand gw = f == nfactors - 1 && dy.last && !pad_copy ? dy : g;
       const size_t wneed = wgrad_workspace_bytes(p, x, gw);
       tail_bytes = std::max(tail_bytes, wneed);
-      if (run) st = wgrad_launch(p, x, gw, tail, wneed, stream);
+      if (run) st = wgrad_launch(p, x, gw, tail, tail_room, stream);
       if (st != KSMM_OK) return st;
     }
     if (f == 0 && !need_input) break;
@@ -1505,16 +1508,21 @@ static int chain_backward_walk(bool run, const void* input, const void* const* v
     p.no_alloc = 1;
     const bool turns = plan.in_last[f] != plan.out_last[f];
     if (turns) p.out_bs_last = plan.out_last[f];
-    const size_t sneed = turns ? 0 : scratch_need(p, auto_choice(p));
+    Choice ch = turns ? Choice{KSMM_ALGO_TC, -1} : auto_choice(p);
+    size_t sneed = turns ? 0 : scratch_need(p, ch);
     tail_bytes = std::max(tail_bytes, wt + sneed);
     if (run) {
+      if (sneed > tail_room - wt) {
+        ch = Choice{KSMM_ALGO_SIMT, -1};
+        sneed = 0;
+      }
       st = launch_transpose_blocks(values[f], tail, static_cast<int64_t>(q[0]) * q[3], q[2], q[1], es, stream);
       if (st != KSMM_OK) return st;
       if (sneed) {
         p.scratch = tail + wt;
         p.scratch_bytes = sneed;
       }
-      st = turns ? run_family(p, KSMM_ALGO_TC, -1, stream) : dispatch(p, KSMM_ALGO_AUTO, -1, stream);
+      st = run_family(p, ch.algo, ch.config, stream);
       if (st != KSMM_OK) return st;
     }
     g = WgradOperand{dst, plan.out_last[f], own_ld};
@@ -1559,8 +1567,8 @@ int ksmm_cu_chain_train_bytes(int nfactors, const int32_t* patterns, int64_t bat
     for (int kind = 0; kind < 2; ++kind) {
       for (int f = 0; f + 1 < nfactors && kind == 1; ++f) layouts[f] = one_layout ? bs_last : 0;
       for (int need_input = 0; need_input < 2; ++need_input) {
-        st = chain_backward_walk(false, nullptr, nullptr, nullptr, layouts, nullptr, nullptr, nullptr, nullptr, nullptr, batch,
-                                 nfactors, patterns, dtype, bs_last, need_input != 0, allow != 0, one_layout, nullptr, &need);
+        st = chain_backward_walk(false, nullptr, nullptr, nullptr, layouts, nullptr, nullptr, nullptr, nullptr, nullptr, SIZE_MAX,
+                                 batch, nfactors, patterns, dtype, bs_last, need_input != 0, allow != 0, one_layout, nullptr, &need);
         if (st != KSMM_OK) return st;
         *backward_bytes = std::max(*backward_bytes, need);
       }
@@ -1618,8 +1626,8 @@ int ksmm_cu_chain_backward(const void* input, const void* const* values, const v
   size_t need = 0;
   for (int run = 0; run < 2; ++run) {
     st = chain_backward_walk(run != 0, input, values, saved, layouts, grad_output, grad_input, grad_values, grad_bias,
-                             static_cast<char*>(workspace), batch, nfactors, patterns, dtype, bs_last, grad_input != nullptr,
-                             allow, one_layout, s, run ? nullptr : &need);
+                             static_cast<char*>(workspace), run ? workspace_bytes : SIZE_MAX, batch, nfactors, patterns, dtype,
+                             bs_last, grad_input != nullptr, allow, one_layout, s, run ? nullptr : &need);
     if (st != KSMM_OK) return st;
     if (!run && need && (!workspace || reinterpret_cast<uintptr_t>(workspace) % 256 || workspace_bytes < need))
       return set_error(KSMM_ERR_WORKSPACE, "chain backward: need %zu bytes aligned to 256, got %zu", need, workspace_bytes);

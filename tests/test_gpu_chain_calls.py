@@ -1,0 +1,59 @@
+"""The C calls behind trainable and fp8 layers, where the Python layers never take them: pointers that torch
+does not hand out, workspaces with a guard behind them, unusual values."""
+import ctypes
+
+import pytest
+import torch
+
+import ksmm_b200 as kb
+from ksmm_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _stream():
+    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+def _train_bytes(pattern_list, batch, code, bs_last):
+    sizes = [ctypes.c_size_t() for _ in range(3)]
+    pat = _lib.int32_array([v for p in pattern_list for v in p])
+    _lib.check(_lib.load().ksmm_cu_chain_train_bytes(len(pattern_list), pat, batch, code, bs_last, *map(ctypes.byref, sizes)))
+    return pat, [s.value for s in sizes]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("pattern,batch", [((1, 64, 64, 4), 64), ((4, 64, 64, 4), 64), ((1, 96, 96, 2), 64), ((1, 64, 64, 2), 96),
+                                           ((1, 64, 64, 16), 70), ((1, 64, 64, 1), 64)])
+@pytest.mark.parametrize("bs_last", [0, 1])
+def test_unaligned_input_gradient_stays_inside_the_workspace(pattern, batch, bs_last, dtype):
+    """grad_input may start anywhere.  Its kernel is then another one, and where that one would want scratch
+    that the workspace does not hold, it runs without.  Tolerance: one rounding step of the type."""
+    a, b, c, d = pattern
+    code = _lib.KSMM_F32 if dtype == torch.float32 else _lib.KSMM_F16
+    pat, (_, _, need) = _train_bytes([pattern], batch, code, bs_last)
+    gen = torch.Generator(device=DEV).manual_seed(batch)
+
+    def make(feats):
+        return torch.randn((feats, batch) if bs_last else (batch, feats), device=DEV, generator=gen).to(dtype)
+
+    x, g = make(a * c * d), make(a * b * d)
+    w = torch.randn(a * d * c, b, device=DEV, generator=gen).to(dtype)
+    dense = kb.from_kernel_format_to_dense(w.double(), pattern)
+    ref = dense.t() @ (g if bs_last else g.t()).double()
+    for shift in (0, 1):
+        guard = torch.full((need + (1 << 20),), 0xA5, dtype=torch.uint8, device=DEV)
+        gx = torch.full((x.numel() + 64,), 7.0, dtype=dtype, device=DEV)
+        gw, gb = torch.empty_like(w), torch.empty(a * b * d, dtype=dtype, device=DEV)
+        _lib.check(_lib.load().ksmm_cu_chain_backward(
+            x.data_ptr(), (ctypes.c_void_p * 1)(w.data_ptr()), None, None, g.data_ptr(), gx[shift:].data_ptr(),
+            (ctypes.c_void_p * 1)(gw.data_ptr()), gb.data_ptr(), guard.data_ptr(), need, batch, 1, pat, code, bs_last, _stream()))
+        torch.cuda.synchronize()
+        assert bool((guard[need:] == 0xA5).all())
+        got = gx[shift:shift + x.numel()].view(x.shape)
+        got = (got if bs_last else got.t()).double()
+        err = (torch.linalg.norm(got - ref) / torch.linalg.norm(ref)).item()
+        assert err < (1e-5 if dtype == torch.float32 else 2.0 ** -11), (shift, err)
+        assert bool((gx[:shift] == 7.0).all()) and bool((gx[shift + x.numel():] == 7.0).all())
+    kb.check_device()
