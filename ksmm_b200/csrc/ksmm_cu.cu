@@ -941,6 +941,12 @@ static int check_chain(int nfactors, const int32_t* patterns, const void* const*
   return KSMM_OK;
 }
 
+static int check_values(int nfactors, const void* const* values) {
+  for (int f = 0; f < nfactors; ++f)
+    if (!values[f]) return set_error(KSMM_ERR_BAD_ARGUMENT, "null pointer (values of factor %d)", f);
+  return KSMM_OK;
+}
+
 size_t ksmm_cu_chain_workspace_bytes_ex(int nfactors, const int32_t* patterns, int64_t batch,
                                         int dtype, int bs_last) {
   return ksmm_cu_chain_workspace_bytes_layouts(nfactors, patterns, batch, dtype, bs_last, bs_last);
@@ -1140,6 +1146,7 @@ int ksmm_cu_chain_forward_fp8(const void* input, int in_dtype, const void* const
   if (st != KSMM_OK) return st;
   if (batch == 0) return KSMM_OK;
   if (!input || !output || !weight_scales) return set_error(KSMM_ERR_BAD_ARGUMENT, "null pointer");
+  if ((st = check_values(nfactors, values)) != KSMM_OK) return st;
   Fp8Buffers buf;
   st = chain_fp8_walk(false, nullptr, in_dtype, nullptr, nullptr, nullptr, nullptr, nullptr, &buf, batch, nfactors,
                       patterns, bs_last, nullptr);
@@ -1590,6 +1597,7 @@ int ksmm_cu_chain_train_forward(const void* input, const void* const* values, vo
                      want[1]);
   if (!layouts && nfactors > 1) return set_error(KSMM_ERR_BAD_ARGUMENT, "null layouts");
   if (!input || !output) return set_error(KSMM_ERR_BAD_ARGUMENT, "null pointer");
+  if ((st = check_values(nfactors, values)) != KSMM_OK) return st;
   const bool one_layout = train_one_layout(nfactors, patterns, batch, dtype, bs_last);
   int allow = !one_layout && aligned16(input) && aligned16(output) ? 1 : 0;
   for (int f = 0; f < nfactors; ++f) allow &= aligned16(values[f]) ? 1 : 0;
@@ -1618,6 +1626,7 @@ int ksmm_cu_chain_backward(const void* input, const void* const* values, const v
     return KSMM_OK;
   }
   if (!input || !grad_output || (nfactors > 1 && !saved)) return set_error(KSMM_ERR_BAD_ARGUMENT, "null pointer");
+  if ((st = check_values(nfactors, values)) != KSMM_OK) return st;
   if (!aligned16(input) || !aligned16(grad_output))
     return set_error(KSMM_ERR_BAD_ARGUMENT, "the backward of a chain takes an input and a gradient aligned to 16 bytes");
   const bool one_layout = train_one_layout(nfactors, patterns, batch, dtype, bs_last);

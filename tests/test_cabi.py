@@ -181,3 +181,55 @@ def test_conversion_family_in_the_choice_cache():
     assert lib.ksmm_cu_get_choice(78, 1, 64, 64, 4, 1, 1, 0, ctypes.byref(algo), ctypes.byref(cfg)) == 0
     assert (algo.value, cfg.value) == (_lib.KSMM_ALGO_CONVERT, 0)
     assert lib.ksmm_cu_set_choice(78, 1, 64, 64, 4, 1, 1, 1, _lib.KSMM_ALGO_CONVERT, 0) == _lib.KSMM_ERR_UNSUPPORTED
+
+
+def _aligned_buffer():
+    """Host memory that no refused call touches: (owner, an address aligned to 256 bytes)."""
+    buf = ctypes.create_string_buffer(1 << 12)
+    return buf, (ctypes.addressof(buf) + 255) // 256 * 256
+
+
+def test_training_and_fp8_calls_refuse_misuse_before_the_device():
+    """Null pointers (those of single factors too), small or unaligned workspaces, layouts and types that do
+    not exist: a status and no launch."""
+    lib = _lib.load()
+    owner, p = _aligned_buffer()
+    pats = [(2, 16, 16, 1), (1, 32, 32, 1)]
+    pat, batch, n, big = _lib.int32_array([v for q in pats for v in q]), 8, 2, 1 << 40
+    bad, small = _lib.KSMM_ERR_BAD_ARGUMENT, _lib.KSMM_ERR_WORKSPACE
+    ptrs = lambda *v: (ctypes.c_void_p * n)(*v)  # noqa: E731
+    vals, lay = ptrs(p, p), (ctypes.c_int32 * n)()
+    before = lib.ksmm_cu_launch_count()
+    sizes = [ctypes.c_size_t() for _ in range(3)]
+
+    def size(pattern=pat, dtype=_lib.KSMM_F16, last=0, batch=batch, out=sizes):
+        return lib.ksmm_cu_chain_train_bytes(n, pattern, batch, dtype, last, *[None if s is None else ctypes.byref(s) for s in out])
+
+    assert size() == _lib.KSMM_OK and all(s.value > 0 for s in sizes[:1] + sizes[2:])
+    assert size(dtype=_lib.KSMM_F8E4M3) == _lib.KSMM_ERR_UNSUPPORTED
+    assert size(dtype=9) == size(last=2) == size(batch=-1) == size(out=[None, None, None]) == bad
+    assert size(pattern=_lib.int32_array([2, 16, 16, 1, 1, 32, 16, 1])) == bad
+
+    def forward(x=p, values=vals, y=p, saved=p, room=big, scratch=p, layouts=lay):
+        return lib.ksmm_cu_chain_train_forward(x, values, y, None, saved, room, scratch, room, batch, n, pat, _lib.KSMM_F16, 0,
+                                               layouts, None)
+
+    assert forward(x=None) == forward(y=None) == forward(values=ptrs(p, None)) == forward(layouts=None) == bad
+    assert forward(saved=None) == forward(saved=p + 16) == forward(room=0) == small
+
+    def backward(x=p, values=vals, saved=p, layouts=lay, g=p, gw=ptrs(p, p), ws=p, room=big):
+        return lib.ksmm_cu_chain_backward(x, values, saved, layouts, g, p, gw, p, ws, room, batch, n, pat, _lib.KSMM_F16, 0, None)
+
+    assert backward(x=None) == backward(g=None) == backward(saved=None) == backward(layouts=None) == backward(gw=None) == bad
+    assert backward(values=ptrs(None, p)) == backward(x=p + 2) == backward(g=p + 8) == bad
+    assert backward(ws=None) == backward(ws=p + 16) == backward(room=16) == small
+
+    scales = (ctypes.c_float * n)(1.0, 1.0)
+
+    def fp8(x=p, code=_lib.KSMM_BF16, values=vals, s=scales, y=p, ws=p, room=big, last=0):
+        return lib.ksmm_cu_chain_forward_fp8(x, code, values, s, y, None, ws, room, batch, n, pat, last, None)
+
+    assert fp8(x=None) == fp8(y=None) == fp8(s=None) == fp8(values=ptrs(p, None)) == fp8(code=_lib.KSMM_F8E4M3) == fp8(last=2) == bad
+    assert fp8(ws=None) == fp8(ws=p + 16) == fp8(room=16) == small
+    assert lib.ksmm_cu_launch_count() == before
+    del owner
