@@ -125,11 +125,16 @@ class KSLinear(nn.Module):
             self.register_parameter("bias", None)
         self._workspace = None
 
-    # -- fp8: weights are quantised once, lazily (per-tensor scale amax/448) -------------
+    # -- fp8: weights are quantised lazily (per-tensor scale amax/448), once per state of the factors ----
     def _fp8_factors(self):
-        if self._fp8_cache is None:
-            self._fp8_cache = [_k.quantize_e4m3(f.data) for f in self.factors]
-        return self._fp8_cache
+        # (A version counts in-place changes, except those made through .data, which torch does not count;
+        # new storage or another device shows in the rest.  The cache holds on to the storages it was made
+        # from, so that no address of the key is used again meanwhile.)
+        state = [(None if f.is_inference() else f._version, f.data_ptr(), f.device) for f in self.factors]
+        if self._fp8_cache is None or self._fp8_cache[0] != state:
+            data = [f.data for f in self.factors]
+            self._fp8_cache = state, [_k.quantize_e4m3(f) for f in data], data
+        return self._fp8_cache[1]
 
     def _forward_2d(self, x, residual=None):
         if _lib.native is not None and not self.is_fp8 and (self.fuse_chain or self.num_mat == 1):

@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 import torch
 
+import ksmm_b200 as kb
 from golden_cases import CASES, make_inputs
 from ksmm_b200 import interface as itf
 from ksmm_b200 import kernel as kmod
@@ -142,3 +143,30 @@ def test_reference_best_table_as_priors(tmp_path):
     with pytest.raises(ValueError):
         (tmp_path / "x.best").write_text("1 2 3\n")
         tuner.read_best_rows(str(tmp_path / "x.best"))
+
+
+def test_fp8_factors_follow_their_weights():
+    """The quantised factors of an fp8 layer are made once and again whenever a factor has changed."""
+    layer = kb.KSLinear.__new__(kb.KSLinear)   # the cache alone: layers themselves live on a GPU
+    torch.nn.Module.__init__(layer)
+    layer.factors = torch.nn.ParameterList([torch.nn.Parameter(torch.randn(8, 4), requires_grad=False) for _ in range(2)])
+    layer._fp8_cache = None
+
+    def stale():
+        return any(not torch.equal(q.float(), kb.quantize_e4m3(f.data)[0].float()) or s != kb.quantize_e4m3(f.data)[1]
+                   for (q, s), f in zip(layer._fp8_factors(), layer.factors))
+
+    first = layer._fp8_factors()
+    assert layer._fp8_factors() is first and not stale()
+    with torch.no_grad():
+        layer.factors[1].mul_(-3)
+    assert not stale()
+    layer.load_state_dict({k: torch.randn_like(v) for k, v in layer.state_dict().items()})
+    assert not stale()
+    layer.factors[0].data = torch.randn(8, 4)
+    assert not stale()
+    layer.factors[0] = torch.nn.Parameter(torch.randn(8, 4), requires_grad=False)
+    assert not stale()
+    with torch.inference_mode():
+        layer.factors[0] = torch.nn.Parameter(torch.randn(8, 4), requires_grad=False)
+        assert not stale() and layer._fp8_factors() is layer._fp8_factors()
