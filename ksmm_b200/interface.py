@@ -54,6 +54,13 @@ def from_kernel_format_to_dense(factor, pattern):
     return torch.block_diag(*torch.unbind(blocks, dim=0))
 
 
+def _state(t):
+    """What a copy made from ``t`` is valid for.  The version counts in-place changes, except those made
+    through ``.data``, which torch does not count; new storage or another device shows in the rest, as long
+    as whoever keeps the copy holds on to the old storage, so that its address is not used again."""
+    return None if t.is_inference() else t._version, t.data_ptr(), t.device
+
+
 class KSLinear(nn.Module):
     r"""Kronecker-sparse linear layer: the weight is a product of factors with
     patterns ``(a,b,c,d)`` (support :math:`I_a \otimes 1_{b\times c} \otimes I_d`),
@@ -127,10 +134,7 @@ class KSLinear(nn.Module):
 
     # -- fp8: weights are quantised lazily (per-tensor scale amax/448), once per state of the factors ----
     def _fp8_factors(self):
-        # (A version counts in-place changes, except those made through .data, which torch does not count;
-        # new storage or another device shows in the rest.  The cache holds on to the storages it was made
-        # from, so that no address of the key is used again meanwhile.)
-        state = [(None if f.is_inference() else f._version, f.data_ptr(), f.device) for f in self.factors]
+        state = [_state(f) for f in self.factors]
         if self._fp8_cache is None or self._fp8_cache[0] != state:
             data = [f.data for f in self.factors]
             self._fp8_cache = state, [_k.quantize_e4m3(f) for f in data], data
@@ -282,9 +286,10 @@ class KSLinearGroup(nn.Module):
         self._versions = None
 
     def _stack(self):
-        versions = [(f._version, f.data_ptr()) for l in self.layers for f in l.factors]
+        tensors = [f for l in self.layers for f in l.factors]
         if self.layers[0].bias is not None:
-            versions += [(l.bias._version, l.bias.data_ptr()) for l in self.layers]
+            tensors += [l.bias for l in self.layers]
+        versions = [_state(t) for t in tensors]
         if self._stacked is None or versions != self._versions:
             nf = self.layers[0].num_mat
             factors = [torch.cat([l.factors[f].data for l in self.layers], dim=0).contiguous() for f in range(nf)]
@@ -292,6 +297,7 @@ class KSLinearGroup(nn.Module):
             if self.layers[0].bias is not None:
                 bias = torch.cat([l.bias.data.reshape(-1) for l in self.layers]).contiguous()
             self._stacked, self._versions = (factors, bias), versions
+            self._made_from = [t.data for t in tensors]
         return self._stacked
 
     def forward(self, tensor):

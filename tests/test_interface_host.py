@@ -170,3 +170,30 @@ def test_fp8_factors_follow_their_weights():
     with torch.inference_mode():
         layer.factors[0] = torch.nn.Parameter(torch.randn(8, 4), requires_grad=False)
         assert not stale() and layer._fp8_factors() is layer._fp8_factors()
+
+
+def test_stacked_factors_follow_their_layers():
+    """The stacked copy of a group is made again for new factors, also where their storage lands at the
+    address of the old one."""
+    group = kb.KSLinearGroup.__new__(kb.KSLinearGroup)
+    torch.nn.Module.__init__(group)
+
+    class Layer(torch.nn.Module):
+        num_mat, bias = 1, None
+
+        def __init__(self):
+            super().__init__()
+            self.factors = torch.nn.ParameterList([torch.nn.Parameter(torch.randn(8, 4), requires_grad=False)])
+
+    group.layers = torch.nn.ModuleList([Layer() for _ in range(2)])
+    group._stacked = group._versions = None
+
+    def stale():
+        return not torch.equal(group._stack()[0][0], torch.cat([l.factors[0].data for l in group.layers]))
+
+    assert not stale() and group._stack() is group._stack()
+    for _ in range(8):
+        values = torch.randn(8, 4)
+        group.layers[0].factors[0] = torch.nn.Parameter(torch.zeros(1), requires_grad=False)
+        group.layers[0].factors[0] = torch.nn.Parameter(values.clone(), requires_grad=False)
+        assert not stale()
