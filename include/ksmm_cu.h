@@ -404,7 +404,10 @@ KSMM_API int ksmm_cu_host_wait(uint64_t ticket);
  * ksmm_cu_config_supported: 1 if (algo, config) can run this problem.
  * ksmm_cu_tune: times every supported candidate on the given buffers (which
  *   must be valid for the problem; output is overwritten), stores the winner
- *   in the in-process cache, and reports it.  best_ms may be NULL.  Every
+ *   in the in-process cache, and reports it.  best_ms may be NULL.  Where
+ *   untuned calls copy a batch-last input into padded rows (see
+ *   ksmm_cu_layout_scratch_bytes) and that is the fastest, nothing is stored
+ *   and *best_algo is KSMM_ALGO_AUTO.  Every
  *   timed launch (nrepeats per candidate, at most 64) starts with a cold L2:
  *   the call allocates a buffer of 1.5x the cache for its own duration and
  *   overwrites it before each launch, outside the timed interval.  An
@@ -419,8 +422,9 @@ KSMM_API int ksmm_cu_host_wait(uint64_t ticket);
  * KSMM_ALGO_CONVERT (one configuration, 0) is that conversion path as a
  *   family of its own, so that the tuner can time it against the direct
  *   kernels and a saved table can name it.  A cached choice is used only when
- *   it can run on the pointers of the actual call; otherwise the heuristic
- *   decides, as if nothing were cached.
+ *   it can run on the pointers of the actual call, and not for the padded
+ *   rows inside a chain; otherwise the heuristic decides, as if nothing were
+ *   cached.
  */
 KSMM_API int ksmm_cu_num_configs(int algo);
 KSMM_API int ksmm_cu_config_supported(int algo, int config, int64_t batch, int a, int b, int c, int d,

@@ -131,6 +131,11 @@ int main(int argc, char** argv) {
   float tuned_ms = 0.f;
   int st = ksmm_cu_tune(&desc, 10, nullptr, &algo, &config, &tuned_ms);
   if (st != KSMM_OK) { fprintf(stderr, "tune: %s\n", ksmm_cu_last_error()); return 3; }
+  void* scratch = nullptr;
+  if ((desc.scratch_bytes = ksmm_cu_layout_scratch_bytes(&desc)) > 0) {
+    CK(cudaMalloc(&scratch, desc.scratch_bytes));
+    desc.scratch = scratch;
+  }
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
@@ -181,6 +186,6 @@ int main(int argc, char** argv) {
   fclose(f);
   printf("%s pattern (%d,%d,%d,%d) batch %lld: family %d config %d, %.4f +/- %.4f ms, rmse %.3e -> %s\n",
          kernel.c_str(), a, b, c, d, batch, algo, config, mean, stdv, rmse, target.c_str());
-  cudaFree(dx); cudaFree(dw); cudaFree(dy);
+  cudaFree(dx); cudaFree(dw); cudaFree(dy); cudaFree(scratch);
   return rmse < thr ? 0 : 5;
 }

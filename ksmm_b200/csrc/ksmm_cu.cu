@@ -171,7 +171,10 @@ static ChoiceKey key_of(const Problem& p) {
   return ChoiceKey(p.batch, p.a, p.b, p.c, p.d, p.in_dtype, p.out_dtype, p.bs_last);
 }
 
+// (A choice was made for rows of exactly the batch.  The padded ones of a chain's intermediates reach
+// kernels that could not run there.)
 static bool lookup_choice(const Problem& p, Choice* out) {
+  if (has_padded_rows(p)) return false;
   std::lock_guard<std::mutex> g(g_choice_mu);
   auto it = g_choices.find(key_of(p));
   if (it == g_choices.end()) return false;
@@ -1943,19 +1946,31 @@ int ksmm_cu_tune(const ksmm_forward_desc_t* desc, int nrepeats, void* stream, in
   g_allocs.fetch_add(1, std::memory_order_relaxed);
   std::vector<cudaEvent_t> ev(2 * static_cast<size_t>(nrepeats));
   for (auto& e : ev) cudaEventCreate(&e);
+  void* padded = nullptr;
   auto cleanup = [&]() {
     for (auto& e : ev) cudaEventDestroy(e);
     cudaFree(flush);
+    cudaFree(padded);
   };
   float best = -1.f;
   Choice win{KSMM_ALGO_SIMT, simt_default_config_for(p)};
-  // candidates: every configuration of the two kernel families that can run the problem, and
-  // the layout-conversion path (transpose, batch-last kernel, transpose) where it exists
-  const int families[3] = {KSMM_ALGO_TC, KSMM_ALGO_SIMT, KSMM_ALGO_CONVERT};
+  // candidates: every configuration of the two kernel families that can run the problem, the
+  // layout-conversion path (transpose, batch-last kernel, transpose) where it exists, and for rows that are
+  // no 16-byte multiples the copy into padded rows, in scratch as callers pass it
+  if (pad_rows_applies(p) && (!p.scratch || reinterpret_cast<uintptr_t>(p.scratch) % 16 || p.scratch_bytes < pad_rows_scratch_bytes(p))) {
+    if (cudaMalloc(&padded, pad_rows_scratch_bytes(p)) != cudaSuccess) {
+      cleanup();
+      return set_error(KSMM_ERR_CUDA, "no memory for the copy of the input");
+    }
+    g_allocs.fetch_add(1, std::memory_order_relaxed);
+    p.scratch = padded;
+    p.scratch_bytes = pad_rows_scratch_bytes(p);
+  }
+  const int families[4] = {KSMM_ALGO_TC, KSMM_ALGO_SIMT, KSMM_ALGO_CONVERT, kAlgoPadRows};
   for (int fam : families) {
-    const int ncfg = fam == KSMM_ALGO_CONVERT ? 1 : ksmm_cu_num_configs(fam);
+    const int ncfg = fam == KSMM_ALGO_CONVERT || fam == kAlgoPadRows ? 1 : ksmm_cu_num_configs(fam);
     for (int cfg = 0; cfg < ncfg; ++cfg) {
-      if (!choice_runnable(p, Choice{fam, cfg})) continue;
+      if (fam == kAlgoPadRows ? !pad_rows_applies(p) : !choice_runnable(p, Choice{fam, cfg})) continue;
       if (fam == KSMM_ALGO_SIMT &&
           !ksmm_cu_config_supported(fam, cfg, p.batch, p.a, p.b, p.c, p.d, p.in_dtype, p.out_dtype, p.bs_last))
         continue;
@@ -1992,7 +2007,13 @@ int ksmm_cu_tune(const ksmm_forward_desc_t* desc, int nrepeats, void* stream, in
   if (best < 0.f) return set_error(KSMM_ERR_UNSUPPORTED, "no kernel candidate ran");
   {
     std::lock_guard<std::mutex> g(g_choice_mu);
-    g_choices[key_of(p)] = win;
+    if (win.algo == kAlgoPadRows) {
+      // what untuned calls with scratch do; those without have to go on choosing another way
+      g_choices.erase(key_of(p));
+      win = Choice{KSMM_ALGO_AUTO, -1};
+    } else {
+      g_choices[key_of(p)] = win;
+    }
   }
   if (best_algo) *best_algo = win.algo;
   if (best_config) *best_config = win.config;

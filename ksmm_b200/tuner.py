@@ -24,7 +24,7 @@ from .kernel import dtype_code
 
 _DT_NAME = {_lib.KSMM_F32: "f32", _lib.KSMM_F16: "f16", _lib.KSMM_BF16: "bf16", _lib.KSMM_F8E4M3: "f8e4m3"}
 _DT_CODE = {v: k for k, v in _DT_NAME.items()}
-_ALGO_NAME = {_lib.KSMM_ALGO_SIMT: "ffma", _lib.KSMM_ALGO_TC: "tensor", _lib.KSMM_ALGO_CONVERT: "convert"}
+_ALGO_NAME = {_lib.KSMM_ALGO_AUTO: "auto", _lib.KSMM_ALGO_SIMT: "ffma", _lib.KSMM_ALGO_TC: "tensor", _lib.KSMM_ALGO_CONVERT: "convert"}
 _ALGO_CODE = {v: k for k, v in _ALGO_NAME.items()}
 
 # entries tuned or loaded in this process: key -> dict
@@ -39,7 +39,8 @@ def _key(batch, pattern, in_dtype, out_dtype, bs_last):
 def tune_factor(pattern, batch, dtype=torch.float16, bs_last=True, out_dtype=None, nrepeats=20,
                 device="cuda"):
     """Time every kernel candidate for one factor on scratch buffers of the real
-    size and remember the fastest.  Returns the table entry."""
+    size and remember the fastest.  Returns the table entry; family "auto" says that untuned calls already
+    run the fastest (a batch-last input copied into padded rows), and nothing is remembered."""
     lib = _lib.load()
     a, b, c, d = (int(v) for v in pattern)
     out_dtype = dtype if out_dtype is None else out_dtype
@@ -63,7 +64,10 @@ def tune_factor(pattern, batch, dtype=torch.float16, bs_last=True, out_dtype=Non
     entry = {"sm": cap[0] * 10 + cap[1], "dtype": _DT_NAME[ic], "out_dtype": _DT_NAME[oc],
              "bs_last": bool(bs_last), "pattern": [a, b, c, d], "batch": int(batch),
              "family": _ALGO_NAME[algo.value], "config": int(cfg.value), "ms": float(ms.value)}
-    _table[_key(batch, pattern, ic, oc, bs_last)] = entry
+    if entry["family"] == "auto":
+        _table.pop(_key(batch, pattern, ic, oc, bs_last), None)
+    else:
+        _table[_key(batch, pattern, ic, oc, bs_last)] = entry
     return entry
 
 
@@ -242,7 +246,7 @@ def tune_set(patterns=BENCHMARK_PATTERNS, batch=25088, dtypes=(torch.float32, to
                 entry = tune_factor(pattern, batch, dtype, bs_last, nrepeats=nrepeats)
                 t_tuned = _time_default(pattern, batch, dtype, bs_last, nrepeats)
                 entry["ms"], entry["ms_heuristic"] = t_tuned, t_default
-                same = (entry["family"] == "convert" and conv0) or \
+                same = entry["family"] == "auto" or (entry["family"] == "convert" and conv0) or \
                     (not conv0 and entry["family"] == fam0 and (entry["config"] == cfg0 or cfg0 < 0))
                 keep = (not same) and t_tuned < (1.0 - min_gain) * t_default
                 if keep:

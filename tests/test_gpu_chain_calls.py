@@ -57,3 +57,26 @@ def test_unaligned_input_gradient_stays_inside_the_workspace(pattern, batch, bs_
         assert err < (1e-5 if dtype == torch.float32 else 2.0 ** -11), (shift, err)
         assert bool((gx[:shift] == 7.0).all()) and bool((gx[shift + x.numel():] == 7.0).all())
     kb.check_device()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_tuning_a_ragged_batch_keeps_the_padded_path(dtype):
+    """The copy into padded rows is among the candidates (several times faster at this size); a choice that is
+    set for the ragged rows does not reach the padded ones of a chain."""
+    pattern, batch = (1, 768, 192, 2), 6501
+    lib, code = _lib.load(), _lib.KSMM_F16 if dtype == torch.float16 else _lib.KSMM_F32
+    before = kb.default_choice(pattern, batch, dtype, True)
+    assert before[2], "this batch is not copied"
+    entry = kb.tuner.tune_factor(pattern, batch, dtype, True, nrepeats=5)
+    algo, cfg = ctypes.c_int(), ctypes.c_int()
+    try:
+        assert entry["family"] == "auto" and kb.default_choice(pattern, batch, dtype, True) == before
+        assert lib.ksmm_cu_get_choice(batch, *pattern, code, code, 1, ctypes.byref(algo), ctypes.byref(cfg)) != _lib.KSMM_OK
+        layer = kb.KSLinear([(6, 64, 64, 1), pattern], dtype=dtype, bs_last=True, device=DEV)
+        x = torch.randn(384, batch, device=DEV).to(dtype)
+        ref = layer(x)
+        _lib.check(lib.ksmm_cu_set_choice(batch, *pattern, code, code, 1, _lib.KSMM_ALGO_SIMT, 2))
+        assert torch.equal(layer(x), ref)   # the same kernel, the same bits
+    finally:
+        lib.ksmm_cu_clear_choice(batch, *pattern, code, code, 1)
+    kb.check_device()
