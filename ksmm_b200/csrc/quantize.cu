@@ -88,14 +88,16 @@ __device__ __forceinline__ float tensor_scale(const uint32_t* parts, int nparts,
 
 // v / s rounded as a division rounds it.  With inv = 1 / s rounded, one residual step on v * inv gives that
 // quotient (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor",
-// theorem on division) as long as nothing underflows, which scales outside [2^-100, 2^100] might: those
-// divide.  Three instructions instead of a division's dozen, which bound the quantising kernels (16.6
-// -> 12.6 us for 12544 x 768 bf16, 20.4 -> 18.4 us transposing; both include the wait for the first
-// launch).  Smaller |v| than 2^-100 rounds to zero either way.
+// theorem on division) as long as the residual of a value that matters is no denormal number.  Values
+// below 2^-11 s quantise to zero either way; the residual of a larger one is a multiple of 2^-48 times it,
+// at least 2^-119 for scales from 2^-60 on.  Other scales divide.  So does a scale of 1, the one that a
+// tensor with a NaN gets: its infinities are 448, and would be NaN by the residual step.  Three instructions
+// instead of a division's dozen, which bound the quantising kernels (16.6 -> 12.6 us for 12544 x 768 bf16,
+// 20.4 -> 18.4 us transposing; both include the wait for the first launch).
 struct Scale {
   float s, inv;
   bool plain;  // divide
-  __device__ explicit Scale(float v) : s(v), inv(1.f / v), plain(!(v > 0x1p-100f && v < 0x1p100f)) {}
+  __device__ explicit Scale(float v) : s(v), inv(1.f / v), plain(!(v > 0x1p-60f && v < 0x1p60f) || v == 1.f) {}
   __device__ __forceinline__ float quotient(float v) const {
     if (plain) return v / s;
     const float q = v * inv;

@@ -80,3 +80,26 @@ def test_tuning_a_ragged_batch_keeps_the_padded_path(dtype):
     finally:
         lib.ksmm_cu_clear_choice(batch, *pattern, code, code, 1)
     kb.check_device()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -14])
+@pytest.mark.parametrize("bs_last", [False, True])
+def test_fp8_activations_with_nan_and_infinity(bs_last, scale, dtype):
+    """A NaN makes the tensor's scale 1: infinities and large values are then 448 as quantize_e4m3 has it, and
+    only the entries that meet the NaN are NaN.  (Identity weights: the results are the quantised inputs.)"""
+    n, batch = 64, 48
+    layer = kb.KSLinear([(1, n, n, 1)], weights=[torch.eye(n).view(1, n, n, 1)], bias=False, dtype=torch.float8_e4m3fn,
+                        bs_last=bs_last, device=DEV)
+    x = torch.randn(batch, n, device=DEV).mul_(600 * scale)
+    x[3, 5], x[7, 9], x[8, 2] = float("nan"), float("inf"), float("-inf")
+    x = (x.t().contiguous() if bs_last else x).to(dtype)
+    for clean in (False, True):
+        if clean:   # without the NaN the scale is infinite
+            x = torch.nan_to_num(x, nan=1.0, posinf=float("inf"), neginf=float("-inf"))
+        (wq, sw), = layer._fp8_factors()
+        q, s = kb.quantize_e4m3(x)
+        ref = kb.forward_fp8(q, wq, bs_last, 1, n, n, 1, s, sw)
+        assert torch.equal(torch.isnan(layer(x)), torch.isnan(ref))
+        assert torch.equal(torch.nan_to_num(layer(x)), torch.nan_to_num(ref))
+    kb.check_device()
