@@ -103,3 +103,22 @@ def test_fp8_activations_with_nan_and_infinity(bs_last, scale, dtype):
         assert torch.equal(torch.isnan(layer(x)), torch.isnan(ref))
         assert torch.equal(torch.nan_to_num(layer(x)), torch.nan_to_num(ref))
     kb.check_device()
+
+
+@pytest.mark.parametrize("patterns", [[(1, 48, 32, 1)], [(6, 64, 64, 1), (1, 768, 192, 2)]])
+@pytest.mark.parametrize("bs_last", [False, True])
+def test_bias_gradient_of_long_fp32_batches(patterns, bs_last):
+    """A tree over at most 64 neighbours in fp32 (an rms error of 2^-25 per level, about 2^-24 in all), longer sums
+    in fp64, one rounding at the end: below 2^-23 of the result's norm at any length."""
+    layer = kb.KSLinear(patterns, dtype=torch.float32, bs_last=bs_last, device=DEV, requires_grad=True)
+    for batch in (640, 50176, 50177):
+        x = torch.zeros((layer.in_size, batch) if bs_last else (batch, layer.in_size), device=DEV)
+        gen = torch.Generator(device=DEV).manual_seed(batch)
+        g = torch.randn((layer.out_size, batch) if bs_last else (batch, layer.out_size), device=DEV, generator=gen)
+        for want_x in (False, True):
+            layer.bias.grad = None
+            layer(x.requires_grad_(want_x)).backward(g)
+            ref = g.double().sum(1 if bs_last else 0)
+            err = torch.linalg.norm(layer.bias.grad.reshape(-1).double() - ref) / torch.linalg.norm(ref)
+            assert err.item() < 2.0 ** -23, (batch, want_x, err.item())
+    kb.check_device()
