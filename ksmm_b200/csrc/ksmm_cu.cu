@@ -1368,6 +1368,25 @@ static bool train_one_layout(int nfactors, const int32_t* patterns, int64_t batc
   return nfactors > 8;
 }
 
+// May the layouts be planned?  Another layout can take an fp32 factor from an FFMA kernel to the tensor-core
+// one, whose error is two to six times as large (tc_f32x3.cu).  A trainable fp32 layer keeps the kernels that
+// its factors have one by one, so its layouts are planned only where those run on the tensor cores anyway.
+// (16-bit results round far above either sum's error.)  `grad`: the multiplications by the transposed
+// factors, without the first one if the input's gradient is not wanted.
+static bool train_may_switch(int nfactors, const int32_t* patterns, int64_t batch, int dtype, int bs_last, bool grad,
+                             bool need_input) {
+  if (dtype != KSMM_F32) return true;
+  void* const at = reinterpret_cast<void*>(256);
+  for (int f = grad && !need_input ? 1 : 0; f < nfactors; ++f) {
+    const int32_t* q = patterns + 4 * f;
+    const Problem p = backward_problem(at, at, at, batch, q[0], q[grad ? 2 : 1], q[grad ? 1 : 2], q[3], dtype, bs_last);
+    Choice ch = auto_choice(p);
+    if (ch.algo == KSMM_ALGO_CONVERT) ch = auto_choice(batch_last_twin(p));
+    if (ch.algo != KSMM_ALGO_TC) return false;
+  }
+  return true;
+}
+
 // bytes of one intermediate's buffer
 static size_t train_buffer_bytes(int nfactors, const int32_t* patterns, int64_t batch, int dtype) {
   size_t mx = 0;
@@ -1602,7 +1621,8 @@ int ksmm_cu_chain_train_forward(const void* input, const void* const* values, vo
   if (!input || !output) return set_error(KSMM_ERR_BAD_ARGUMENT, "null pointer");
   if ((st = check_values(nfactors, values)) != KSMM_OK) return st;
   const bool one_layout = train_one_layout(nfactors, patterns, batch, dtype, bs_last);
-  int allow = !one_layout && aligned16(input) && aligned16(output) ? 1 : 0;
+  int allow = !one_layout && aligned16(input) && aligned16(output) &&
+              train_may_switch(nfactors, patterns, batch, dtype, bs_last, false, true) ? 1 : 0;
   for (int f = 0; f < nfactors; ++f) allow &= aligned16(values[f]) ? 1 : 0;
   return chain_walk(true, input, values, output, bias, saved, want[0], scratch, scratch_bytes, /*no_alloc=*/1, batch, nfactors,
                     patterns, dtype, bs_last, bs_last, 0, static_cast<cudaStream_t>(stream), nullptr, allow,
@@ -1633,7 +1653,7 @@ int ksmm_cu_chain_backward(const void* input, const void* const* values, const v
   if (!aligned16(input) || !aligned16(grad_output))
     return set_error(KSMM_ERR_BAD_ARGUMENT, "the backward of a chain takes an input and a gradient aligned to 16 bytes");
   const bool one_layout = train_one_layout(nfactors, patterns, batch, dtype, bs_last);
-  bool allow = aligned16(grad_input);
+  bool allow = aligned16(grad_input) && train_may_switch(nfactors, patterns, batch, dtype, bs_last, true, grad_input != nullptr);
   for (int f = 0; f < nfactors; ++f) allow = allow && aligned16(values[f]);
   size_t need = 0;
   for (int run = 0; run < 2; ++run) {

@@ -122,3 +122,38 @@ def test_bias_gradient_of_long_fp32_batches(patterns, bs_last):
             err = torch.linalg.norm(layer.bias.grad.reshape(-1).double() - ref) / torch.linalg.norm(ref)
             assert err.item() < 2.0 ** -23, (batch, want_x, err.item())
     kb.check_device()
+
+
+@pytest.mark.parametrize("bs_last", [False, True])
+@pytest.mark.parametrize("patterns", [[(1, 64, 64, 16), (4, 64, 64, 4), (16, 64, 64, 1)], [(6, 64, 64, 1), (1, 768, 192, 2)],
+                                      [(1, 192, 768, 4), (4, 192, 192, 1)]])
+def test_trainable_fp32_layers_keep_their_precision(patterns, bs_last):
+    """Against fp64, the layer's result and its input's gradient are no further off than one factor after the
+    other (a tenth more at most: the same sums may run in another order)."""
+    layer = kb.KSLinear(patterns, dtype=torch.float32, bs_last=bs_last, bias=False, device=DEV, requires_grad=True)
+    dense = [kb.from_kernel_format_to_dense(f.data.double(), p) for f, p in zip(layer.factors, patterns)]
+    for batch in (100, 640, 1001):
+        gen = torch.Generator(device=DEV).manual_seed(batch)
+        x = torch.randn((layer.in_size, batch) if bs_last else (batch, layer.in_size), device=DEV, generator=gen)
+        g = torch.randn((layer.out_size, batch) if bs_last else (batch, layer.out_size), device=DEV, generator=gen)
+        y64, x64 = (x if bs_last else x.t()).double(), (g if bs_last else g.t()).double()
+        for m in dense:
+            y64 = m @ y64
+        for m in reversed(dense):
+            x64 = m.t() @ x64
+
+        def errors(run):
+            xi = x.clone().requires_grad_(True)
+            y = run(xi)
+            y.backward(g)
+            return [(torch.linalg.norm((v if bs_last else v.t()).double() - r) / torch.linalg.norm(r)).item()
+                    for v, r in ((y.detach(), y64), (xi.grad, x64))]
+
+        def one_by_one(y):
+            for p, f in zip(patterns, layer.factors):
+                y = kb.FactorFunction.apply(y, f, bs_last, *p)
+            return y
+
+        for name, new, old in zip(("y", "x"), errors(layer), errors(one_by_one)):
+            assert new < 1.1 * old, (name, batch, new, old)
+    kb.check_device()
