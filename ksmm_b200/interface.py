@@ -150,7 +150,8 @@ class KSLinear(nn.Module):
         bias = None if self.bias is None else self.bias.reshape(-1)
         if self.is_fp8:
             quantised = self._fp8_factors()
-            if x.is_cuda and x.numel() and x.dtype in (torch.bfloat16, torch.float16, torch.float32):
+            if x.is_cuda and x.numel() and x.dtype in (torch.bfloat16, torch.float16, torch.float32) \
+                    and self.num_mat <= _k.MAX_FP8_FACTORS:
                 y = _k.chain_forward_fp8(x.detach(), [w for w, _ in quantised], [s for _, s in quantised],
                                          self.patterns, self.bs_last, bias=bias)
             else:

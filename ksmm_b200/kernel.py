@@ -230,6 +230,9 @@ def chain_forward(input, factors, patterns, bs_last, bias=None, workspace=None, 
     return out
 
 
+MAX_FP8_FACTORS = 64  # of one ksmm_cu_chain_forward_fp8 call
+
+
 def chain_forward_fp8(input, factors, scales, patterns, bs_last, bias=None):
     """All factors of an fp8 KSLinear in one library call (``ksmm_cu_chain_forward_fp8``): ``factors[f]`` and
     ``scales[f]`` come from ``quantize_e4m3``; every factor's input is quantised on the device the way

@@ -157,3 +157,18 @@ def test_trainable_fp32_layers_keep_their_precision(patterns, bs_last):
         for name, new, old in zip(("y", "x"), errors(layer), errors(one_by_one)):
             assert new < 1.1 * old, (name, batch, new, old)
     kb.check_device()
+
+
+def test_fp8_layer_of_more_factors_than_one_call_takes():
+    """65 factors run one by one; with 64 of them both ways agree."""
+    n = 16
+    for count in (64, 65):
+        layer = kb.KSLinear([(1, n, n, 1)] * count, weights=[torch.eye(n).view(1, n, n, 1)] * count, bias=False,
+                            dtype=torch.float8_e4m3fn, device=DEV)
+        x = torch.randn(8, n, device=DEV, dtype=torch.bfloat16)
+        y = x
+        for wq, sw in layer._fp8_factors():
+            q, s = kb.quantize_e4m3(y)
+            y = kb.forward_fp8(q, wq, False, 1, n, n, 1, s, sw)
+        assert torch.equal(layer(x), y)
+    kb.check_device()
