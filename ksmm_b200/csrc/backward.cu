@@ -34,6 +34,8 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cfloat>
+#include <cstdint>
 
 #include "backward.h"
 #include "tc_host.h"
@@ -339,11 +341,36 @@ __global__ void __launch_bounds__(kThreadsW, 1)
   }
 }
 
+// What an fp32 sum that is not finite is computed again from.  The three-product split (tc_wgrad_f32.cu) turns
+// an infinite operand into NaN, its rest being inf - inf, and may overflow a little below the largest float.
+struct Again {
+  const float *x, *g;
+  int64_t batch;
+  int b, c, d;
+  // address of (feature r of block (i, l), entry n): i * i + r * r + l * l + n * n
+  struct Strides { int64_t i, r, l, n; } xs, gs;
+};
+
+// the sum of products of element e in the order and precision of wgrad_simt_kernel
+__device__ __noinline__ float sum_again(const Again& A, int64_t e) {
+  const int j = static_cast<int>(e % A.b), k = static_cast<int>(e / A.b % A.c);
+  const int64_t blk = e / A.b / A.c, i = blk / A.d, l = blk % A.d;
+  const float* x = A.x + i * A.xs.i + k * A.xs.r + l * A.xs.l;
+  const float* g = A.g + i * A.gs.i + j * A.gs.r + l * A.gs.l;
+  float acc = 0.f;
+  for (int64_t n0 = 0; n0 < A.batch && acc == acc; n0 += 32) {  // (a NaN stays one)
+    const int64_t end = min(n0 + 32, A.batch);
+#pragma unroll 8
+    for (int64_t n = n0; n < end; ++n) acc = fmaf(x[n * A.xs.n], g[n * A.gs.n], acc);
+  }
+  return acc;
+}
+
 // Sums the partial tiles of the splits in a fixed order and converts to the weights' type.  Four
 // elements per thread (elems is a multiple of 4 in the vector form), four splits in flight.
 template <typename T, int V>
 __global__ void __launch_bounds__(256)
-    wgrad_reduce_kernel(const float* part, T* dw, int64_t elems, int splits) {
+    wgrad_reduce_kernel(const float* part, T* dw, int64_t elems, int splits, const Again A) {
   // (no read-only loads in this kernel: the compiler may move those above the wait)
   grid_dep_wait();
   grid_dep_launch();
@@ -363,18 +390,33 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
       for (int u = 0; u < V; ++u) s[u] += v[u];
     }
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+      for (int u = 0; u < V; ++u)
+        if (!(fabsf(s[u]) <= FLT_MAX)) s[u] = sum_again(A, e * V + u);
+    }
     store_vec<T, V>(dw + e * V, s);
   }
 }
 
 template <typename T>
-static cudaError_t launch_reduce(const float* part, void* dw, int64_t elems, int splits, cudaStream_t stream) {
+static cudaError_t launch_reduce(const Problem& p, const WgradOperand& x, const WgradOperand& g, const float* part,
+                                 int splits, cudaStream_t stream) {
+  void* dw = p.out;
+  const int64_t elems = static_cast<int64_t>(p.a) * p.b * p.c * p.d, d = p.d;
+  auto strides = [&](const WgradOperand& o, int64_t f) {
+    if (o.last) return Again::Strides{f * d * o.ld, d * o.ld, o.ld, 1};
+    if (o.regrouped) return Again::Strides{f * d, 1, f, p.a * f * d};
+    return Again::Strides{f * d, d, 1, p.a * f * d};
+  };
+  const Again A{static_cast<const float*>(x.ptr), static_cast<const float*>(g.ptr), p.batch, p.b, p.c, p.d,
+                strides(x, p.c), strides(g, p.b)};
   const bool vec = elems % 4 == 0 && reinterpret_cast<uintptr_t>(dw) % 16 == 0;
   const int64_t items = vec ? elems / 4 : elems;
   const unsigned grid = static_cast<unsigned>(std::min<int64_t>((items + 255) / 256, 148 * 8));
   if (vec)
-    return launch_pdl(wgrad_reduce_kernel<T, 4>, grid, 256, 0, stream, part, static_cast<T*>(dw), elems, splits);
-  return launch_pdl(wgrad_reduce_kernel<T, 1>, grid, 256, 0, stream, part, static_cast<T*>(dw), elems, splits);
+    return launch_pdl(wgrad_reduce_kernel<T, 4>, grid, 256, 0, stream, part, static_cast<T*>(dw), elems, splits, A);
+  return launch_pdl(wgrad_reduce_kernel<T, 1>, grid, 256, 0, stream, part, static_cast<T*>(dw), elems, splits, A);
 }
 
 template <bool X_LAST, bool G_LAST, int MB, int NT, int SX>
@@ -729,9 +771,9 @@ int wgrad_launch(const Problem& p, WgradOperand x, WgradOperand g, void* workspa
                   : tc::launch_w_tile<false, false>(p, x, g, part, w.mb, w.nt, w.splits, stream);
     }
     if (st != KSMM_OK) return st;
-    cudaError_t err = p.in_dtype == KSMM_F32  ? tc::launch_reduce<float>(part, p.out, elems, w.splits, stream)
-                      : p.in_dtype == KSMM_F16 ? tc::launch_reduce<__half>(part, p.out, elems, w.splits, stream)
-                                               : tc::launch_reduce<__nv_bfloat16>(part, p.out, elems, w.splits, stream);
+    cudaError_t err = p.in_dtype == KSMM_F32   ? tc::launch_reduce<float>(p, x, g, part, w.splits, stream)
+                      : p.in_dtype == KSMM_F16 ? tc::launch_reduce<__half>(p, x, g, part, w.splits, stream)
+                                               : tc::launch_reduce<__nv_bfloat16>(p, x, g, part, w.splits, stream);
     count_launch();
     if (err == cudaSuccess) err = cudaGetLastError();
     if (err != cudaSuccess)

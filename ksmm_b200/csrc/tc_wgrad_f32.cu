@@ -2,7 +2,8 @@
 //   dW[i,j,k,l] = sum_n dY4[i,j,l,n] X4[i,k,l,n],
 // a*d independent (c x B) @ (B x b) products, each term as three tf32 products:
 // hi(x) hi(g) + lo(x) hi(g) + hi(x) lo(g) with fp32 accumulation; hi is the value rounded to a tf32
-// operand, lo the rest.  (An infinite gradient gives NaN, its rest being inf - inf.)
+// operand, lo the rest.  (Infinite operands give NaN, their rest being inf - inf; the reduction in backward.cu
+// computes sums that are not finite once more.)
 //
 // Accumulator rows are k (128 per tile), columns j (NT = 64 or 128), the K dimension of the MMAs is
 // the batch, 32 entries per stage.  A stage holds [X hi | X lo | G hi | G lo]; six splitter warps round

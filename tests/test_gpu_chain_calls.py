@@ -172,3 +172,41 @@ def test_fp8_layer_of_more_factors_than_one_call_takes():
             y = kb.forward_fp8(q, wq, False, 1, n, n, 1, s, sw)
         assert torch.equal(layer(x), y)
     kb.check_device()
+
+
+def _weight_gradient(x, g, bs_last, pattern, fallback=False):
+    """ksmm_cu_backward_weights; without a workspace it runs on the FFMA kernel."""
+    a, b, c, d = pattern
+    lib, code = _lib.load(), {torch.float32: _lib.KSMM_F32, torch.float16: _lib.KSMM_F16, torch.bfloat16: _lib.KSMM_BF16}[x.dtype]
+    batch = x.shape[1] if bs_last else x.shape[0]
+    need = 0 if fallback else lib.ksmm_cu_backward_weights_workspace_bytes(batch, a, b, c, d, code, int(bs_last))
+    ws, out = torch.empty(max(need, 1), dtype=torch.uint8, device=DEV), torch.empty(a * c * d, b, dtype=x.dtype, device=DEV)
+    _lib.check(lib.ksmm_cu_backward_weights(x.data_ptr(), g.data_ptr(), out.data_ptr(), ws.data_ptr() if need else None, need,
+                                            batch, a, b, c, d, code, int(bs_last), _stream()))
+    return out
+
+
+@pytest.mark.parametrize("bs_last", [False, True])
+@pytest.mark.parametrize("pattern", [(1, 64, 64, 1), (2, 64, 32, 2), (1, 50, 70, 3), (1, 41, 37, 1)])
+def test_fp32_weight_gradients_of_infinite_operands(pattern, bs_last):
+    """Infinities, NaN and sums past the largest float are what the FFMA kernel makes of them, bit for bit; the
+    other sums are those of the finite operands."""
+    a, b, c, d = pattern
+    for batch in (128, 1001):
+        gen = torch.Generator(device=DEV).manual_seed(batch)
+        x = torch.randn(a * c * d, batch, device=DEV, generator=gen)
+        g = torch.randn(a * b * d, batch, device=DEV, generator=gen)
+        g[10, batch - 1] = 0.0
+        finite = _weight_gradient(*((x, g) if bs_last else (x.t().contiguous(), g.t().contiguous())), bs_last, pattern)
+        inf = float("inf")
+        x[3, 5], x[7, batch - 1], x[11, 40], x[12, 3] = inf, -inf, 3e38, float("nan")
+        g[2, 9], g[8, 0], g[9, 40] = -inf, inf, -3e38
+        x, g = (x, g) if bs_last else (x.t().contiguous(), g.t().contiguous())
+        dw, ref = (_weight_gradient(x, g, bs_last, pattern, fallback=f) for f in (False, True))
+        odd = ~torch.isfinite(ref)
+        assert odd.any() and torch.isinf(ref).any() and not odd.all()
+        assert torch.equal(torch.isfinite(dw), ~odd)
+        assert torch.equal(torch.nan_to_num(dw[odd], nan=7.0), torch.nan_to_num(ref[odd], nan=7.0))
+        same = ~odd & torch.isfinite(finite) & (ref.abs() < 1e30)
+        assert (torch.linalg.norm((dw - finite)[same]) / torch.linalg.norm(finite[same])).item() < 1e-5
+    kb.check_device()
