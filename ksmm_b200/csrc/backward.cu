@@ -341,8 +341,8 @@ __global__ void __launch_bounds__(kThreadsW, 1)
   }
 }
 
-// What an fp32 sum that is not finite is computed again from.  The three-product split (tc_wgrad_f32.cu) turns
-// an infinite operand into NaN, its rest being inf - inf, and may overflow a little below the largest float.
+// What an fp32 sum that is not finite is computed again from.  The split of the operands (tc_wgrad_f32.cu) turns
+// an infinite one into NaN, its rest being inf - inf, and may overflow a little below the largest float.
 struct Again {
   const float *x, *g;
   int64_t batch;
@@ -547,7 +547,7 @@ WgradPlan plan_wgrad(const Problem& p, const WgradOperand& x, const WgradOperand
   if (p.batch <= 0 || p.batch > 0x7fffffffLL) return w;
   const bool f32 = p.in_dtype == KSMM_F32;
   if (!f32 && p.in_dtype != KSMM_F16 && p.in_dtype != KSMM_BF16) return w;
-  if (f32 && p.batch < 128) return w;  // the FFMA kernel is the more exact one there (tc_wgrad_f32.cu)
+  if (f32 && p.batch < 128) return w;  // the FFMA kernel is the faster one there (tc_wgrad_f32.cu)
   w.copy_x = !wgrad_operand_direct(p, x, p.c, check_pointers);
   w.copy_g = !wgrad_operand_direct(p, g, p.b, check_pointers);
   // The padding of a tile is all the work there is for blocks of a few rows; the FFMA kernel, one CTA
@@ -563,7 +563,7 @@ WgradPlan plan_wgrad(const Problem& p, const WgradOperand& x, const WgradOperand
   if (f32) {
     w.mb = 1;
     w.nt = p.b <= 64 ? 64 : 128;
-    // the three products per term are the time of a chunk of 32 entries (about 0.65 us), not its bytes
+    // (a chunk of 32 entries takes 1.5 us whatever its bytes; 63e3 for it gave the same times)
     w.splits = wgrad_splits(blocks * ((p.c + 127) / 128) * ((p.b + w.nt - 1) / w.nt), (p.batch + 31) / 32,
                             w.nt == 64 ? 22e3 : 30e3, 128.0 * w.nt * 4, elems);
   } else {

@@ -1,33 +1,40 @@
 // fp32 weight gradients on the tensor cores:
 //   dW[i,j,k,l] = sum_n dY4[i,j,l,n] X4[i,k,l,n],
-// a*d independent (c x B) @ (B x b) products, each term as three tf32 products:
-// hi(x) hi(g) + lo(x) hi(g) + hi(x) lo(g) with fp32 accumulation; hi is the value rounded to a tf32
-// operand, lo the rest.  (Infinite operands give NaN, their rest being inf - inf; the reduction in backward.cu
-// computes sums that are not finite once more.)
+// a*d independent (c x B) @ (B x b) products.  Every operand is cut into three bf16 values, each the rounded
+// rest of the ones before it: v = v1 + v2 + v3 exactly (8 + 8 + 8 bits, the signs of the rests included; below
+// 2^-110 the last one may fall under the smallest bf16).  A term is the six products x1 g1, x1 g2, x2 g1,
+// x2 g2, x1 g3, x3 g1, each exact in fp32; x2 g3 and x3 g2, at most 2^-25 of it, are left out (2^-28 on average,
+// next to the 2^-25.3 of one rounding), so that a term is as exact as an fp32 FMA's.  (Two tf32 parts cannot
+// hold 24 bits: one bit was dropped from a quarter of the operands, and gradients of a few entries were two to
+// three times as far from 64 bits as by FFMAs.)  The six bf16 products take the tensor time of three tf32
+// ones.  Infinite operands give NaN, their rest being inf - inf; the reduction in backward.cu computes sums
+// that are not finite once more.
 //
 // Accumulator rows are k (128 per tile), columns j (NT = 64 or 128), the K dimension of the MMAs is
-// the batch, 32 entries per stage.  A stage holds [X hi | X lo | G hi | G lo]; six splitter warps round
-// the raw tiles that TMA delivers in place and add the lo tiles at the same offsets.  G lo follows G hi directly, so the two are one operand of 2 NT rows.  A batch-last operand
-// has rows of consecutive batch entries: K-major, plain 128-byte swizzle.  A batch-first one (d = 1)
-// has rows of consecutive features: MN-major, atoms of 32 features x 32 batch rows with the 128-byte
-// swizzle of 32-byte pieces.  The split is element-wise, so any combination of the two works.
+// the batch, 32 entries per chunk.  TMA delivers raw tiles into one ring; eight splitter warps write their pieces
+// [x1 | x2 | x3 | g1 | g2 | g3] into a second one, whose stages the MMAs read.  g2 follows g1 directly, so
+// the two are one operand of 2 NT rows.  A batch-last operand has rows of consecutive batch entries: K-major
+// pieces with rows of 64 bytes and the 64-byte swizzle.  A batch-first one (d = 1) has rows of consecutive
+// features: MN-major pieces, groups of 64 features x 32 batch rows with the 128-byte swizzle.  The split is
+// element-wise, so any combination of the two works.
 //
 // The contraction is long (a training batch), and the tensor core truncates when it adds into its
-// accumulator, once per step of 8 entries.  So the accumulator only ever sums kFlush chunks (128
-// entries, 16 additions); the epilogue warps then add it, rounded to nearest, to sums in registers,
+// accumulator, once per step of 16 entries.  So the accumulator only ever sums kFlush chunks (128
+// entries, 8 additions); the epilogue warps then add it, rounded to nearest, to sums in registers,
 // while the MMAs fill the other accumulator buffer.  Relative error against 64 bits for N(0,1) operands
-// (the FFMA kernel's in brackets): 1.8e-7 (1.8e-7) at 100 entries, 2.0e-7 (3.2e-7) at 320, 3.5e-7
-// (1.4e-6) at 6272.  With hi cut off instead of rounded and a flush every 512 entries it was 4.8e-7,
-// 4.9e-7 and 1.5e-6.  Below 128 entries the FFMA kernel runs: its few roundings are the smaller error.
+// (the FFMA kernel's in brackets): 7.6e-8 (1.8e-7) at 128 entries, 8.3e-8 (3.2e-7) at 320, 1.4e-7 to 1.8e-7
+// (1.4e-6) at 6272, 2.6e-8 (2.5e-8) where a single entry is not zero.  With two tf32 parts it was 2.0e-7, 2.0e-7,
+// 3.5e-7 and 8.1e-8.  Below 128 entries the FFMA kernel runs: its launch is the shorter one there, (6,64,64,1) at
+// 128 entries 20 us against 26, (1,768,192,2) 34 against 33 and at 256 46 against 33.
 //
-// What bounds it: the shared-memory pipe.  A chunk of 32 entries (NT = 128) is written once by TMA
-// (32 KB), read and written twice by the splitters (96 KB) and read by the MMAs (80 KB), about 1660
-// cycles at 128 bytes a cycle against 1080 for its eight MMAs.  The batch is split over CTAs as in
-// backward.cu; (1,768,192,2) at 6272 batch entries: 49 us (485 us on the FFMA kernel, 47 us without
-// the second write of the splitters).
+// What bounds it: the chain of a chunk, about 1.5 us for NT = 128 (TMA, split, ten MMAs), at the number of stages
+// that fit.  (1,768,192,2) at 6272 batch entries: 58 us with the reduction, as with two tf32 parts (485 us on the
+// FFMA kernel); (1,64,64,16) at 12544 52 us (56 with the tf32 parts), (1,768,192,4) 184 (177), batch-first
+// (1,768,768,1) 148 (134).  For (1,768,192,2) six splitter warps take 62 us, four 64, ten 60; two raw stages and three
+// of pieces 67.
 //
-// Roles (512 threads): warp 0 TMA producer, warp 1 TMEM owner and MMA issuer, warps 2..7 splitters,
-// warps 8..15 epilogue.  Waits are bounded and report through the device status word.
+// Roles (576 threads): warp 0 TMA producer, warp 1 TMEM owner and MMA issuer, warps 2..9 splitters,
+// warps 10..17 epilogue.  Waits are bounded and report through the device status word.
 #include <cuda.h>
 
 #include <atomic>
@@ -51,69 +58,94 @@ struct ParamsWF {
   int* status;
 };
 
-constexpr int kSplitWarpsWF = 6;
+constexpr int kSplitWarpsWF = 8;
 constexpr int kThreadsWF = (2 + kSplitWarpsWF + 8) * 32;
 constexpr int kFlush = 4;  // chunks per accumulator buffer
 
-__device__ __forceinline__ void umma_tf32_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// v = hi + lo: hi the nearest value with the 11 significant bits of a tf32 operand (towards zero where
-// rounding would leave the range), lo the exact rest, at most 12 bits of which the tensor core drops one
-__device__ __forceinline__ uint32_t hi_of(uint32_t v) {
-  const uint32_t r = (v & 0x7fffffffu) < 0x7f7ff000u ? v + 0x1000u : v;
-  return r & 0xFFFFE000u;
-}
-__device__ __forceinline__ uint32_t rest_of(uint32_t v, uint32_t hi) {
-  return __float_as_uint(__uint_as_float(v) - __uint_as_float(hi));
+// the three pieces of two neighbouring values; v becomes the rest of the first two
+__device__ __forceinline__ uint32_t next_piece(float& v0, float& v1) {
+  const __nv_bfloat162 p = __floats2bfloat162_rn(v0, v1);
+  const uint32_t w = *reinterpret_cast<const uint32_t*>(&p);
+  v0 -= __uint_as_float(w << 16);
+  v1 -= __uint_as_float(w & 0xffff0000u);
+  return w;
 }
 
-template <int NT, int ST>
+// Cuts one unit of a tile, eight values that lie next to each other in 16-byte pieces of a 128-byte swizzled raw row,
+// into 16 bytes of each piece tile.  K-major (LAST): row = feature, q = octet of batch entries; MN-major: row =
+// batch entry, q = octet of features.  Eight neighbouring lanes take eight rows: no bank conflicts on either side.
+template <bool LAST>
+__device__ __forceinline__ void split_unit(uint32_t raw, uint32_t pieces, uint32_t piece_bytes, int u, int rows) {
+  const int row = LAST ? u & (rows - 1) : u & 31, q = LAST ? u / rows : u >> 5;
+  const uint32_t src = raw + (LAST ? row * 128 : (q >> 2) * 4096 + row * 128);
+  const int p = (LAST ? q : q & 3) * 2;
+  const uint32_t dst = pieces + (LAST ? row * 64 + ((q ^ ((row >> 1) & 3)) << 4)
+                                      : (q >> 3) * 4096 + row * 128 + (((q & 7) ^ (row & 7)) << 4));
+  float v[8];
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v[4 * h]), "=f"(v[4 * h + 1]), "=f"(v[4 * h + 2]), "=f"(v[4 * h + 3])
+                 : "r"(src + (((p + h) ^ (row & 7)) << 4))
+                 : "memory");
+#pragma unroll
+  for (int t = 0; t < 3; ++t) {
+    uint32_t w[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) w[e] = next_piece(v[2 * e], v[2 * e + 1]);
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + t * piece_bytes), "r"(w[0]), "r"(w[1]), "r"(w[2]),
+                 "r"(w[3])
+                 : "memory");
+  }
+}
+
+// RT raw stages, ST stages of pieces
+template <int NT, int RT, int ST>
 struct CfgWF {
-  static constexpr int X_BYTES = 128 * 128;  // 128 k x 32 batch entries (either order)
-  static constexpr int G_BYTES = NT * 128;   // NT j x 32 batch entries
-  static constexpr int G_OFF = 2 * X_BYTES;
-  static constexpr int STAGE_BYTES = 2 * X_BYTES + 2 * G_BYTES;
-  static constexpr int NBAR = 3 * ST + 4;
+  static constexpr int X_RAW = 128 * 128, RAW_BYTES = X_RAW + NT * 128;  // 32 batch entries of 128 k and NT j (either order)
+  static constexpr int X_PIECE = 128 * 64, G_PIECE = NT * 64;
+  static constexpr int G_OFF = 3 * X_PIECE;
+  static constexpr int STAGE_BYTES = 3 * X_PIECE + 3 * G_PIECE;
+  static constexpr int NBAR = 2 * RT + 2 * ST + 4;
   static constexpr int BAR_BYTES = 256;
-  static constexpr int SMEM_BYTES = ST * STAGE_BYTES + BAR_BYTES + 1024;
+  static constexpr int SMEM_BYTES = RT * RAW_BYTES + ST * STAGE_BYTES + BAR_BYTES + 1024;
   static constexpr int BUF_COLS = 2 * NT;  // leading accumulator | small-terms accumulator
   static constexpr int TMEM_COLS = 2 * BUF_COLS;
   static_assert(NT == 64 || NT == 128, "j tile");
+  static_assert(RT * RAW_BYTES >= 8 * (NT / 64) * 4096, "staging of the partial tile");
   static_assert(SMEM_BYTES <= 232448, "shared memory budget");
   static_assert(SMEM_BYTES > 116 * 1024, "one CTA per SM, so that the TMEM allocation never waits");
   static_assert(8 * NBAR + 16 <= BAR_BYTES, "barrier area");
 };
 
-template <bool X_LAST, bool G_LAST, int NT, int ST>
+template <bool X_LAST, bool G_LAST, int NT, int RT, int ST>
 __global__ void __launch_bounds__(kThreadsWF, 1)
     ksmm_tc_wgrad_f32_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmG,
                              const __grid_constant__ CUtensorMap tmP, const ParamsWF P) {
-  using C = CfgWF<NT, ST>;
+  using C = CfgWF<NT, RT, ST>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t sm0 = (raw + 1023u) & ~1023u;
   uint8_t* sm_gen = smem_raw + (sm0 - raw);
-  const uint32_t stage0 = sm0;
+  const uint32_t raw0 = sm0, stage0 = raw0 + RT * C::RAW_BYTES;
   const uint32_t bar0 = stage0 + ST * C::STAGE_BYTES;
-  uint8_t* bar_gen = sm_gen + ST * C::STAGE_BYTES;
-  auto full_bar = [&](int s) { return bar0 + 8u * s; };             // TMA: raw tiles landed
-  auto split_bar = [&](int s) { return bar0 + 8u * (ST + s); };     // splitters: lo tiles written
-  auto free_bar = [&](int s) { return bar0 + 8u * (2 * ST + s); };  // MMA commit: stage consumed
-  auto tfull_bar = [&](int q) { return bar0 + 8u * (3 * ST + q); };
-  auto tempty_bar = [&](int q) { return bar0 + 8u * (3 * ST + 2 + q); };
+  uint8_t* bar_gen = sm_gen + RT * C::RAW_BYTES + ST * C::STAGE_BYTES;
+  auto full_bar = [&](int s) { return bar0 + 8u * s; };                    // TMA: raw tiles landed
+  auto read_bar = [&](int s) { return bar0 + 8u * (RT + s); };             // splitters: raw tiles read
+  auto split_bar = [&](int s) { return bar0 + 8u * (2 * RT + s); };        // splitters: pieces written
+  auto free_bar = [&](int s) { return bar0 + 8u * (2 * RT + ST + s); };    // MMA commit: pieces consumed
+  auto tfull_bar = [&](int q) { return bar0 + 8u * (2 * RT + 2 * ST + q); };
+  auto tempty_bar = [&](int q) { return bar0 + 8u * (2 * RT + 2 * ST + 2 + q); };
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_gen + 8 * C::NBAR);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bar_gen + 8 * C::NBAR + 4);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < ST; ++s) {
+    for (int s = 0; s < RT; ++s) {
       mbar_init(full_bar(s), 1);
+      mbar_init(read_bar(s), kSplitWarpsWF);
+    }
+    for (int s = 0; s < ST; ++s) {
       mbar_init(split_bar(s), kSplitWarpsWF);
       mbar_init(free_bar(s), 1);
     }
@@ -156,16 +188,16 @@ __global__ void __launch_bounds__(kThreadsWF, 1)
     if (lane == 0) {
       uint32_t si = 0, sph = 0;
       for (int ch = ch_begin; ch < ch_end; ++ch) {
-        if (!mbar_wait<64>(free_bar(si), sph ^ 1u, abort_flag, P.status, 61)) break;
-        const uint32_t dst = stage0 + si * C::STAGE_BYTES;
+        if (!mbar_wait<64>(read_bar(si), sph ^ 1u, abort_flag, P.status, 61)) break;
+        const uint32_t dst = raw0 + si * C::RAW_BYTES;
         const uint32_t bar = full_bar(si);
-        mbar_expect_tx(bar, C::X_BYTES + C::G_BYTES);
+        mbar_expect_tx(bar, C::RAW_BYTES);
         const int n0 = ch * 32;
         if constexpr (X_LAST) tma_load_4d(dst, &tmX, bar, n0, l, k0, i);
         else tma_load_4d(dst, &tmX, bar, 0, n0, k0 / 32, blk);
-        if constexpr (G_LAST) tma_load_4d(dst + C::G_OFF, &tmG, bar, n0, l, j0, i);
-        else tma_load_4d(dst + C::G_OFF, &tmG, bar, 0, n0, j0 / 32, blk);
-        if (++si == ST) { si = 0; sph ^= 1u; }
+        if constexpr (G_LAST) tma_load_4d(dst + C::X_RAW, &tmG, bar, n0, l, j0, i);
+        else tma_load_4d(dst + C::X_RAW, &tmG, bar, 0, n0, j0 / 32, blk);
+        if (++si == RT) { si = 0; sph ^= 1u; }
       }
     }
     __syncwarp();
@@ -184,18 +216,24 @@ __global__ void __launch_bounds__(kThreadsWF, 1)
           if (!mbar_wait<0>(split_bar(si), sph, abort_flag, P.status, 63)) { ok = false; break; }
           tc_fence_after();
           const uint32_t xb = stage0 + si * C::STAGE_BYTES, gb = xb + C::G_OFF;
+          // K-major: 8 rows of 64 bytes are 512 bytes apart, a k step of 16 entries is 32 bytes inside the row;
+          // MN-major: 4 KB between groups of 64 features, 1 KB between groups of 8 batch rows
+          auto xd = [&](int t, int ks) {
+            const uint32_t at = xb + t * C::X_PIECE;
+            return X_LAST ? make_desc(at + ks * 32, 16, 512, 4) : make_desc(at + ks * 2048, 4096, 1024, 2);
+          };
+          auto gd = [&](int t, int ks) {
+            const uint32_t at = gb + t * C::G_PIECE;
+            return G_LAST ? make_desc(at + ks * 32, 16, 512, 4) : make_desc(at + ks * 2048, 4096, 1024, 2);
+          };
 #pragma unroll
-          for (int ks = 0; ks < 4; ++ks) {
-            // K-major rows of 32 entries: a k step is 32 bytes inside the row; MN-major atoms of 32
-            // features: 4 KB between atoms, 512 bytes between groups of 4 batch rows
-            const uint64_t xhi = X_LAST ? make_desc(xb + ks * 32, 16, 1024, 2) : make_desc(xb + ks * 1024, 4096, 512, 1);
-            const uint64_t xlo = X_LAST ? make_desc(xb + C::X_BYTES + ks * 32, 16, 1024, 2)
-                                        : make_desc(xb + C::X_BYTES + ks * 1024, 4096, 512, 1);
-            const uint64_t gst = G_LAST ? make_desc(gb + ks * 32, 16, 1024, 2) : make_desc(gb + ks * 1024, 4096, 512, 1);
-            // hi(x) * [hi(g) | lo(g)]: the leading accumulator and, next to it, the small one
-            umma_tf32_ss(dcol, xhi, gst, P.idesc2, (first && ks == 0) ? 0u : 1u);
-            // lo(x) * hi(g): only the first NT rows of the same operand
-            umma_tf32_ss(dsmall, xlo, gst, P.idesc, 1u);
+          for (int ks = 0; ks < 2; ++ks) {
+            // x1 * [g1 | g2]: the leading accumulator and, next to it, the small one
+            umma<2>(dcol, xd(0, ks), gd(0, ks), P.idesc2, (first && ks == 0) ? 0u : 1u);
+            umma<2>(dsmall, xd(0, ks), gd(2, ks), P.idesc, 1u);
+            umma<2>(dsmall, xd(1, ks), gd(0, ks), P.idesc, 1u);
+            umma<2>(dsmall, xd(1, ks), gd(1, ks), P.idesc, 1u);
+            umma<2>(dsmall, xd(2, ks), gd(0, ks), P.idesc, 1u);
           }
           umma_commit(free_bar(si));
           if (++si == ST) { si = 0; sph ^= 1u; }
@@ -207,34 +245,28 @@ __global__ void __launch_bounds__(kThreadsWF, 1)
   } else if (warp < 2 + kSplitWarpsWF) {
     // ===================== splitters =====================
     const int tt = (warp - 2) * 32 + lane;
-    constexpr int kXP = C::X_BYTES / 16, kP = (C::X_BYTES + C::G_BYTES) / 16;
-    uint32_t si = 0, sph = 0;
+    constexpr int kXU = 128 * 4, kU = kXU + NT * 4;  // units of 8 values
+    uint32_t ri = 0, rph = 0, si = 0, sph = 0;
     for (int ch = ch_begin; ch < ch_end; ++ch) {
       int got = 1;
-      if (lane == 0) got = mbar_wait<32>(full_bar(si), sph, abort_flag, P.status, 64) ? 1 : 0;
+      if (lane == 0)
+        got = mbar_wait<32>(full_bar(ri), rph, abort_flag, P.status, 64) &&
+              mbar_wait<32>(free_bar(si), sph ^ 1u, abort_flag, P.status, 66) ? 1 : 0;
       got = __shfl_sync(0xffffffffu, got, 0);
       if (!got) break;
-      const uint32_t sb = stage0 + si * C::STAGE_BYTES;
-#pragma unroll 4
-      for (int pc = tt; pc < kP; pc += kSplitWarpsWF * 32) {
-        const bool on_g = pc >= kXP;
-        const uint32_t hb = sb + (on_g ? C::G_OFF + (pc - kXP) * 16 : pc * 16);
-        const uint32_t lb = hb + (on_g ? C::G_BYTES : C::X_BYTES);
-        uint32_t v[4];
-        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
-                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
-                     : "r"(hb)
-                     : "memory");
-        const uint32_t h0 = hi_of(v[0]), h1 = hi_of(v[1]), h2 = hi_of(v[2]), h3 = hi_of(v[3]);
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(hb), "r"(h0), "r"(h1), "r"(h2), "r"(h3)
-                     : "memory");
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(lb), "r"(rest_of(v[0], h0)),
-                     "r"(rest_of(v[1], h1)), "r"(rest_of(v[2], h2)), "r"(rest_of(v[3], h3))
-                     : "memory");
+      const uint32_t rb = raw0 + ri * C::RAW_BYTES, sb = stage0 + si * C::STAGE_BYTES;
+#pragma unroll 2
+      for (int u = tt; u < kU; u += kSplitWarpsWF * 32) {
+        if (u < kXU) split_unit<X_LAST>(rb, sb, C::X_PIECE, u, 128);
+        else split_unit<G_LAST>(rb + C::X_RAW, sb + C::G_OFF, C::G_PIECE, u - kXU, NT);
       }
-      fence_proxy_async();  // the tiles are read by the tensor core through the async proxy
+      fence_proxy_async();  // the pieces are read by the tensor core through the async proxy
       __syncwarp();
-      if (lane == 0) mbar_arrive(split_bar(si));
+      if (lane == 0) {
+        mbar_arrive(split_bar(si));
+        mbar_arrive(read_bar(ri));
+      }
+      if (++ri == RT) { ri = 0; rph ^= 1u; }
       if (++si == ST) { si = 0; sph ^= 1u; }
     }
     __syncwarp();
@@ -270,14 +302,14 @@ __global__ void __launch_bounds__(kThreadsWF, 1)
     }
     const int krow0 = k0 + q * 32;
     if (ok && krow0 < P.c) {
-      // the last buffer is complete, so every stage has been consumed: the ring is free for staging
+      // the last buffer is complete, so every raw tile has been read: that ring is free for staging
       const int pz = sp * P.a * P.d + blk;
 #pragma unroll
       for (int cg = 0; cg < NT / 64; ++cg) {
         const int jc = j0 + h * (NT / 2) + cg * 32;
         if (jc >= P.b) break;
         if (P.tma_part) {
-          const uint32_t stg = stage0 + ((warp - 2 - kSplitWarpsWF) * 2 + cg) * 4096;
+          const uint32_t stg = raw0 + ((warp - 2 - kSplitWarpsWF) * 2 + cg) * 4096;
 #pragma unroll
           for (int c4 = 0; c4 < 8; ++c4)
             asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stg + lane * 128 + ((c4 ^ (lane & 7)) << 4)),
@@ -314,11 +346,11 @@ __global__ void __launch_bounds__(kThreadsWF, 1)
   }
 }
 
-template <bool X_LAST, bool G_LAST, int NT, int ST>
+template <bool X_LAST, bool G_LAST, int NT, int RT, int ST>
 static int launch_wf(const Problem& p, const WgradOperand& x, const WgradOperand& g, float* part, int splits,
                      cudaStream_t stream) {
-  using C = CfgWF<NT, ST>;
-  auto kern = ksmm_tc_wgrad_f32_kernel<X_LAST, G_LAST, NT, ST>;
+  using C = CfgWF<NT, RT, ST>;
+  auto kern = ksmm_tc_wgrad_f32_kernel<X_LAST, G_LAST, NT, RT, ST>;
   static std::atomic<bool> attr_set[64];  // zero-initialised; set once per device (a repeated set is harmless)
   int dev = 0;
   cudaGetDevice(&dev);
@@ -338,12 +370,12 @@ static int launch_wf(const Problem& p, const WgradOperand& x, const WgradOperand
       const uint64_t L = o.ld;
       const uint64_t dims[4] = {B, d, f, a}, str[4] = {1, L, d * L, f * d * L};
       const uint32_t box[4] = {32, 1, rows, 1};
-      return encode_map(tm, KSMM_F32, 4, o.ptr, dims, str, box, true, false);
+      return encode_map(tm, KSMM_F32, 4, o.ptr, dims, str, box);
     }
     // d = 1: (feature % 32, batch, feature / 32, a): rows / 32 atoms of 32 features x 32 batch rows
     const uint64_t dims[4] = {32, B, f / 32, a}, str[4] = {1, a * f, 32, f};
     const uint32_t box[4] = {32, 32, rows / 32, 1};
-    return encode_map(tm, KSMM_F32, 4, o.ptr, dims, str, box, true, true);
+    return encode_map(tm, KSMM_F32, 4, o.ptr, dims, str, box);
   };
   if ((st = operand_map(&tmX, X_LAST, x, c, 128)) != KSMM_OK) return st;
   if ((st = operand_map(&tmG, G_LAST, g, b, NT)) != KSMM_OK) return st;
@@ -363,8 +395,8 @@ static int launch_wf(const Problem& p, const WgradOperand& x, const WgradOperand
   }
   P.status = status_word();
   if (!P.status) return set_error(KSMM_ERR_CUDA, "cannot resolve the device status word");
-  // fp32 accumulate, tf32 operands, M = 128; batch-last operands are K-major, batch-first ones MN-major
-  const uint32_t common = (1u << 4) | (2u << 7) | (2u << 10) | (X_LAST ? 0u : 1u << 15) | (G_LAST ? 0u : 1u << 16) |
+  // fp32 accumulate, bf16 operands, M = 128; batch-last operands are K-major, batch-first ones MN-major
+  const uint32_t common = (1u << 4) | (1u << 7) | (1u << 10) | (X_LAST ? 0u : 1u << 15) | (G_LAST ? 0u : 1u << 16) |
                           (static_cast<uint32_t>(128 >> 4) << 24);
   P.idesc = common | (static_cast<uint32_t>(NT >> 3) << 17);
   P.idesc2 = common | (static_cast<uint32_t>(2 * NT >> 3) << 17);
@@ -383,8 +415,8 @@ static int launch_wf(const Problem& p, const WgradOperand& x, const WgradOperand
 template <bool X_LAST, bool G_LAST>
 static int launch_wf_tile(const Problem& p, const WgradOperand& x, const WgradOperand& g, float* part, int nt,
                           int splits, cudaStream_t stream) {
-  return nt == 64 ? launch_wf<X_LAST, G_LAST, 64, 4>(p, x, g, part, splits, stream)
-                  : launch_wf<X_LAST, G_LAST, 128, 3>(p, x, g, part, splits, stream);
+  return nt == 64 ? launch_wf<X_LAST, G_LAST, 64, 4, 3>(p, x, g, part, splits, stream)
+                  : launch_wf<X_LAST, G_LAST, 128, 4, 2>(p, x, g, part, splits, stream);
 }
 
 }  // namespace tc

@@ -199,7 +199,7 @@ def test_fp32_weight_gradients_of_infinite_operands(pattern, bs_last):
         g[10, batch - 1] = 0.0
         finite = _weight_gradient(*((x, g) if bs_last else (x.t().contiguous(), g.t().contiguous())), bs_last, pattern)
         inf = float("inf")
-        x[3, 5], x[7, batch - 1], x[11, 40], x[12, 3] = inf, -inf, 3e38, float("nan")
+        x[3, 5], x[7, batch - 1], x[11, 40], x[12, 3] = inf, -inf, 3.4e38, float("nan")
         g[2, 9], g[8, 0], g[9, 40] = -inf, inf, -3e38
         x, g = (x, g) if bs_last else (x.t().contiguous(), g.t().contiguous())
         dw, ref = (_weight_gradient(x, g, bs_last, pattern, fallback=f) for f in (False, True))
@@ -209,4 +209,29 @@ def test_fp32_weight_gradients_of_infinite_operands(pattern, bs_last):
         assert torch.equal(torch.nan_to_num(dw[odd], nan=7.0), torch.nan_to_num(ref[odd], nan=7.0))
         same = ~odd & torch.isfinite(finite) & (ref.abs() < 1e30)
         assert (torch.linalg.norm((dw - finite)[same]) / torch.linalg.norm(finite[same])).item() < 1e-5
+    kb.check_device()
+
+
+@pytest.mark.parametrize("bs_last", [False, True])
+@pytest.mark.parametrize("pattern", [(1, 64, 64, 1), (2, 96, 160, 2), (1, 50, 70, 3)])
+def test_fp32_weight_gradients_of_a_few_entries(pattern, bs_last):
+    """Masked batches, against 64 bits and the FFMA kernel.  One entry is one product, rounded once, 2^-24, after the
+    split has left out two terms of at most 2^-25: as the FMA has it.  m entries in different splits of the batch
+    round every term and every sum, 2 m - 1 times where a chain of FMAs rounds m times: below sqrt(2) times its
+    error.  Dense batches are closer than the chain."""
+    a, b, c, d = pattern
+    for batch in (128, 1001, 6272):
+        for count in (1, 2, 3, 4, 16, 64, batch):
+            gen = torch.Generator(device=DEV).manual_seed(batch + count)
+            x = torch.randn(a * c * d, batch, device=DEV, generator=gen)
+            g = torch.randn(a * b * d, batch, device=DEV, generator=gen)
+            g[:, torch.randperm(batch, device=DEV, generator=gen)[count:]] = 0
+            ref = torch.einsum("ikln,ijln->ilkj", x.double().reshape(a, c, d, batch), g.double().reshape(a, b, d, batch))
+            ref = ref.reshape(a * d * c, b)
+            x, g = (x, g) if bs_last else (x.t().contiguous(), g.t().contiguous())
+            off = [_weight_gradient(x, g, bs_last, pattern, fallback=f).double() - ref for f in (False, True)]
+            new, old = (torch.linalg.norm(o).item() for o in off)
+            assert new < {1: 1.05, batch: 1.0}.get(count, 2 ** 0.5) * old, (batch, count, new, old)
+            if count == 1:
+                assert (off[0].abs() / ref.abs()).max().item() < 2.0 ** -23
     kb.check_device()
