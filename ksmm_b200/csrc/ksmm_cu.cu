@@ -992,6 +992,9 @@ static int chain_forward_impl(const void* input, const void* const* values, void
   if (out_bs_last != 0 && out_bs_last != 1)
     return set_error(KSMM_ERR_BAD_ARGUMENT, "the output layout must be 0 (batch-first) or 1 (batch-last)");
   if (batch < 0) return set_error(KSMM_ERR_BAD_ARGUMENT, "negative batch");
+  // (an empty batch has empty, possibly null, buffers)
+  if (batch > 0 && (!input || !output)) return set_error(KSMM_ERR_BAD_ARGUMENT, "null pointer");
+  if (batch > 0 && (st = check_values(nfactors, values)) != KSMM_OK) return st;
   // layout-changing factors go through TMA on both sides: every buffer has to be 16-byte aligned
   auto al16 = [](const void* q) { return reinterpret_cast<uintptr_t>(q) % 16 == 0; };
   int allow_switch = al16(input) && al16(output) && al16(workspace) && al16(residual) ? 1 : 0;
@@ -1214,6 +1217,8 @@ int ksmm_cu_grouped_chain_forward(const void* input, const void* const* values, 
   if (st != KSMM_OK) return st;
   if (bs_last != 0 && bs_last != 1) return set_error(KSMM_ERR_BAD_ARGUMENT, "bs_last must be 0 or 1");
   if (batch < 0) return set_error(KSMM_ERR_BAD_ARGUMENT, "negative batch");
+  if (batch > 0 && (!input || !output)) return set_error(KSMM_ERR_BAD_ARGUMENT, "null pointer");
+  if (batch > 0 && (st = check_values(nfactors, values)) != KSMM_OK) return st;
   // per group: the intermediates of one chain; whatever follows the groups' intermediates is
   // layout scratch for the factors that run group by group
   const size_t inter1 = chain_intermediate_bytes(nfactors, patterns, batch, dtype, 0);

@@ -233,3 +233,29 @@ def test_training_and_fp8_calls_refuse_misuse_before_the_device():
     assert fp8(ws=None) == fp8(ws=p + 16) == fp8(room=16) == small
     assert lib.ksmm_cu_launch_count() == before
     del owner
+
+
+def test_chain_calls_refuse_null_pointers_before_the_device():
+    """Null input, output or factor: a status and no launch, also where the chain would begin with a copy of its
+    input (a ragged batch-last one, a change of layout) or run its groups in one launch.  An empty batch has none."""
+    lib = _lib.load()
+    owner, p = _aligned_buffer()
+    pats = [(2, 64, 64, 1), (1, 64, 64, 2)]
+    pat, n, big = _lib.int32_array([v for q in pats for v in q]), 2, 1 << 40
+    bad = _lib.KSMM_ERR_BAD_ARGUMENT
+    ptrs = lambda *v: (ctypes.c_void_p * n)(*v)  # noqa: E731
+    before = lib.ksmm_cu_launch_count()
+    for batch in (64, 61):
+        for last in (0, 1):
+            for x, vals, y in ((None, ptrs(p, p), p), (p, ptrs(p, p), None), (p, ptrs(None, p), p), (p, ptrs(p, None), p)):
+                for out_last in (0, 1):
+                    assert lib.ksmm_cu_chain_forward_layouts(x, vals, y, None, p, big, batch, n, pat, _lib.KSMM_F16, last,
+                                                             out_last, 0, None) == bad
+                assert lib.ksmm_cu_grouped_chain_forward(x, vals, y, None, p, big, batch, n, pat, _lib.KSMM_F16, last, 3,
+                                                         None) == bad
+    assert lib.ksmm_cu_chain_forward_layouts(None, ptrs(None, None), None, None, None, 0, 0, n, pat, _lib.KSMM_F16, 0, 0, 0,
+                                             None) == _lib.KSMM_OK
+    assert lib.ksmm_cu_grouped_chain_forward(None, ptrs(None, None), None, None, None, 0, 0, n, pat, _lib.KSMM_F16, 0, 3,
+                                             None) == _lib.KSMM_OK
+    assert lib.ksmm_cu_launch_count() == before
+    del owner
