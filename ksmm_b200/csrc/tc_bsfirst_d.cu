@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(kThreadsD, 1)
       const uint32_t buf = ut % C::NBUF, bph = (ut / C::NBUF) & 1u;
       int got = 1;
       if (etron) KSMM_TRACE(3, 20);
-      if (lane == 0) got = mbar_wait<128>(tfull_bar(buf), bph, abort_flag, P.status, 17) ? 1 : 0;
+      if (lane == 0) got = mbar_wait<128>(tfull_bar(buf), bph, abort_flag, P.status, 20) ? 1 : 0;
       got = __shfl_sync(0xffffffffu, got, 0);
       if (!got) break;
       if (etron) KSMM_TRACE(3, 21);

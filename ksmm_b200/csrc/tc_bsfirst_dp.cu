@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(kThreadsP, 1)
         const int n0 = static_cast<int>(row % P.tiles_n) * 128;
         for (int lp = 0; lp < D / 2 && ok; ++lp) {
           for (int kc = 0; kc < nkc; ++kc) {
-            if (!mbar_wait<64>(free_bar(si), sph ^ 1u, abort_flag, P.status, 51)) { ok = false; break; }
+            if (!mbar_wait<64>(free_bar(si), sph ^ 1u, abort_flag, P.status, 71)) { ok = false; break; }
             const uint32_t sb = stage0 + si * C::STAGE_BYTES;
             mbar_expect_tx(full_bar(si), C::STAGE_BYTES);
             // regrouped input seen as (k, n, l, i, group): two tiles of 128 rows x 64 k
@@ -177,12 +177,12 @@ __global__ void __launch_bounds__(kThreadsP, 1)
       bool ok = true;
       for (uint32_t row = row_begin; row < row_end && ok; ++row, ++ut) {
         const uint32_t buf = ut % C::NBUF, bph = (ut / C::NBUF) & 1u;
-        if (!mbar_wait<0>(tempty_bar(buf), bph ^ 1u, abort_flag, P.status, 52)) { ok = false; break; }
+        if (!mbar_wait<0>(tempty_bar(buf), bph ^ 1u, abort_flag, P.status, 72)) { ok = false; break; }
         tc_fence_after();
         const uint32_t dcol = tmem_base + buf * C::BUF_COLS;
         for (int lp = 0; lp < D / 2 && ok; ++lp) {
           for (int kc = 0; kc < nkc; ++kc) {
-            if (!mbar_wait<0>(full_bar(si), sph, abort_flag, P.status, 53)) { ok = false; break; }
+            if (!mbar_wait<0>(full_bar(si), sph, abort_flag, P.status, 73)) { ok = false; break; }
             tc_fence_after();
             const uint32_t ab = stage0 + si * C::STAGE_BYTES, wb = ab + C::A_BYTES;
 #pragma unroll
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(kThreadsP, 1)
       const uint32_t buf = ut % C::NBUF, bph = (ut / C::NBUF) & 1u;
       int got = 1;
       if (etron) KSMM_TRACE(3, 20);
-      if (lane == 0) got = mbar_wait<128>(tfull_bar(buf), bph, abort_flag, P.status, 17) ? 1 : 0;
+      if (lane == 0) got = mbar_wait<128>(tfull_bar(buf), bph, abort_flag, P.status, 74) ? 1 : 0;
       got = __shfl_sync(0xffffffffu, got, 0);
       if (!got) break;
       if (etron) KSMM_TRACE(3, 21);

@@ -1020,6 +1020,20 @@ int tc_wait_probe(long long limit_cycles, int code, cudaStream_t stream) {
   return KSMM_OK;
 }
 
+// The kernel whose bounded wait has the code; which of its waits it is shows at the call of mbar_wait.
+static const char* wait_place(int code) {
+  if (code < 10) return "the tensor-core kernel (tc_kernel.cu)";
+  if (code < 21) return "the batch-first kernel for interleaved blocks (tc_bsfirst_d.cu)";
+  if (code < 23) return "the fp32 FFMA kernel (ffma_tma_kernel.cu)";
+  if (code < 30) return "the batch-first fp32 FFMA kernel (ffma_tma_first.cu)";
+  if (code < 50) return "the fp32 tensor-core kernel (tc_f32x3.cu)";
+  if (code < 60) return "the weight-gradient kernel (backward.cu)";
+  if (code < 70) return "the batch-first kernel for groups of eight blocks (tc_bsfirst_g.cu)";
+  if (code < 80) return "the kernel for block-ordered inputs (tc_bsfirst_dp.cu)";
+  if (code < 90) return "the fp32 weight-gradient kernel (tc_wgrad_f32.cu)";
+  return "the wait probe";
+}
+
 int tc_check_device(cudaStream_t stream) {
   cudaError_t e = cudaStreamSynchronize(stream);
   if (e != cudaSuccess)
@@ -1034,11 +1048,7 @@ int tc_check_device(cudaStream_t stream) {
   if (code != 0) {
     int zero = 0;
     cudaMemcpy(w, &zero, sizeof(int), cudaMemcpyHostToDevice);
-    return set_error(KSMM_ERR_DEVICE_TIMEOUT,
-                     "a tensor-core kernel gave up waiting (code %d: 1 producer/input slot, "
-                     "2 producer/weight stage, 3 mma/accumulator, 4 mma/input, 5 mma/weights, "
-                     "6 epilogue/accumulator)",
-                     code);
+    return set_error(KSMM_ERR_DEVICE_TIMEOUT, "%s gave up waiting (code %d)", wait_place(code), code);
   }
   return KSMM_OK;
 }

@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(kThreadsWF, 1)
     if (lane == 0) {
       uint32_t si = 0, sph = 0;
       for (int ch = ch_begin; ch < ch_end; ++ch) {
-        if (!mbar_wait<64>(read_bar(si), sph ^ 1u, abort_flag, P.status, 61)) break;
+        if (!mbar_wait<64>(read_bar(si), sph ^ 1u, abort_flag, P.status, 81)) break;
         const uint32_t dst = raw0 + si * C::RAW_BYTES;
         const uint32_t bar = full_bar(si);
         mbar_expect_tx(bar, C::RAW_BYTES);
@@ -208,12 +208,12 @@ __global__ void __launch_bounds__(kThreadsWF, 1)
       bool ok = true;
       for (int ch = ch_begin; ch < ch_end && ok; ++ut) {
         const uint32_t buf = ut & 1u, bph = (ut >> 1) & 1u;
-        if (!mbar_wait<0>(tempty_bar(buf), bph ^ 1u, abort_flag, P.status, 62)) { ok = false; break; }
+        if (!mbar_wait<0>(tempty_bar(buf), bph ^ 1u, abort_flag, P.status, 82)) { ok = false; break; }
         tc_fence_after();
         const uint32_t dcol = tmem_base + buf * C::BUF_COLS, dsmall = dcol + NT;
         const int stop = min(ch + kFlush, ch_end);
         for (bool first = true; ch < stop; ++ch, first = false) {
-          if (!mbar_wait<0>(split_bar(si), sph, abort_flag, P.status, 63)) { ok = false; break; }
+          if (!mbar_wait<0>(split_bar(si), sph, abort_flag, P.status, 83)) { ok = false; break; }
           tc_fence_after();
           const uint32_t xb = stage0 + si * C::STAGE_BYTES, gb = xb + C::G_OFF;
           // K-major: 8 rows of 64 bytes are 512 bytes apart, a k step of 16 entries is 32 bytes inside the row;
@@ -250,8 +250,8 @@ __global__ void __launch_bounds__(kThreadsWF, 1)
     for (int ch = ch_begin; ch < ch_end; ++ch) {
       int got = 1;
       if (lane == 0)
-        got = mbar_wait<32>(full_bar(ri), rph, abort_flag, P.status, 64) &&
-              mbar_wait<32>(free_bar(si), sph ^ 1u, abort_flag, P.status, 66) ? 1 : 0;
+        got = mbar_wait<32>(full_bar(ri), rph, abort_flag, P.status, 84) &&
+              mbar_wait<32>(free_bar(si), sph ^ 1u, abort_flag, P.status, 86) ? 1 : 0;
       got = __shfl_sync(0xffffffffu, got, 0);
       if (!got) break;
       const uint32_t rb = raw0 + ri * C::RAW_BYTES, sb = stage0 + si * C::STAGE_BYTES;
@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(kThreadsWF, 1)
     for (int ch = ch_begin; ch < ch_end; ch += kFlush, ++ut) {
       const uint32_t buf = ut & 1u, bph = (ut >> 1) & 1u;
       int got = 1;
-      if (lane == 0) got = mbar_wait<128>(tfull_bar(buf), bph, abort_flag, P.status, 65) ? 1 : 0;
+      if (lane == 0) got = mbar_wait<128>(tfull_bar(buf), bph, abort_flag, P.status, 85) ? 1 : 0;
       got = __shfl_sync(0xffffffffu, got, 0);
       if (!got) { ok = false; break; }
       tc_fence_after();

@@ -259,3 +259,19 @@ def test_chain_calls_refuse_null_pointers_before_the_device():
                                              None) == _lib.KSMM_OK
     assert lib.ksmm_cu_launch_count() == before
     del owner
+
+
+def test_wait_codes_name_one_place():
+    """Every bounded wait of the kernels has a code of its own, and the message of ksmm_cu_check_device names the
+    file that it stands in."""
+    import pathlib
+    import re
+    csrc = pathlib.Path(__file__).resolve().parent.parent / "ksmm_b200" / "csrc"
+    place = {}
+    for f in sorted(csrc.glob("*.cu")):
+        for code in re.findall(r"status, (\d+)\)", f.read_text()):
+            assert place.setdefault(int(code), f.name) == f.name, f"code {code}: {place[int(code)]} and {f.name}"
+    rules = re.findall(r'if \(code < (\d+)\) return ".*\((\w+\.cu)\)"', (csrc / "tc_kernel.cu").read_text())
+    assert len(place) > 40 and len(rules) == 9
+    for code, name in place.items():
+        assert name == next(n for limit, n in rules if code < int(limit)), code
