@@ -13,7 +13,7 @@
 // zero-filled by TMA; stores are predicated.
 //
 // Requirements (else the register-staged kernel runs): fp32, batch-last,
-// batch % 4 == 0, b % 4 == 0, 16-byte aligned pointers.
+// b % 4 == 0, input rows (of the batch, or padded) that are multiples of 16 bytes, input and weights aligned to 16 bytes.
 //
 // Reference counterpart: kernel_bs_last_float
 // (src/ksmm_py/layer/kronecker_sparse/template_kernels_float.cuh:301-491).

@@ -70,8 +70,8 @@ static int simt_launch_raw(const Problem& p, int config, cudaStream_t stream) {
   if (config == kFfmaTmaWide || config == kFfmaTmaNarrow) {
     if (!ffma_tma_supported(p, true))
       return set_error(KSMM_ERR_UNSUPPORTED,
-                       "the TMA-staged fp32 kernel needs fp32, batch-last, batch %% 4 == 0, "
-                       "b %% 4 == 0 and 16-byte aligned pointers");
+                       "the TMA-staged fp32 kernel needs fp32, batch-last, input rows that are multiples of "
+                       "16 bytes, b %% 4 == 0 and an input and weights aligned to 16 bytes");
     return ffma_tma_launch(p, config == kFfmaTmaWide, stream);
   }
   if (config == kFfmaTmaFirst) {

@@ -516,7 +516,6 @@ __global__ void __launch_bounds__(kThreads, Cfg<IN_LAST, OUT_LAST, ES, OS, NT, K
                     if (lane == 0) y16[0] = static_cast<uint16_t>(w[rr]);
                     else if (2 * lane < cols) *reinterpret_cast<uint32_t*>(y16 + 2 * lane - 1) = (prev[rr] >> 16) | (w[rr] << 16);
                     else if (2 * lane - 1 < cols) y16[2 * lane - 1] = static_cast<uint16_t>(prev[rr] >> 16);
-                    if (lane == 31 && cols > 63) y16[63] = static_cast<uint16_t>(w[rr] >> 16);
                   }
                 }
               }
