@@ -244,6 +244,10 @@ def chain_forward_fp8(input, factors, scales, patterns, bs_last, bias=None):
     lib = _lib.load()
     bs_last = int(bool(bs_last))
     nf = len(patterns)
+    if nf == 0 or len(factors) != nf or len(scales) != nf:
+        raise ValueError("need one factor and one scale per pattern")
+    if input.dim() != 2 or not input.is_cuda or not input.is_contiguous():
+        raise ValueError("input must be a contiguous 2-D CUDA tensor")
     feats = input.shape[0] if bs_last else input.shape[1]
     for (a, b, c, d), w in zip(patterns, factors):
         if feats != a * c * d:
@@ -253,8 +257,9 @@ def chain_forward_fp8(input, factors, scales, patterns, bs_last, bias=None):
         if w.device != input.device:
             raise ValueError("input and factor live on different devices")
         feats = a * b * d
-    if bias is not None and (bias.numel() != feats or bias.dtype != torch.bfloat16 or not bias.is_contiguous()):
-        raise ValueError("bias must hold a*b*d contiguous elements of the output dtype")
+    if bias is not None and (bias.numel() != feats or bias.dtype != torch.bfloat16 or not bias.is_contiguous()
+                             or bias.device != input.device):
+        raise ValueError("bias must hold a*b*d contiguous elements of the output dtype on the input's device")
     batch = input.shape[1] if bs_last else input.shape[0]
     out = torch.empty((feats, batch) if bs_last else (batch, feats), dtype=torch.bfloat16, device=input.device)
     pat = _lib.int32_array([int(v) for p in patterns for v in p])

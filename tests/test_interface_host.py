@@ -197,3 +197,13 @@ def test_stacked_factors_follow_their_layers():
         group.layers[0].factors[0] = torch.nn.Parameter(torch.zeros(1), requires_grad=False)
         group.layers[0].factors[0] = torch.nn.Parameter(values.clone(), requires_grad=False)
         assert not stale()
+
+
+def test_fp8_chain_refuses_what_it_cannot_read():
+    """Host tensors, strided inputs, missing factors or scales: an error before any pointer reaches the library."""
+    x = torch.zeros(8, 16)
+    w = torch.zeros(16, 16).to(torch.float8_e4m3fn)
+    pat = [(1, 16, 16, 1)]
+    for args in ((x, [w], [1.0], pat), (x[0], [w], [1.0], pat), (x, [], [], []), (x, [w], [], pat), (x, [], [1.0], pat)):
+        with pytest.raises(ValueError):
+            kmod.chain_forward_fp8(*args, False)
