@@ -372,8 +372,9 @@ static int launch_wf(const Problem& p, const WgradOperand& x, const WgradOperand
       const uint32_t box[4] = {32, 1, rows, 1};
       return encode_map(tm, KSMM_F32, 4, o.ptr, dims, str, box);
     }
-    // d = 1: (feature % 32, batch, feature / 32, a): rows / 32 atoms of 32 features x 32 batch rows
-    const uint64_t dims[4] = {32, B, f / 32, a}, str[4] = {1, a * f, 32, f};
+    // (feature % 32, batch, feature / 32, block): rows / 32 atoms of 32 features x 32 batch rows.  The a blocks of
+    // d = 1 and the a * d of block-ordered rows follow one another.
+    const uint64_t dims[4] = {32, B, f / 32, a * d}, str[4] = {1, a * d * f, 32, f};
     const uint32_t box[4] = {32, 32, rows / 32, 1};
     return encode_map(tm, KSMM_F32, 4, o.ptr, dims, str, box);
   };

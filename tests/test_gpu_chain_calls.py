@@ -235,3 +235,26 @@ def test_fp32_weight_gradients_of_a_few_entries(pattern, bs_last):
             if count == 1:
                 assert (off[0].abs() / ref.abs()).max().item() < 2.0 ** -23
     kb.check_device()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("d", [2, 4])
+def test_weight_gradient_of_a_block_ordered_intermediate(d, dtype):
+    """Layout 2 of ksmm_cu_chain_backward, also where no forward of that type keeps it: every block of the factor is
+    read.  Tolerance: one rounding step of the type (fp32: its sums)."""
+    pats, batch = [(2, 32 * d, 64, 1), (1, 96, 64, d)], 200
+    gen = torch.Generator(device=DEV).manual_seed(d)
+    code = _lib.KSMM_F32 if dtype == torch.float32 else _lib.KSMM_F16
+    pat, (saved_bytes, _, need) = _train_bytes(pats, batch, code, 0)
+    x, h, g = (torch.randn(batch, n, device=DEV, generator=gen).to(dtype) for n in (128, 64 * d, 96 * d))
+    w = [torch.randn(a * c * q, b, device=DEV, generator=gen).to(dtype) for a, b, c, q in pats]
+    saved = torch.zeros(saved_bytes, dtype=torch.uint8, device=DEV)
+    saved.view(dtype)[:h.numel()] = h.view(batch, 64, d).transpose(1, 2).reshape(-1)
+    gw, ws = torch.empty_like(w[1]), torch.empty(need, dtype=torch.uint8, device=DEV)
+    _lib.check(_lib.load().ksmm_cu_chain_backward(
+        x.data_ptr(), (ctypes.c_void_p * 2)(*[v.data_ptr() for v in w]), saved.data_ptr(), (ctypes.c_int32 * 1)(2), g.data_ptr(), None,
+        (ctypes.c_void_p * 2)(None, gw.data_ptr()), None, ws.data_ptr(), need, batch, 2, pat, code, 0, _stream()))
+    ref = torch.einsum("nkl,njl->lkj", h.double().view(batch, 64, d), g.double().view(batch, 96, d)).reshape(64 * d, 96)
+    err = (torch.linalg.norm(gw.double() - ref) / torch.linalg.norm(ref)).item()
+    assert err < (1e-6 if dtype == torch.float32 else 2.0 ** -11), err
+    kb.check_device()
