@@ -12,7 +12,8 @@
 // workspace allocation, stream): a layer of two factors on
 // 16 rows 51 -> 19 us, a training step of two factors 270 -> 160 us where the kernels take less.  They return None where an
 // argument is not what the call takes; the Python wrappers then run the same call through ctypes and raise
-// what is wrong with it.  A status other than KSMM_OK comes back as that number.
+// what is wrong with it.  A status other than KSMM_OK comes back as that number; inside the autograd node of
+// layer_train it raises what the wrappers raise for it.
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
@@ -346,6 +347,13 @@ py::object grouped_forward(const at::Tensor& x, const std::vector<at::Tensor>& f
   return result(st, out);
 }
 
+// Raises ksmm_b200.KsmmError for a status, on whichever thread autograd runs (with or without the GIL).
+void raise_status(int st) {
+  if (st == KSMM_OK) return;
+  py::gil_scoped_acquire gil;
+  py::module_::import("ksmm_b200._lib").attr("check")(st);
+}
+
 // A trainable layer as one autograd node: ksmm_b200.kernel.ChainFunction without Python in its backward.
 at::Tensor aligned(const at::Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 ? t.clone() : t; }
 
@@ -360,13 +368,13 @@ struct ChainNode : torch::autograd::Function<ChainNode> {
     const int64_t batch = x.size(last ? 1 : 0), n_out = static_cast<int64_t>(pl[0]) * pl[1] * pl[3];
     const int code = dtype_code(x);
     size_t bytes[3];
-    check_status(ksmm_cu_chain_train_bytes(n, flat.data(), batch, code, last, &bytes[0], &bytes[1], &bytes[2]));
+    raise_status(ksmm_cu_chain_train_bytes(n, flat.data(), batch, code, last, &bytes[0], &bytes[1], &bytes[2]));
     at::Tensor out = new_tensor(n_out, batch, last, x.options());
     const at::Tensor saved = new_bytes(bytes[0], x), scratch = new_bytes(bytes[1], x);
     std::vector<const void*> vals(n);
     for (int f = 0; f < n; ++f) vals[f] = factors[f].data_ptr();
     int32_t layouts[16] = {};
-    check_status(ksmm_cu_chain_train_forward(x.data_ptr(), vals.data(), out.data_ptr(), ptr_or_null(bias), saved.data_ptr(),
+    raise_status(ksmm_cu_chain_train_forward(x.data_ptr(), vals.data(), out.data_ptr(), ptr_or_null(bias), saved.data_ptr(),
                                              bytes[0], scratch.data_ptr(), bytes[1], batch, n, flat.data(), code, last, layouts,
                                              stream_of(x)));
     torch::autograd::variable_list keep{x, saved};
@@ -413,7 +421,7 @@ struct ChainNode : torch::autograd::Function<ChainNode> {
       }
     }
     const at::Tensor ws = new_bytes(need, x);
-    check_status(ksmm_cu_chain_backward(x.data_ptr(), vals.data(), saved.data_ptr(), layouts.data(), g.data_ptr(),
+    raise_status(ksmm_cu_chain_backward(x.data_ptr(), vals.data(), saved.data_ptr(), layouts.data(), g.data_ptr(),
                                         gx.defined() ? gx.data_ptr() : nullptr, outs.data(),
                                         gb.defined() ? gb.data_ptr() : nullptr, ws.data_ptr(), need, x.size(last ? 1 : 0), n,
                                         flat.data(), dtype_code(x), last, stream_of(x)));

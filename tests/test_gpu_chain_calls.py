@@ -258,3 +258,20 @@ def test_weight_gradient_of_a_block_ordered_intermediate(d, dtype):
     err = (torch.linalg.norm(gw.double() - ref) / torch.linalg.norm(ref)).item()
     assert err < (1e-6 if dtype == torch.float32 else 2.0 ** -11), err
     kb.check_device()
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_training_raises_library_statuses(native, monkeypatch):
+    """A status in the backward (fp32 batches this short take at most 65535 blocks) is a KsmmError with that status,
+    through the extension module as through ctypes."""
+    from ksmm_b200 import kernel as kk
+    if not native:
+        monkeypatch.setattr(kk, "_native", None)
+    layer = kb.KSLinear([(65536, 1, 1, 1)], dtype=torch.float32, bias=False, device=DEV, requires_grad=True)
+    x = torch.randn(2, 65536, device=DEV, requires_grad=True)
+    y = layer(x)
+    assert torch.equal(y.detach(), x.detach() * layer.factors[0].detach().reshape(-1))
+    with pytest.raises(kb.KsmmError) as err:
+        y.sum().backward()
+    assert err.value.status == _lib.KSMM_ERR_UNSUPPORTED and "blocks" in str(err.value)
+    kb.check_device()
