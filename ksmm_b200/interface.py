@@ -171,14 +171,17 @@ class KSLinear(nn.Module):
                 or (self.bias is not None and self.bias.requires_grad)):
             # differentiable path: one autograd node for the factors and the bias (one per factor for very
             # long chains); the activation is a torch op
+            # (the node takes a bias of the input's type; any other is added as torch promotes it)
+            own_bias = self.bias is None or (self.bias.dtype == x.dtype and self.bias.is_contiguous()
+                                             and self.num_mat <= 16)
             if self.num_mat <= 16:
-                y = _k.chain_train(x, list(self.factors), self.patterns, self.bs_last, self.bias)
+                y = _k.chain_train(x, list(self.factors), self.patterns, self.bs_last, self.bias if own_bias else None)
             else:
                 y = x
                 for p, f in zip(self.patterns, self.factors):
                     y = _k.FactorFunction.apply(y, f, self.bs_last, *p)
-                if self.bias is not None:
-                    y = y + (self.bias.reshape(-1, 1) if self.bs_last else self.bias.reshape(1, -1))
+            if not own_bias:
+                y = y + (self.bias.reshape(-1, 1) if self.bs_last else self.bias.reshape(1, -1))
             if self.out_bs_last != bool(self.bs_last):
                 y = y.t().contiguous()
             if self.activation == "gelu":

@@ -275,3 +275,23 @@ def test_training_raises_library_statuses(native, monkeypatch):
         y.sum().backward()
     assert err.value.status == _lib.KSMM_ERR_UNSUPPORTED and "blocks" in str(err.value)
     kb.check_device()
+
+
+@pytest.mark.parametrize("bs_last", [False, True])
+def test_trainable_layers_with_another_bias(bs_last):
+    """A bias of another type or with strides is added outside the node, as torch promotes it."""
+    layer = kb.KSLinear([(4, 48, 48, 1), (1, 192, 48, 4)], dtype=torch.float16, bs_last=bs_last, device=DEV, requires_grad=True)
+    x = torch.randn((192, 40) if bs_last else (40, 192), device=DEV, dtype=torch.float16)
+    shape = layer.bias.shape
+    with torch.no_grad():
+        plain = layer(x) - layer.bias.detach().reshape((-1, 1) if bs_last else (1, -1))
+    for bias in (torch.randn(768, device=DEV), torch.randn(768, 2, device=DEV, dtype=torch.float16)[:, 0]):
+        layer.bias = torch.nn.Parameter(bias.view(shape) if bias.is_contiguous() else bias)
+        y = layer(x)
+        want = plain.float() + bias.float().reshape((-1, 1) if bs_last else (1, -1))
+        assert y.dtype == torch.promote_types(torch.float16, bias.dtype)
+        assert (torch.linalg.norm(y.float() - want) / torch.linalg.norm(want)).item() < 2.0 ** -10
+        y.float().sum().backward()
+        assert torch.equal(layer.bias.grad.float(), torch.full_like(layer.bias.grad, 40.0).float())
+        layer.zero_grad(set_to_none=True)
+    kb.check_device()
