@@ -1067,6 +1067,7 @@ int ksmm_cu_chain_forward_layouts(const void* input, const void* const* values, 
 // ---------------------------------------------------------------------------
 struct Fp8Buffers {
   size_t q = 0, y = 0;  // bytes of the quantised input, of one of the two bf16 intermediates
+  int turn_at = -1;     // the factor whose input turns batch-last
   size_t parts() const { return align_up(quantize_parts_bytes(), 256); }
   size_t total() const { return 256 + parts() + q + 2 * y; }  // (scales first)
 };
@@ -1096,7 +1097,9 @@ static int chain_fp8_walk(bool run, const void* input, int in_dtype, const void*
     p.no_alloc = 1;
     p.bs_last = layout;
     p.out = ybuf;
-    const bool turn = !layout && auto_choice(p).algo == KSMM_ALGO_CONVERT;
+    // (the run turns where the sizes of its buffers were made for it, whatever has been tuned in between)
+    if (!run && !layout && auto_choice(p).algo == KSMM_ALGO_CONVERT) buf->turn_at = f;
+    const bool turn = buf->turn_at == f;
     if (turn) p.bs_last = 1;
     const int64_t q_ld = p.bs_last ? padded_ld(batch, 1) : n_in;
     const int64_t y_ld = p.bs_last ? padded_ld(batch, 2) : n_out;
