@@ -295,3 +295,27 @@ def test_trainable_layers_with_another_bias(bs_last):
         assert torch.equal(layer.bias.grad.float(), torch.full_like(layer.bias.grad, 40.0).float())
         layer.zero_grad(set_to_none=True)
     kb.check_device()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("patterns", [[(4, 192, 192, 1), (1, 192, 192, 4)], [(2, 64, 40, 1), (1, 72, 32, 4)],
+                                      [(2, 128, 64, 1), (2, 136, 64, 2)]])
+def test_grouped_block_ordered_chains(patterns, dtype):
+    """One launch per factor for all groups, each group with its own weights and bias, at batches that end inside a
+    tile.  Tolerance: two factors, one rounding step each."""
+    gen = torch.Generator(device=DEV).manual_seed(7)
+    group = kb.KSLinearGroup([kb.KSLinear(patterns, dtype=dtype, device=DEV) for _ in range(3)])
+    for batch in (1, 33, 197, 1001):
+        x = torch.randn(batch, group.layers[0].in_size, device=DEV, generator=gen).to(dtype)
+        group(x)
+        before = kb.launch_count()
+        out = group(x)
+        assert kb.launch_count() - before == len(patterns), batch
+        for y, layer in zip(out, group.layers):
+            ref = x.double()
+            for f, p in zip(layer.factors, patterns):
+                ref = ref @ kb.from_kernel_format_to_dense(f.data.double(), p).t()
+            ref = ref + layer.bias.double()
+            err = (torch.linalg.norm(y.double() - ref) / torch.linalg.norm(ref)).item()
+            assert err < (2.0 ** -10 if dtype == torch.float16 else 2.0 ** -7), (batch, err)
+    kb.check_device()
