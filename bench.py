@@ -263,6 +263,22 @@ def run_profile_case(name, local_rank):
             g = torch.randn((a * b * d, BATCH), device=dev, dtype=torch.float16, generator=gen)
             for _ in range(3):
                 y = kb.backward_weights(x, g, True, a, b, c, d)
+        elif name == "wgrad_fp32":
+            a, b, c, d = 1, 768, 192, 2
+            x = torch.randn((a * c * d, 6272), device=dev, generator=gen)
+            g = torch.randn((a * b * d, 6272), device=dev, generator=gen)
+            for _ in range(3):
+                y = kb.backward_weights(x, g, True, a, b, c, d)
+        elif name == "fp8":
+            layer = kb.KSLinear([(4, 192, 192, 1), (1, 768, 192, 4)], dtype=torch.float8_e4m3fn, bs_last=False, device=dev)
+            x = torch.randn((12544, 768), device=dev, generator=gen).to(torch.bfloat16)
+            for _ in range(3):
+                y = layer(x)
+        elif name == "ragged":
+            layer = kb.KSLinear([(6, 64, 64, 1), (1, 768, 192, 2)], dtype=torch.float16, bs_last=True, device=dev)
+            x = torch.randn((384, 6501), device=dev, generator=gen).to(torch.float16)
+            for _ in range(3):
+                y = layer(x)
         elif name == "qkv":
             layers = [kb.KSLinear([(1, 768, 768, 1)], bias=False, dtype=torch.float16, bs_last=False, device=dev)
                       for _ in range(3)]
@@ -797,7 +813,7 @@ def main():
                     help="skip re-timing the fp32 cases on the FFMA family (the fp32_ffma_only line)")
     ap.add_argument("--sweep-configs", action="store_true",
                     help="also time every tile configuration of every case (printed to stderr)")
-    ap.add_argument("--profile-case", default=None, choices=["mlp_pair", "wgrad", "qkv", "chain_fp32"],
+    ap.add_argument("--profile-case", default=None, choices=["mlp_pair", "wgrad", "wgrad_fp32", "fp8", "ragged", "qkv", "chain_fp32"],
                     help="run a few launches of a chain / backward / grouped workload and exit (profiler captures)")
     ap.add_argument("--only", default=None,
                     help='restrict the sweep: "dtype:layout:a,b,c,d", e.g. "fp16:bs_last:1,768,192,4"')

@@ -308,10 +308,14 @@ KSMM_API int ksmm_cu_chain_backward(const void* input, const void* const* values
  *   grad_output has the forward output's shape, grad_input the input's.
  * ksmm_cu_backward_weights: grad_values[(i*d + l)*c + k, j] = sum over the
  *   batch of grad_output[(i, j, l), n] * input[(i, k, l), n], in the kernel
- *   format and type of the weights (fp32 accumulation).  16-bit batch-last
- *   and batch-first d = 1 problems run on the tensor cores with the batch
- *   split over CTAs; they need ..._workspace_bytes of fp32 partial sums
- *   (without it, and for every other case, a plain FFMA kernel runs).
+ *   format and type of the weights (fp32 accumulation).  Blocks with b, c >= 16
+ *   (16-bit: smaller ones too where the operands need no copy) run on the
+ *   tensor cores with the batch split over CTAs, in every layout; fp32 from 128
+ *   entries on, every operand cut into three bf16 parts that hold all its
+ *   bits, so that a sum is as close to 64 bits as by fp32 FMAs (a few entries
+ *   in different splits of the batch: within sqrt(2) of it) and infinities and
+ *   NaN come out as by FMAs.  They need ..._workspace_bytes for partial sums and
+ *   copies (without it, and for every other case, a plain FFMA kernel runs).
  */
 KSMM_API size_t ksmm_cu_backward_input_workspace_bytes(int64_t batch, int a, int b, int c, int d,
                                                        int dtype, int bs_last);

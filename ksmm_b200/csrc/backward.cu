@@ -517,7 +517,7 @@ struct WgradPlan {
 };
 
 // Splits of the batch.  A CTA's time is its chunks plus its partial tile, both as bytes that cross
-// L2 (about 45 GB/s per SM in these kernels), plus a fixed 2 us; CTAs run in waves of one per SM; the
+// L2 (45 to 52 GB/s per SM in the 16-bit kernel: 308 MB in 41 us on 144 CTAs), plus a fixed 2 us; CTAs run in waves of one per SM; the
 // reduction then reads all partials.
 int wgrad_splits(int64_t tiles, int64_t nchunks, double chunk_bytes, double tile_bytes, double elems) {
   int sms = tc::num_sms();

@@ -473,9 +473,8 @@ __global__ void __launch_bounds__(kThreads, Cfg<IN_LAST, OUT_LAST, ES, OS, NT, K
             // Rows that start anywhere: the warp writes the staging tile one output row at a time, 32
             // words per store instruction.  A 16-bit row that starts on an odd element takes its
             // words from two neighbouring lanes and its two ends as single elements.  Sixteen rows are
-            // read ahead of their stores; the stores are what it costs, about 11 cycles each per SM:
-            // (1,768,192,2) fp16 13 us at 6504 columns, 22 at 6502, 30 at 6501.  (Runs of 128 entries whose
-            // pieces meet on 128-byte lines, three shorter stores a row, measured 34 and 48 us.)
+            // read ahead of their stores; the stores are what it costs: a call of (1,768,192,2) fp16 takes
+            // 12.5 us at 6504 columns, 28 at 6502 and 41 at 6501 (the copy of the input included).
             __syncwarp();
             const int cols = col_limit - cbi * C::CB;                      // columns of this tile that exist
             const int rows_here = min(32, row_limit - q * 32);

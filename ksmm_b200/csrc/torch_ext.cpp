@@ -9,8 +9,8 @@
 //
 // The package's own layers go through layer_forward, layer_train, factor_forward, fp8_forward and
 // grouped_forward below, which hold everything between Python and the C ABI (argument checks, output and
-// workspace allocation, stream): a layer of two factors on
-// 16 rows 51 -> 19 us, a training step of two factors 270 -> 160 us where the kernels take less.  They return None where an
+// workspace allocation, stream): two factors (384 -> 1536, fp16) on 16 rows 48 -> 20 us against the same calls
+// through ctypes, a training step of that layer 241 -> 151 us.  They return None where an
 // argument is not what the call takes; the Python wrappers then run the same call through ctypes and raise
 // what is wrong with it.  A status other than KSMM_OK comes back as that number; inside the autograd node of
 // layer_train it raises what the wrappers raise for it.

@@ -196,8 +196,8 @@ int launch_transpose(const void* in, void* out, int64_t rows, int64_t cols, int 
 // the source start anywhere.  A thread makes 16-byte pieces of the destination out of the two aligned
 // 16-byte words that hold them in the source (byte shifts in registers), so that every access of a warp
 // is a run of whole lines; the last piece of a row, and pieces whose words would reach outside the
-// source tensor, go element by element.  Bound by memory: 384 x 6501 fp16 (10 MB moved) 3 us, 9 us with
-// one element per thread and access.
+// source tensor, go element by element.  384 x 6501 fp16, 5 MB read from DRAM and 5 MB
+// written: 6.7 us, a launch and the loads' latency.
 struct PitchArgs {
   const uint8_t* in;
   uint8_t* out;
