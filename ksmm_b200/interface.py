@@ -171,9 +171,10 @@ class KSLinear(nn.Module):
                 or (self.bias is not None and self.bias.requires_grad)):
             # differentiable path: one autograd node for the factors and the bias (one per factor for very
             # long chains); the activation is a torch op
-            # (the node takes a bias of the input's type; any other is added as torch promotes it)
+            # (the node takes a bias of the input's type with an element per output; any other is added as torch
+            # promotes and broadcasts it)
             own_bias = self.bias is None or (self.bias.dtype == x.dtype and self.bias.is_contiguous()
-                                             and self.num_mat <= 16)
+                                             and self.bias.numel() == self.out_size and self.num_mat <= 16)
             if self.num_mat <= 16:
                 y = _k.chain_train(x, list(self.factors), self.patterns, self.bs_last, self.bias if own_bias else None)
             else:

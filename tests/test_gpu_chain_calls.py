@@ -297,6 +297,21 @@ def test_trainable_layers_with_another_bias(bs_last):
     kb.check_device()
 
 
+@pytest.mark.parametrize("bs_last", [False, True])
+def test_trainable_layers_with_one_bias_for_all_outputs(bs_last):
+    """A bias of one element is added to every output, and its gradient is the sum over all of them."""
+    layer = kb.KSLinear([(4, 48, 48, 1), (1, 192, 48, 4)], dtype=torch.float32, bs_last=bs_last, device=DEV, requires_grad=True)
+    x = torch.randn((192, 40) if bs_last else (40, 192), device=DEV)
+    layer.bias = torch.nn.Parameter(torch.zeros(1, device=DEV))
+    plain = layer(x).detach()
+    layer.bias = torch.nn.Parameter(torch.full((1,), 0.5, device=DEV))
+    y = layer(x)
+    assert torch.equal(y.detach(), plain + 0.5)
+    y.sum().backward()
+    assert layer.bias.grad.item() == 768 * 40
+    kb.check_device()
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("patterns", [[(4, 192, 192, 1), (1, 192, 192, 4)], [(2, 64, 40, 1), (1, 72, 32, 4)],
                                       [(2, 128, 64, 1), (2, 136, 64, 2)]])
