@@ -415,6 +415,13 @@ static size_t scratch_need(const Problem& p, const Choice& ch) {
   return 0;
 }
 
+// the same where a conversion may do without padded rows
+static size_t least_scratch_need(const Problem& p, const Choice& ch) {
+  Problem u = p;
+  u.no_pad = 1;
+  return std::min(scratch_need(p, ch), ch.algo == KSMM_ALGO_CONVERT ? scratch_need(u, ch) : SIZE_MAX);
+}
+
 static int dispatch(const Problem& p, int algo, int config, cudaStream_t stream) {
   int st = check_problem(p);
   if (st != KSMM_OK) return st;
@@ -787,6 +794,7 @@ static int chain_walk(bool run, const void* input, const void* const* values, vo
   void* f_scratch = nullptr;
   size_t f_scratch_bytes = 0;
   int f_no_alloc = no_alloc;
+  bool own_region = false;
   if (run && batch > 0) {
     size_t total = 0;
     int stp = chain_walk(false, nullptr, nullptr, nullptr, nullptr, nullptr, inter_bytes, nullptr, 0, 0, batch,
@@ -803,7 +811,8 @@ static int chain_walk(bool run, const void* input, const void* const* values, vo
       t_post = t_pre + pre_bytes;
       f_scratch = t_post + post_bytes;
       f_scratch_bytes = total - pre_bytes - post_bytes;
-      f_no_alloc = 1;  // what the factors need is inside the region by construction
+      f_no_alloc = 1;  // what the factors need on aligned addresses is inside the region by construction
+      own_region = !no_alloc;
     }
   }
   if (plan.pre_transpose && run && batch > 0) {
@@ -874,7 +883,10 @@ static int chain_walk(bool run, const void* input, const void* const* values, vo
     } else if (next_regrouped) {
       if (run) st = run_family(p, KSMM_ALGO_TC, -1, stream);
     } else if (run) {
-      st = dispatch(p, KSMM_ALGO_AUTO, -1, stream);
+      // An input that starts anywhere may want a kernel that the region was not sized for: the register-staged
+      // one, which needs none of it.
+      const bool lacks = own_region && least_scratch_need(p, auto_choice(p)) > f_scratch_bytes;
+      st = dispatch(p, lacks ? KSMM_ALGO_SIMT : KSMM_ALGO_AUTO, -1, stream);
     } else {
       st = check_problem(p);
       if (st == KSMM_OK && batch > 0) {

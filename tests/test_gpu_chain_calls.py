@@ -297,6 +297,30 @@ def test_trainable_layers_with_another_bias(bs_last):
     kb.check_device()
 
 
+@pytest.mark.parametrize("patterns,dtype,batch,turn", [
+    ([(4, 40, 33, 16), (1, 72, 160, 16)], torch.bfloat16, 128, False), ([(3, 48, 192, 2), (1, 136, 48, 6)], torch.bfloat16, 1024, False),
+    ([(3, 72, 136, 4), (1, 64, 216, 4)], torch.float32, 256, False), ([(1, 100, 128, 4)], torch.float32, 300, True),
+    ([(4, 32, 40, 4)], torch.float16, 64, True), ([(2, 40, 17, 8)], torch.bfloat16, 129, True), ([(2, 64, 64, 1)], torch.float16, 64, True)])
+def test_layers_take_inputs_that_start_anywhere(patterns, dtype, batch, turn):
+    """Layers whose chain has a region for transposed copies, on a view that starts off a 16-byte boundary: the
+    first factor's kernel is another one, with other scratch.  Tolerance: one rounding step per factor (fp32: its
+    sums)."""
+    layer = kb.KSLinear(patterns, dtype=dtype, bs_last=False, out_bs_last=turn, device=DEV)
+    buf = torch.randn(batch * layer.in_size + 8, device=DEV).to(dtype)
+    step = {torch.float32: 2.0 ** -19, torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}[dtype]
+    for shift in (0, 1, 2):
+        x = buf[shift:shift + batch * layer.in_size].view(batch, layer.in_size)
+        with torch.no_grad():
+            y = layer(x)
+        ref = x.double()
+        for f, p in zip(layer.factors, patterns):
+            ref = ref @ kb.from_kernel_format_to_dense(f.data.double(), p).t()
+        ref = ref + layer.bias.double().reshape(1, -1)
+        err = (torch.linalg.norm((y.t() if turn else y).double() - ref) / torch.linalg.norm(ref)).item()
+        assert err < step * len(patterns), (shift, err)
+    kb.check_device()
+
+
 @pytest.mark.parametrize("bs_last", [False, True])
 def test_trainable_layers_with_one_bias_for_all_outputs(bs_last):
     """A bias of one element is added to every output, and its gradient is the sum over all of them."""
