@@ -231,7 +231,7 @@ def run_reference(args, rank, world):
 
 
 def workload_config():
-    return {"workload": "single-factor sweep (configs[1] restricted to the 8 benchmark patterns): "
+    return {"workload": "single-factor sweep (the 8 benchmark patterns): "
                         "fp32+fp16 x batch-last+batch-first, B=25088 per GPU, 32 cases per step",
             "patterns": [list(p) for p in PATTERNS], "batch_per_gpu": BATCH,
             "l2": "a step touches ~5.4 GB of distinct buffers (> 126 MB L2) before any buffer repeats"}
